@@ -28,6 +28,7 @@ SOURCES = [
     "groupby.cu",
     "radix.cu",
     "sort.cu",
+    "rank_sort.cu",
     "abi.cu",
     "noalloc.cu",
     "batch.cu",

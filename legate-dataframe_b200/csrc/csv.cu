@@ -1163,9 +1163,9 @@ void csv_read(const uint8_t* text, int64_t n, char delimiter, int skip_first, co
     int64_t h_total = 0;
     unsigned long long h_first = 0;
     int h_nfields = 0;
-    LDF_CUDA(cudaMemcpyAsync(&h_total, misc.get(), sizeof(h_total), cudaMemcpyDeviceToHost, s));
-    LDF_CUDA(cudaMemcpyAsync(&h_first, first.get(), sizeof(h_first), cudaMemcpyDeviceToHost, s));
-    LDF_CUDA(cudaMemcpyAsync(&h_nfields, nfields.get(), sizeof(h_nfields), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(&h_total, misc.get(), sizeof(h_total));
+    ctx.fetch(&h_first, first.get(), sizeof(h_first));
+    ctx.fetch(&h_nfields, nfields.get(), sizeof(h_nfields));
     ctx.finish();
     const bool has_first = h_first < static_cast<unsigned long long>(nrec);
     rows                 = h_total - (skip_first && has_first ? 1 : 0);
@@ -1196,13 +1196,13 @@ void csv_read(const uint8_t* text, int64_t n, char delimiter, int skip_first, co
     }
     unsigned long long h_err = ~0ull;
     unsigned int h_deferred  = 0;
-    LDF_CUDA(cudaMemcpyAsync(&h_err, first.get() + 1, sizeof(h_err), cudaMemcpyDeviceToHost, s));
-    LDF_CUDA(cudaMemcpyAsync(&h_deferred, ndeferred.get(), sizeof(h_deferred), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(&h_err, first.get() + 1, sizeof(h_err));
+    ctx.fetch(&h_deferred, ndeferred.get(), sizeof(h_deferred));
     ctx.finish();
     if (h_err == ~0ull && h_deferred > 0) {  // floats the 19-digit conversion could not round
       const unsigned int count = std::min<unsigned int>(h_deferred, kCsvMaxDeferred);
       launch("csv_exact_float", csv_exact_float_kernel, csv_blocks(count, 64), 64, 0, s, P, O, count, first.get() + 1);
-      LDF_CUDA(cudaMemcpyAsync(&h_err, first.get() + 1, sizeof(h_err), cudaMemcpyDeviceToHost, s));
+      ctx.fetch(&h_err, first.get() + 1, sizeof(h_err));
       ctx.finish();
     }
     if (h_err != ~0ull) {

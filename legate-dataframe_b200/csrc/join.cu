@@ -899,7 +899,7 @@ void partition_table(const OpContext& ctx, const DCol& key, int64_t n, const std
           : key.width == 2 ? part_hist_kernel<2> : part_hist_kernel<1>;
   launch("part_hist", hk, grid, kPartThreads, 0, s, key, n, ntiles, hist.get(), totals.get());
   unsigned long long h[kPartBuckets];
-  LDF_CUDA(cudaMemcpyAsync(h, totals.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+  ctx.fetch(h, totals.get(), sizeof(h));
   ctx.finish();
   int64_t hb[kPartBuckets], acc = 0;
   for (int b = 0; b < kPartBuckets; ++b) {
@@ -973,7 +973,7 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
     LDF_CUDA(cudaMemcpyAsync(mm.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
     launch("key_range", key_range_kernel, grid_stride_blocks(n_build, 256), 256, 0, s, bk.c[0], n_build, mm.get());
     unsigned long long h[3];
-    LDF_CUDA(cudaMemcpyAsync(h, mm.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(h, mm.get(), sizeof(h));
     ctx.finish();
     const uint64_t span  = h[0] <= h[1] ? (h[1] - h[0]) : ~0ull;  // max - min (order-preserving words)
     const uint64_t limit = static_cast<uint64_t>(std::max<int64_t>(2 * n_build, int64_t(1) << 16));
@@ -985,7 +985,7 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
       launch("direct_build", direct_build_kernel, grid_stride_blocks(n_build, 256), 256, 0, s, bk.c[0], n_build,
              dmin, direct.get(), reinterpret_cast<int*>(mm.get() + 3));
       unsigned long long dup = 0;
-      LDF_CUDA(cudaMemcpyAsync(&dup, mm.get() + 3, sizeof(dup), cudaMemcpyDeviceToHost, s));
+      ctx.fetch(&dup, mm.get() + 3, sizeof(dup));
       ctx.finish();
       if (dup == 0) {
         t.direct = direct.get();
@@ -1036,8 +1036,8 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
     if (t.null_count) unique = ctx.read_i64(t.null_count) <= 1;
   } else if (M == KeyMode::K32 && n_build > 1) {
     int64_t h[2] = {0, 0};  // duplicate flag, null-key rows (all equal with nulls_equal)
-    LDF_CUDA(cudaMemcpyAsync(&h[0], dupflag.get(), sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    if (t.null_count) LDF_CUDA(cudaMemcpyAsync(&h[1], t.null_count, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(&h[0], dupflag.get(), sizeof(int64_t));
+    if (t.null_count) ctx.fetch(&h[1], t.null_count, sizeof(int64_t));
     ctx.finish();
     unique = static_cast<int>(h[0]) == 0 && h[1] <= 1;
   } else if (n_build > 1) {
@@ -1170,7 +1170,7 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
     launch("full_tail", full_tail_kernel, static_cast<unsigned>(btiles), kProbeThreads, 0, s, ta);
     LDF_CHECK_LAUNCH();
     int64_t h[2];
-    LDF_CUDA(cudaMemcpyAsync(h, d_total.get(), 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(h, d_total.get(), 2 * sizeof(int64_t));
     ctx.finish();
     rows = h[0] + h[1];
   } else {

@@ -1550,7 +1550,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
            static_cast<const PqPage*>(d_pages.get()), static_cast<const int*>(d_lists.get()) + nsn + nds, C,
            static_cast<const int64_t*>(entry_off.get()), static_cast<const int32_t*>(entry_len.get()), d_err.get());
   unsigned long long h_err = ~0ull;
-  LDF_CUDA(cudaMemcpyAsync(&h_err, d_err.get(), sizeof(h_err), cudaMemcpyDeviceToHost, s));
+  ctx.fetch(&h_err, d_err.get(), sizeof(h_err));
   ctx.finish();
   if (h_err != ~0ull) {
     for (int j = 0; j < ncols; ++j) free_out_column(al, out[j]);

@@ -16,64 +16,6 @@ constexpr int RI    = kRadixItems;
 constexpr int RTILE = kRadixTile;
 constexpr int RW    = RT / 32;
 
-// Order-preserving word of a sort key from the value's raw bits (zero for a
-// null or a NaN: those rows are placed by the CLASS pass).
-__device__ __forceinline__ uint64_t sort_word_of(const SortKeyDesc& k, uint64_t raw, bool valid)
-{
-  if (!valid) return 0;
-  uint64_t o;
-  switch (k.col.type) {
-    case LDF_INT8: o = (raw & 0xffu) ^ 0x80u; break;
-    case LDF_INT16: o = (raw & 0xffffu) ^ 0x8000u; break;
-    case LDF_INT32: o = (raw & 0xffffffffu) ^ 0x80000000u; break;
-    case LDF_INT64:
-    case LDF_TIMESTAMP_US: o = raw ^ (1ull << 63); break;
-    case LDF_FLOAT32: {
-      uint32_t b = static_cast<uint32_t>(raw);
-      if ((b & 0x7f800000u) == 0x7f800000u && (b & 0x007fffffu)) return 0;  // NaN: CLASS pass
-      if ((b & 0x7fffffffu) == 0) b = 0;                                    // -0.0 == 0.0
-      o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-      o &= 0xffffffffull;
-      break;
-    }
-    case LDF_FLOAT64: {
-      uint64_t b = raw;
-      if ((b & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (b & 0x000fffffffffffffull)) return 0;
-      if ((b & 0x7fffffffffffffffull) == 0) b = 0;
-      o = (b & (1ull << 63)) ? ~b : (b | (1ull << 63));
-      break;
-    }
-    default: o = raw; break;  // unsigned, bool, string ranks (uint32)
-  }
-  if (k.descending) {
-    const uint64_t mask = k.key_bytes >= 8 ? ~0ull : ((1ull << (8 * k.key_bytes)) - 1);
-    o                   = ~o & mask;
-  }
-  return o;
-}
-
-__device__ __forceinline__ uint64_t sort_word(const SortKeyDesc& k, int64_t row)
-{
-  return sort_word_of(k, dbits(k.col, row), dvalid(k.col, row));
-}
-
-// 0 = value, 1 = NaN, 2 = null when nulls_at_end; reversed otherwise
-// (Arrow places NaN next to the values and nulls outermost, either direction).
-__device__ __forceinline__ uint32_t class_digit(const SortKeyDesc& k, int64_t row)
-{
-  const DCol& c = k.col;
-  uint32_t cls  = 0;
-  if (!dvalid(c, row)) cls = 2;
-  else if (c.type == LDF_FLOAT64) {
-    uint64_t b = static_cast<const uint64_t*>(c.data)[row];
-    if ((b & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (b & 0x000fffffffffffffull)) cls = 1;
-  } else if (c.type == LDF_FLOAT32) {
-    uint32_t b = static_cast<const uint32_t*>(c.data)[row];
-    if ((b & 0x7f800000u) == 0x7f800000u && (b & 0x007fffffu)) cls = 1;
-  }
-  return k.nulls_at_end ? cls : 2 - cls;
-}
-
 __device__ __forceinline__ uint64_t bucket_word(const RadixPass& p, int64_t row)
 {
   return key_bits<KeyMode::GEN>(p.hash_keys, row) % p.nparts;
@@ -802,7 +744,7 @@ void sort_word_ranges(const OpContext& ctx, const SortKeyDesc* keys, int nkeys, 
   a.n = nkeys;
   for (int k = 0; k < nkeys; ++k) a.key[k] = keys[k];
   if (n > 0) launch("word_range", word_range_kernel, hblocks(n), 256, 0, s, a, n, mm.get());
-  LDF_CUDA(cudaMemcpyAsync(h.data(), mm.get(), h.size() * 8, cudaMemcpyDeviceToHost, s));
+  ctx.fetch(h.data(), mm.get(), h.size() * 8);
   ctx.finish();
   for (int k = 0; k < nkeys; ++k) {
     mn[k] = h[2 * k];
@@ -842,8 +784,7 @@ void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes,
   if (P > 0 && n > 0) {
     Buffer<uint32_t> d_hist(al, P * 256);
     radix_histograms(ctx, passes, n, d_hist.get(), fused);
-    LDF_CUDA(cudaMemcpyAsync(hist.data(), d_hist.get(), P * 256 * sizeof(uint32_t),
-                             cudaMemcpyDeviceToHost, s));
+    ctx.fetch(hist.data(), d_hist.get(), P * 256 * sizeof(uint32_t));
     ctx.finish();
   }
   if (hist_out) *hist_out = hist;

@@ -32,6 +32,64 @@ struct SortKeyDesc {
   int key_bytes;  // bytes of the transformed word (1..8)
 };
 
+// Order-preserving word of a sort key from the value's raw bits (zero for a
+// null or a NaN: those rows are placed by the CLASS pass).
+__device__ __forceinline__ uint64_t sort_word_of(const SortKeyDesc& k, uint64_t raw, bool valid)
+{
+  if (!valid) return 0;
+  uint64_t o;
+  switch (k.col.type) {
+    case LDF_INT8: o = (raw & 0xffu) ^ 0x80u; break;
+    case LDF_INT16: o = (raw & 0xffffu) ^ 0x8000u; break;
+    case LDF_INT32: o = (raw & 0xffffffffu) ^ 0x80000000u; break;
+    case LDF_INT64:
+    case LDF_TIMESTAMP_US: o = raw ^ (1ull << 63); break;
+    case LDF_FLOAT32: {
+      uint32_t b = static_cast<uint32_t>(raw);
+      if ((b & 0x7f800000u) == 0x7f800000u && (b & 0x007fffffu)) return 0;  // NaN: CLASS pass
+      if ((b & 0x7fffffffu) == 0) b = 0;                                    // -0.0 == 0.0
+      o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+      o &= 0xffffffffull;
+      break;
+    }
+    case LDF_FLOAT64: {
+      uint64_t b = raw;
+      if ((b & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (b & 0x000fffffffffffffull)) return 0;
+      if ((b & 0x7fffffffffffffffull) == 0) b = 0;
+      o = (b & (1ull << 63)) ? ~b : (b | (1ull << 63));
+      break;
+    }
+    default: o = raw; break;  // unsigned, bool, string ranks (uint32)
+  }
+  if (k.descending) {
+    const uint64_t mask = k.key_bytes >= 8 ? ~0ull : ((1ull << (8 * k.key_bytes)) - 1);
+    o                   = ~o & mask;
+  }
+  return o;
+}
+
+__device__ __forceinline__ uint64_t sort_word(const SortKeyDesc& k, int64_t row)
+{
+  return sort_word_of(k, dbits(k.col, row), dvalid(k.col, row));
+}
+
+// 0 = value, 1 = NaN, 2 = null when nulls_at_end; reversed otherwise
+// (Arrow places NaN next to the values and nulls outermost, either direction).
+__device__ __forceinline__ uint32_t class_digit(const SortKeyDesc& k, int64_t row)
+{
+  const DCol& c = k.col;
+  uint32_t cls  = 0;
+  if (!dvalid(c, row)) cls = 2;
+  else if (c.type == LDF_FLOAT64) {
+    uint64_t b = static_cast<const uint64_t*>(c.data)[row];
+    if ((b & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (b & 0x000fffffffffffffull)) cls = 1;
+  } else if (c.type == LDF_FLOAT32) {
+    uint32_t b = static_cast<const uint32_t*>(c.data)[row];
+    if ((b & 0x7f800000u) == 0x7f800000u && (b & 0x007fffffu)) cls = 1;
+  }
+  return k.nulls_at_end ? cls : 2 - cls;
+}
+
 struct RadixPass {
   DigitSrc src;
   int shift;      // bit offset of the digit in the key word (FUSED: in C)
@@ -104,5 +162,19 @@ inline bool payload_empty(const RadixPayload& p) { return p.n == 0 && p.nparts =
 void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
                      int32_t* perm, std::vector<uint32_t>* hist_out = nullptr, int32_t* inv = nullptr,
                      const RadixPayload* payload = nullptr, const FusedKey* fused = nullptr);
+
+// ---- small inputs (rank_sort.cu) -----------------------------------------
+// The whole sort of a table of at most kRankSortRows rows in one or two
+// launches: a row's position is the number of rows that sort before it.
+// `kd`: the keys, least significant first.  False (nothing done) when the
+// table is larger or the keys do not fit.
+constexpr int64_t kRankSortRows = 16384;
+bool rank_sort(const OpContext& ctx, const ldf_column* table, int ncols, const std::vector<SortKeyDesc>& kd, int64_t n,
+               int64_t first, int64_t rows, ldf_column* out);
+
+// rank[d] = bytewise rank of the string of row repr[d] among the D distinct
+// strings of rows repr[0..D), for D of at most kRankStrings.
+constexpr int64_t kRankStrings = 8192;
+void rank_distinct_strings(const OpContext& ctx, const DCol& col, const int32_t* repr, int64_t D, uint32_t* rank);
 
 }  // namespace ldf

@@ -154,10 +154,51 @@ Allocator::~Allocator()
   for (void* c : chunks_) deallocate(c, kScratchChunk);
 }
 
-OpContext::OpContext(const ldf_allocator* a, cudaStream_t s) : alloc_(a, s)
+// ---------------------------------------------------------------------------
+// Read-backs.  Every thread keeps one pinned page group for the small values
+// its calls read back, from its first read-back until it ends; `used` is the
+// part that copies in flight write to.
+// ---------------------------------------------------------------------------
+namespace {
+constexpr size_t kFetchBytes = size_t(64) << 10;
+struct FetchArea {
+  char* p     = nullptr;
+  size_t used = 0;
+  ~FetchArea()
+  {
+    if (p) cudaFreeHost(p);
+  }
+};
+thread_local FetchArea t_fetch;
+}  // namespace
+
+OpContext::~OpContext()
 {
-  err_ = Buffer<int>(alloc_, 1);
-  LDF_CUDA(cudaMemsetAsync(err_.get(), 0, sizeof(int), s));
+  if (fetched_.empty()) return;  // a call that failed between fetch() and finish()
+  cudaStreamSynchronize(stream());
+  t_fetch.used = fetched_.front().off;
+}
+
+int* OpContext::err() const
+{
+  if (err_.get() == nullptr) {
+    err_ = Buffer<int>(alloc_, 1);
+    LDF_CUDA(cudaMemsetAsync(err_.get(), 0, sizeof(int), stream()));
+  }
+  return err_.get();
+}
+
+void OpContext::fetch(void* host, const void* dev, size_t nbytes) const
+{
+  if (t_fetch.p == nullptr)
+    LDF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&t_fetch.p), kFetchBytes, cudaHostAllocPortable));
+  if (nbytes > kFetchBytes - t_fetch.used) {
+    LDF_CUDA(cudaMemcpyAsync(host, dev, nbytes, cudaMemcpyDeviceToHost, stream()));
+    return;
+  }
+  fetched_.push_back(Fetched{host, t_fetch.used, nbytes});
+  t_fetch.used += (nbytes + 15) & ~size_t(15);
+  LDF_CUDA(cudaMemcpyAsync(t_fetch.p + fetched_.back().off, dev, nbytes, cudaMemcpyDeviceToHost, stream()));
 }
 
 static void raise_device_error(int h)
@@ -169,20 +210,20 @@ static void raise_device_error(int h)
 
 int64_t OpContext::read_i64(const int64_t* d) const
 {
-  int64_t h[1] = {0};
-  int e        = 0;
-  LDF_CUDA(cudaMemcpyAsync(h, d, sizeof(int64_t), cudaMemcpyDeviceToHost, stream()));
-  LDF_CUDA(cudaMemcpyAsync(&e, err_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream()));
-  LDF_CUDA(cudaStreamSynchronize(stream()));
-  raise_device_error(e);
-  return h[0];
+  int64_t h = 0;
+  fetch(&h, d, sizeof(h));
+  finish();
+  return h;
 }
 
 void OpContext::finish() const
 {
   int e = 0;
-  LDF_CUDA(cudaMemcpyAsync(&e, err_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream()));
+  if (err_.get() != nullptr) fetch(&e, err_.get(), sizeof(int));
   LDF_CUDA(cudaStreamSynchronize(stream()));
+  for (const Fetched& f : fetched_) std::memcpy(f.host, t_fetch.p + f.off, f.nbytes);
+  if (!fetched_.empty()) t_fetch.used = fetched_.front().off;
+  fetched_.clear();
   raise_device_error(e);
 }
 

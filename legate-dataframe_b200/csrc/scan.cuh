@@ -119,22 +119,36 @@ __device__ __forceinline__ int64_t next_tile_id(unsigned long long* counter, int
 // Host helpers (scan.cu).
 // ---------------------------------------------------------------------------
 // Per-call context: allocator, stream and the call's device error word, which
-// bounded waits set instead of trapping.  The word is checked whenever the host
-// reads a result back (the only synchronisation points of an op).
+// bounded waits set instead of trapping.  The word is made when a kernel first
+// asks for it, and checked whenever the host reads a result back (the only
+// synchronisation points of an op).
 class OpContext {
  public:
-  OpContext(const ldf_allocator* a, cudaStream_t s);
+  OpContext(const ldf_allocator* a, cudaStream_t s) : alloc_(a, s) {}
+  ~OpContext();
+  OpContext(const OpContext&)            = delete;
+  OpContext& operator=(const OpContext&) = delete;
   const Allocator& alloc() const { return alloc_; }
   cudaStream_t stream() const { return alloc_.stream(); }
-  int* err() const { return err_.get(); }
+  int* err() const;
+  // Queue a copy of `nbytes` device bytes to `host`, which holds them after
+  // the next finish() (or read_i64()).  Small copies go through pinned memory
+  // of the calling thread: they queue behind one another and cost one wait,
+  // where each copy to pageable memory waits for itself.
+  void fetch(void* host, const void* dev, size_t nbytes) const;
   // Copy one device int64 to the host, wait, and check the error word.
   int64_t read_i64(const int64_t* d) const;
-  // Wait for the stream and check the error word.
+  // Wait for the stream, deliver the fetched values and check the error word.
   void finish() const;
 
  private:
+  struct Fetched {
+    void* host;
+    size_t off, nbytes;
+  };
   Allocator alloc_;
-  Buffer<int> err_;
+  mutable Buffer<int> err_;
+  mutable std::vector<Fetched> fetched_;
 };
 
 // out[i] = sum(in[0..i)) for counts; *d_total (device) = sum(in).

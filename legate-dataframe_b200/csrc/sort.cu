@@ -323,7 +323,7 @@ int64_t string_ranks(const OpContext& ctx, const DCol& col, int64_t n, uint32_t*
     launch("distinct_stats", distinct_stats_kernel, blocks_for(static_cast<int64_t>(scap)), 256, 0, s,
            static_cast<const unsigned int*>(scount.get()), static_cast<int64_t>(scap), sm.get());
     unsigned long long h[3];
-    LDF_CUDA(cudaMemcpyAsync(h, sm.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(h, sm.get(), sizeof(h));
     ctx.finish();
     if (h[2] == 0) {
       const double est = std::sqrt(static_cast<double>(n) / kSample) * static_cast<double>(h[1]) +
@@ -335,6 +335,9 @@ int64_t string_ranks(const OpContext& ctx, const DCol& col, int64_t n, uint32_t*
   Buffer<int32_t> row_slot(al, n);
   Buffer<int64_t> misc(al, 4);
   Buffer<unsigned long long> slots;
+  Buffer<int32_t> slot_id;
+  Buffer<int32_t> repr(al, n);
+  int64_t D = 0;
   int* overflow              = reinterpret_cast<int*>(misc.get());
   unsigned long long* dcount = reinterpret_cast<unsigned long long*>(misc.get() + 1);
   unsigned long long* maxlen = reinterpret_cast<unsigned long long*>(misc.get() + 2);
@@ -344,21 +347,24 @@ int64_t string_ranks(const OpContext& ctx, const DCol& col, int64_t n, uint32_t*
     LDF_CUDA(cudaMemsetAsync(misc.get(), 0, 32, s));
     launch("str_find_insert", str_find_insert_kernel, blocks_for(n), 256, 0, s, col, n, int64_t(1), slots.get(), cap,
            row_slot.get(), overflow);
+    // compacted at once: a table that overflowed is compacted in vain, one
+    // that did not (the usual case) needs a single read-back
+    slot_id = Buffer<int32_t>(al, cap);
+    launch("str_compact", str_compact_kernel, blocks_for(cap), 256, 0, s, slots.get(), cap, slot_id.get(), repr.get(),
+           dcount);
     int ov = 0;
-    LDF_CUDA(cudaMemcpyAsync(&ov, overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
+    ctx.fetch(&ov, overflow, sizeof(int));
+    ctx.fetch(&D, dcount, sizeof(D));
     ctx.finish();
     if (ov == 0) break;
     const uint64_t full = static_cast<uint64_t>(2 * n + 64);
     if (attempt > 0 || cap >= full) fail(LDF_ERR_INTERNAL, "string dictionary overflow");
     cap = full;  // the estimate was too low: room for every row
   }
-  Buffer<int32_t> slot_id(al, cap);
-  Buffer<int32_t> repr(al, n);
-  launch("str_compact", str_compact_kernel, blocks_for(cap), 256, 0, s, slots.get(), cap, slot_id.get(), repr.get(), dcount);
-  LDF_CHECK_LAUNCH();
-  const int64_t D = ctx.read_i64(misc.get() + 1);
   Buffer<uint32_t> rank(al, std::max<int64_t>(D, 1));
-  if (D > 0) {
+  if (D > 0 && D <= kRankStrings) {
+    rank_distinct_strings(ctx, col, repr.get(), D, rank.get());
+  } else if (D > 0) {
     launch("max_len", max_len_kernel, blocks_for(D), 256, 0, s, col, repr.get(), D, maxlen);
     LDF_CHECK_LAUNCH();
     const int64_t L = ctx.read_i64(misc.get() + 2);
@@ -621,7 +627,7 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
     if (c.type == LDF_STRING) {
       ranks.emplace_back(al, std::max<int64_t>(n, 1));
       int32_t* rep = nullptr;
-      if (whole && keys[j] < kPassPayload) {  // a column the last pass moves
+      if (whole && keys[j] < kPassPayload && n > kRankSortRows) {  // a column the last pass moves
         reps.emplace_back(al, std::max<int64_t>(n, 1));
         rep            = reps.back().get();
         rep_of[keys[j]] = rep;
@@ -636,6 +642,10 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
     k.key_bytes = k.col.width;
     if (c.valid != nullptr || is_float(c.type)) fusable = false;  // those need CLASS passes
     kd.push_back(k);
+  }
+  if (rank_sort(ctx, table, ncols, kd, n, first, rows, out)) {
+    ctx.finish();
+    return;
   }
   // Keys without nulls or floats whose value ranges fit one word of at most
   // kFusedMaxBits bits are sorted on that word: its first pass loads every key
@@ -811,7 +821,7 @@ void hash_partition(const ldf_column* table, int ncols, const int32_t* keys, int
   if (!fsrc.empty()) inv = Buffer<int32_t>(al, std::max<int64_t>(n, 1));
   radix_sort_rows(ctx, passes, n, perm.get(), nullptr, fsrc.empty() ? nullptr : inv.get(), &mv.pay);
   std::vector<unsigned long long> h(nparts);
-  LDF_CUDA(cudaMemcpyAsync(h.data(), counts.get(), static_cast<size_t>(nparts) * 8, cudaMemcpyDeviceToHost, s));
+  ctx.fetch(h.data(), counts.get(), static_cast<size_t>(nparts) * 8);
   scatter_fixed_columns(ctx, fsrc.data(), inv.get(), n, fdst.data(), static_cast<int>(fsrc.size()));
   move_strings_in_order(ctx, table, mv, n, out);
   for (int j = 0; j < ncols; ++j)
