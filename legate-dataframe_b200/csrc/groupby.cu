@@ -232,10 +232,10 @@ __device__ __forceinline__ double chunks_to_double(const unsigned long long* acc
 }
 
 // ---- group ids ------------------------------------------------------------
-// Key table slots.  K32: one word (id << 32 | key32), published by one CAS.
-// K64 / GEN: two words {key word, id}; the key word is claimed by CAS and the
-// id stored right after, so a reader that sees the key before its id waits
-// (bounded) for the id.  Empty key word: kEmpty, or kSentinel64 for K64.
+// Key table slots.  K32: one word (id << 32 | key32); K64 / GEN: two words
+// {key word, id}.  The key is claimed by CAS (K32 with kBusyId in the id's
+// place) and the id stored after, so a reader that sees the key before its id
+// waits (bounded) for the id.  Empty key word: kEmpty, or kSentinel64 for K64.
 template <KeyMode M>
 __device__ __forceinline__ uint64_t empty_word()
 {
@@ -256,6 +256,25 @@ __device__ __forceinline__ uint32_t wait_id(const unsigned long long* slot_hi, i
   return kUnsetId;
 }
 
+// The same for a K32 slot, claimed with kBusyId in the id's place.
+constexpr uint64_t kBusyId = 0xfffffffeull;
+__device__ __forceinline__ uint32_t wait_id32(const unsigned long long* slot, int* err)
+{
+  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(slot) : "memory");
+    if ((v >> 32) != kBusyId) return static_cast<uint32_t>(v >> 32);
+    __nanosleep(64);
+  }
+  atomicExch(err, LDF_ERR_TIMEOUT);
+  return kUnsetId;
+}
+
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, uint64_t v)
+{
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 template <KeyMode M>
 __device__ __forceinline__ bool same_key(const GbPlan& p, uint64_t v, uint64_t word, uint64_t h, int64_t r)
 {
@@ -265,27 +284,36 @@ __device__ __forceinline__ bool same_key(const GbPlan& p, uint64_t v, uint64_t w
          keys_equal(p.k, r, p.k, static_cast<int64_t>(v >> 32));
 }
 
-// Per-warp pool of pre-zeroed group ids (warp-uniform state).
+// Per-warp pool of pre-zeroed group ids (warp-uniform state).  The first
+// refills take exactly the ids in need, later ones 32 at a time: few groups
+// leave few unused ids behind (a fixed pool of 32 left 300,000 for 10,000
+// groups, which overflowed the tables and re-ran the pass), and many groups
+// do not queue up on the counter.
+constexpr int kExactRefills = 4;
 struct IdPool {
   uint64_t next, end;
+  int refills;
 };
 
-// Take ids for the lanes with `need` set; refills the pool (32 ids, records
-// zeroed, one fence) when it runs short.  All 32 lanes call it together.
+// Take ids for the lanes with `need` set (records zeroed, one fence per
+// refill); kEmpty when none are left.  All 32 lanes call it together.
 __device__ __forceinline__ uint64_t pool_take(const GbPlan& p, IdPool& pool, bool need)
 {
   const uint32_t want = __ballot_sync(0xffffffffu, need);
   if (want == 0) return kEmpty;
   const uint32_t k = __popc(want);
   if (pool.end - pool.next < k) {
+    const unsigned long long take = pool.refills < kExactRefills ? k : 32;
+    ++pool.refills;
     unsigned long long base = 0;
-    if (lane_id() == 0) base = atomicAdd(p.id_counter, 32ull);
+    if (lane_id() == 0) base = atomicAdd(p.id_counter, take);
     base = __shfl_sync(0xffffffffu, base, 0);
-    const uint64_t end = base + 32 < p.id_cap ? base + 32 : p.id_cap;
+    const uint64_t end = base + take < p.id_cap ? base + take : p.id_cap;
     if (base < end) {
       const uint64_t w0 = base * p.stride, w1 = end * p.stride;
       for (uint64_t w = w0 + lane_id(); w < w1; w += 32) p.states[w] = 0;
       __threadfence();
+      __syncwarp();
     }
     pool.next = base;
     pool.end  = end > base ? end : base;
@@ -311,6 +339,10 @@ __host__ __device__ constexpr int assign_rows()
 }
 
 // Group ids of the R rows of this lane (kUnsetId for rows past the end).
+// A row that finds an empty slot claims it with its key; only the rows whose
+// claim succeeded take an id and publish it.  Rows that met a claimed slot
+// read the id last: a warp has then published all its own claims, so a wait
+// is always on another warp.
 template <KeyMode M, int R>
 __device__ void group_ids(const GbPlan& p, IdPool& pool, const int64_t (&r)[R], uint32_t (&id)[R])
 {
@@ -358,19 +390,29 @@ __device__ void group_ids(const GbPlan& p, IdPool& pool, const int64_t (&r)[R], 
       hi[j]              = t.y;
     }
   }
-  bool need[R];
+  bool won[R], later[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) {
-    need[j] = false;
+    won[j] = later[j] = false;
     if (!pending[j]) continue;
     for (int probe = 0; probe < kMaxProbe; ++probe) {
       if (v[j] == empty) {
-        need[j] = true;
-        break;
+        const uint64_t claim = M == KeyMode::K32 ? (kBusyId << 32) | (word[j] & 0xffffffffull) : word[j];
+        v[j]                 = atomicCAS(s + sw * idx[j], empty, claim);
+        if (v[j] == empty) {
+          won[j] = true;
+          break;
+        }
+        hi[j] = kEmpty;
       }
       if (same_key<M>(p, v[j], word[j], h[j], r[j])) {
-        if (M == KeyMode::K32) id[j] = static_cast<uint32_t>(v[j] >> 32);
-        else id[j] = hi[j] != kEmpty ? static_cast<uint32_t>(hi[j]) : wait_id(s + 2 * idx[j] + 1, p.err);
+        if (M == KeyMode::K32) {
+          id[j]    = static_cast<uint32_t>(v[j] >> 32);
+          later[j] = id[j] == static_cast<uint32_t>(kBusyId);
+        } else {
+          id[j]    = static_cast<uint32_t>(hi[j]);
+          later[j] = hi[j] == kEmpty;
+        }
         break;
       }
       idx[j] = idx[j] + 1 == p.cap ? 0 : idx[j] + 1;
@@ -384,38 +426,32 @@ __device__ void group_ids(const GbPlan& p, IdPool& pool, const int64_t (&r)[R], 
       if (probe + 1 == kMaxProbe) atomicExch(p.overflow, 1);
     }
   }
-  // inserts: ids from the warp pool, then publish
+  // the winners' ids (kUnsetId when none are left: the call re-runs)
 #pragma unroll
   for (int j = 0; j < R; ++j) {
-    const uint64_t mine = pool_take(p, pool, need[j]);
-    if (!need[j] || mine == kEmpty) continue;
-    p.id_key[mine]      = M == KeyMode::GEN ? static_cast<uint64_t>(r[j]) : word[j];
-    const uint64_t full = M == KeyMode::K32 ? ((mine << 32) | (word[j] & 0xffffffffull)) : word[j];
-    for (int probe = 0; probe < kMaxProbe; ++probe) {
-      const uint64_t old = atomicCAS(s + sw * idx[j], empty, full);
-      if (old == empty) {
-        if (M != KeyMode::K32) s[2 * idx[j] + 1] = mine;
-        id[j] = static_cast<uint32_t>(mine);
-        break;
-      }
-      if (same_key<M>(p, old, word[j], h[j], r[j])) {  // lost the race: `mine` stays a zeroed hole
-        id[j] = M == KeyMode::K32 ? static_cast<uint32_t>(old >> 32) : wait_id(s + 2 * idx[j] + 1, p.err);
-        break;
-      }
-      // another key took the slot: probe on to the key or the next empty slot
-      bool done = false;
-      for (; probe < kMaxProbe; ++probe) {
-        idx[j]           = idx[j] + 1 == p.cap ? 0 : idx[j] + 1;
-        const uint64_t t = s[sw * idx[j]];
-        if (t == empty) break;
-        if (same_key<M>(p, t, word[j], h[j], r[j])) {
-          id[j] = M == KeyMode::K32 ? static_cast<uint32_t>(t >> 32) : wait_id(s + 2 * idx[j] + 1, p.err);
-          done  = true;
-          break;
-        }
-      }
-      if (done) break;
-      if (probe >= kMaxProbe - 1) atomicExch(p.overflow, 1);
+    const uint64_t mine = pool_take(p, pool, won[j]);
+    if (!won[j]) continue;
+    id[j] = mine == kEmpty ? kUnsetId : static_cast<uint32_t>(mine);
+    if (mine != kEmpty) p.id_key[mine] = M == KeyMode::GEN ? static_cast<uint64_t>(r[j]) : word[j];
+    // relaxed: the records were zeroed behind the refill's fence, and no one
+    // reads id_key before the pass ends
+    if (M == KeyMode::K32) st_relaxed_u64(s + idx[j], (static_cast<uint64_t>(id[j]) << 32) | (word[j] & 0xffffffffull));
+    else st_relaxed_u64(s + 2 * idx[j] + 1, id[j]);
+  }
+  __syncwarp();
+  // The slot was read while its id was missing, and this SM's L1 may keep that
+  // copy for as long as the key stays frequent: storing the id over itself
+  // puts it into the copy (without it every later row of a frequent key came
+  // through here, 5.3 against 2.8 ms on 200M Zipf rows).
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    if (!later[j]) continue;
+    if (M == KeyMode::K32) {
+      id[j]     = wait_id32(s + idx[j], p.err);
+      s[idx[j]] = (static_cast<uint64_t>(id[j]) << 32) | (word[j] & 0xffffffffull);
+    } else {
+      id[j]             = wait_id(s + 2 * idx[j] + 1, p.err);
+      s[2 * idx[j] + 1] = id[j];
     }
   }
 }
@@ -485,7 +521,7 @@ __global__ void __launch_bounds__(kGbThreads) assign_kernel(GbPlan p, uint32_t* 
   const int H   = p.hot;
   for (int i = threadIdx.x; i < H; i += blockDim.x) cnt[i] = 0;
   __syncthreads();
-  IdPool pool{0, 0};
+  IdPool pool{0, 0, 0};
   constexpr int R          = assign_rows<M>();
   constexpr int64_t kChunk = 32 * R * 8;  // rows per dynamically scheduled chunk
   for (;;) {
@@ -517,6 +553,32 @@ __global__ void __launch_bounds__(kGbThreads) assign_kernel(GbPlan p, uint32_t* 
   __syncthreads();
   for (int g = threadIdx.x; g < H; g += blockDim.x)
     if (cnt[g]) red_add(p.states + static_cast<int64_t>(g) * p.stride, cnt[g]);
+}
+
+// The keys of a strided sample of at most kSeedRows rows inserted before the
+// assign pass, by a few CTAs: the frequent keys then have the lowest ids, which
+// the pass counts in shared memory (left to the race of its first wave, a key
+// holding an eighth of the rows could get any id, and 24M reductions on one
+// word took assign from 2.8 to 5-8 ms on 200M rows), and their slots are
+// complete before the wave starts.
+constexpr int64_t kSeedRows = 16384;
+template <KeyMode M>
+__global__ void __launch_bounds__(kGbThreads) seed_keys_kernel(GbPlan p, int64_t rows, int64_t stride)
+{
+  IdPool pool{0, 0, 0};
+  constexpr int R    = assign_rows<M>();
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x * R;
+  for (int64_t base = (static_cast<int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31)) * R; base < rows;
+       base += step) {
+    int64_t r[R];
+    uint32_t id[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int64_t i = base + j * 32 + lane_id();
+      r[j]            = i < rows ? i * stride : p.n;
+    }
+    group_ids<M, R>(p, pool, r, id);
+  }
 }
 
 // Factor from the sampled group estimate to the key-table sizing estimate
@@ -1284,9 +1346,10 @@ struct FinArgs {
   GbPlan p;
   const unsigned long long* rec;  // field-major records of the frequency ranks
   uint64_t ld;
-  const int32_t* perm;            // rank -> assign-pass id
+  const int32_t* perm;            // rank -> assign-pass id (null: the same)
   int key_mode;
-  const int64_t* groups;
+  const int64_t* groups;          // output row -> rank (null: the same)
+  const uint32_t* special_ids;    // ids of the null key and of kSentinel64 (null: kIdNull, kIdSentinel)
   int64_t ngroups;
   int nkeys;
   OCol key_dst[kMaxKeys];
@@ -1345,113 +1408,120 @@ __device__ __forceinline__ double float_sum(const ColPlan& c, const unsigned lon
   return chunks_to_double(rec + c.off_sum * L, L) + c.fb[id];
 }
 
+// Output row i.
+__device__ __forceinline__ void finalize_row(const FinArgs& f, int64_t i)
+{
+  const int64_t id              = f.groups ? f.groups[i] : i;  // frequency rank
+  const GbPlan& p               = f.p;
+  const uint64_t L              = f.ld;
+  const unsigned long long* rec = f.rec + id;
+  const int64_t old             = f.perm ? f.perm[id] : id;  // assign-pass id
+  const int64_t null_id         = f.special_ids ? f.special_ids[0] : kIdNull;
+  const int64_t sentinel_id     = f.special_ids ? f.special_ids[1] : kIdSentinel;
+  // keys
+  if (f.key_mode == static_cast<int>(KeyMode::GEN)) {
+    const int64_t rr = static_cast<int64_t>(p.id_key[old]);
+    f.repr[i]        = static_cast<int32_t>(rr);
+    for (int j = 0; j < f.nkeys; ++j) {
+      const OCol& d = f.key_dst[j];
+      if (d.type == LDF_STRING) continue;
+      copy_fixed(d.data, i, p.k.c[j].data, rr, d.width);
+      if (d.valid) d.valid[i] = dvalid(p.k.c[j], rr) ? 1 : 0;
+    }
+  } else {
+    const OCol& d      = f.key_dst[0];
+    const bool is_null = old == null_id;
+    const uint64_t kb  = old == sentinel_id ? kSentinel64 : is_null ? 0 : p.id_key[old];
+    store_int(OCol{d.data, nullptr, LDF_UINT64, d.width}, i, kb);
+    if (d.valid) d.valid[i] = is_null ? 0 : 1;
+  }
+  const uint64_t call = rec[0];
+  // the exact float sum of a column, rounded once, is shared by its SUM and MEAN
+  int sum_col      = -1;
+  double sum_val   = 0.0;
+  bool sum_special = false;
+  double sum_sval  = 0.0;
+  for (int a = 0; a < f.nagg; ++a) {
+    const AggOut& o = f.a[a];
+    const OCol& d   = o.dst;
+    if (o.kind == LDF_AGG_COUNT_ALL) {
+      store_int(d, i, call);
+      if (d.valid) d.valid[i] = 1;
+      continue;
+    }
+    const ColPlan& c               = p.c[o.col];
+    const unsigned long long* crec = c.crec + static_cast<uint64_t>(id) * c.cw;
+    const uint64_t vc              = c.nullable ? crec[c.off_vcount] : call;
+    bool ok           = vc > 0;
+    switch (o.kind) {
+      case LDF_AGG_COUNT: {
+        uint64_t v = o.count_mode == LDF_COUNT_ALL ? call : o.count_mode == LDF_COUNT_ONLY_NULL ? call - vc : vc;
+        store_int(d, i, v);
+        ok = true;
+        break;
+      }
+      case LDF_AGG_COUNT_DISTINCT: {
+        uint64_t has_null = call > vc ? 1 : 0;
+        uint64_t nd       = (c.states & ST_NDIST) ? rec[c.off_nd * L] : 0;
+        uint64_t v = o.count_mode == LDF_COUNT_ALL ? nd + has_null : o.count_mode == LDF_COUNT_ONLY_NULL ? has_null : nd;
+        store_int(d, i, v);
+        ok = true;
+        break;
+      }
+      case LDF_AGG_SUM:
+      case LDF_AGG_MEAN: {
+        if (!ok) {
+          store_int(d, i, 0);
+          break;
+        }
+        if (c.fixed) {
+          if (sum_col != o.col) {
+            sum_val = float_sum(c, crec, 1, id, sum_special, sum_sval);
+            sum_col = o.col;
+          }
+          double sv = sum_special ? sum_sval : sum_val;
+          if (o.kind == LDF_AGG_MEAN) sv = sv / static_cast<double>(vc);
+          store_double(d, i, sv);
+        } else {
+          const uint64_t s = crec[c.off_sum];
+          const double sd  = is_signed_int_dev(o.in_type) ? static_cast<double>(static_cast<int64_t>(s))
+                                                          : static_cast<double>(s);
+          if (o.kind == LDF_AGG_MEAN) store_double(d, i, sd / static_cast<double>(vc));
+          else if (d.type == LDF_FLOAT64 || d.type == LDF_FLOAT32) store_double(d, i, sd);
+          else store_int(d, i, s);
+        }
+        break;
+      }
+      case LDF_AGG_MIN:
+      case LDF_AGG_MAX: {
+        if (!ok) {
+          store_int(d, i, 0);
+          break;
+        }
+        const uint64_t o64 = o.kind == LDF_AGG_MIN ? ~crec[c.off_mn] : crec[c.off_mx];
+        const uint64_t b   = unordered_bits(o.in_type, o64);
+        if (d.type == o.in_type) {
+          store_int(OCol{d.data, nullptr, LDF_UINT64, d.width}, i, b);
+        } else if (o.in_type == LDF_FLOAT32) {
+          store_double(d, i, static_cast<double>(__uint_as_float(static_cast<uint32_t>(b))));
+        } else if (o.in_type == LDF_FLOAT64) {
+          store_double(d, i, __longlong_as_double(static_cast<long long>(b)));
+        } else {
+          store_int(d, i, b);
+        }
+        break;
+      }
+      default: break;
+    }
+    if (d.valid) d.valid[i] = ok ? 1 : 0;
+  }
+}
+
 __global__ void finalize_kernel(FinArgs f)
 {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < f.ngroups;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t id              = f.groups[i];  // frequency rank
-    const GbPlan& p               = f.p;
-    const uint64_t L              = f.ld;
-    const unsigned long long* rec = f.rec + id;
-    const int64_t old             = f.perm[id];  // assign-pass id
-    // keys
-    if (f.key_mode == static_cast<int>(KeyMode::GEN)) {
-      const int64_t rr = static_cast<int64_t>(p.id_key[old]);
-      f.repr[i]        = static_cast<int32_t>(rr);
-      for (int j = 0; j < f.nkeys; ++j) {
-        const OCol& d = f.key_dst[j];
-        if (d.type == LDF_STRING) continue;
-        copy_fixed(d.data, i, p.k.c[j].data, rr, d.width);
-        if (d.valid) d.valid[i] = dvalid(p.k.c[j], rr) ? 1 : 0;
-      }
-    } else {
-      const OCol& d      = f.key_dst[0];
-      const bool is_null = old == kIdNull;
-      const uint64_t kb  = old == kIdSentinel ? kSentinel64 : is_null ? 0 : p.id_key[old];
-      store_int(OCol{d.data, nullptr, LDF_UINT64, d.width}, i, kb);
-      if (d.valid) d.valid[i] = is_null ? 0 : 1;
-    }
-    const uint64_t call = rec[0];
-    // the exact float sum of a column, rounded once, is shared by its SUM and MEAN
-    int sum_col      = -1;
-    double sum_val   = 0.0;
-    bool sum_special = false;
-    double sum_sval  = 0.0;
-    for (int a = 0; a < f.nagg; ++a) {
-      const AggOut& o = f.a[a];
-      const OCol& d   = o.dst;
-      if (o.kind == LDF_AGG_COUNT_ALL) {
-        store_int(d, i, call);
-        if (d.valid) d.valid[i] = 1;
-        continue;
-      }
-      const ColPlan& c               = p.c[o.col];
-      const unsigned long long* crec = c.crec + static_cast<uint64_t>(id) * c.cw;
-      const uint64_t vc              = c.nullable ? crec[c.off_vcount] : call;
-      bool ok           = vc > 0;
-      switch (o.kind) {
-        case LDF_AGG_COUNT: {
-          uint64_t v = o.count_mode == LDF_COUNT_ALL ? call : o.count_mode == LDF_COUNT_ONLY_NULL ? call - vc : vc;
-          store_int(d, i, v);
-          ok = true;
-          break;
-        }
-        case LDF_AGG_COUNT_DISTINCT: {
-          uint64_t has_null = call > vc ? 1 : 0;
-          uint64_t nd       = (c.states & ST_NDIST) ? rec[c.off_nd * L] : 0;
-          uint64_t v = o.count_mode == LDF_COUNT_ALL ? nd + has_null : o.count_mode == LDF_COUNT_ONLY_NULL ? has_null : nd;
-          store_int(d, i, v);
-          ok = true;
-          break;
-        }
-        case LDF_AGG_SUM:
-        case LDF_AGG_MEAN: {
-          if (!ok) {
-            store_int(d, i, 0);
-            break;
-          }
-          if (c.fixed) {
-            if (sum_col != o.col) {
-              sum_val = float_sum(c, crec, 1, id, sum_special, sum_sval);
-              sum_col = o.col;
-            }
-            double sv = sum_special ? sum_sval : sum_val;
-            if (o.kind == LDF_AGG_MEAN) sv = sv / static_cast<double>(vc);
-            store_double(d, i, sv);
-          } else {
-            const uint64_t s = crec[c.off_sum];
-            const double sd  = is_signed_int_dev(o.in_type) ? static_cast<double>(static_cast<int64_t>(s))
-                                                            : static_cast<double>(s);
-            if (o.kind == LDF_AGG_MEAN) store_double(d, i, sd / static_cast<double>(vc));
-            else if (d.type == LDF_FLOAT64 || d.type == LDF_FLOAT32) store_double(d, i, sd);
-            else store_int(d, i, s);
-          }
-          break;
-        }
-        case LDF_AGG_MIN:
-        case LDF_AGG_MAX: {
-          if (!ok) {
-            store_int(d, i, 0);
-            break;
-          }
-          const uint64_t o64 = o.kind == LDF_AGG_MIN ? ~crec[c.off_mn] : crec[c.off_mx];
-          const uint64_t b   = unordered_bits(o.in_type, o64);
-          if (d.type == o.in_type) {
-            store_int(OCol{d.data, nullptr, LDF_UINT64, d.width}, i, b);
-          } else if (o.in_type == LDF_FLOAT32) {
-            store_double(d, i, static_cast<double>(__uint_as_float(static_cast<uint32_t>(b))));
-          } else if (o.in_type == LDF_FLOAT64) {
-            store_double(d, i, __longlong_as_double(static_cast<long long>(b)));
-          } else {
-            store_int(d, i, b);
-          }
-          break;
-        }
-        default: break;
-      }
-      if (d.valid) d.valid[i] = ok ? 1 : 0;
-    }
-  }
+       i += (int64_t)gridDim.x * blockDim.x)
+    finalize_row(f, i);
 }
 
 unsigned gs_blocks(int64_t n, int threads)
@@ -1486,6 +1556,436 @@ void launch_column(ColArgs& a, int type, cudaStream_t s)
     case LDF_FLOAT64: go(column_kernel<8, false, true>); break;
     default: fail(LDF_ERR_UNSUPPORTED, "unsupported aggregation column type");
   }
+}
+
+// Output columns of `rows` rows, allocated and bound to f; `repr`: the
+// representative row of every output row (multi-column and string keys).
+void bind_outputs(const Allocator& al, const ldf_column* table, const int32_t* keys, int nkeys,
+                  const ldf_aggregation* aggs, int naggs, const std::vector<int>& agg_col, bool need_repr, int64_t rows,
+                  ldf_column* out, FinArgs& f, Buffer<int32_t>& repr)
+{
+  f.nkeys = nkeys;
+  for (int j = 0; j < nkeys; ++j) {
+    const ldf_column& kc = table[keys[j]];
+    out[j]               = alloc_out_column(al, kc.type, rows, kc.valid != nullptr);
+    f.key_dst[j]         = OCol{out[j].data, out[j].valid, kc.type, type_width(kc.type)};
+  }
+  if (need_repr) {
+    repr   = Buffer<int32_t>(al, std::max<int64_t>(rows, 1));
+    f.repr = repr.get();
+  }
+  f.nagg = naggs;
+  for (int a = 0; a < naggs; ++a) {
+    const ldf_aggregation& ag = aggs[a];
+    const bool nullable       = !(ag.kind == LDF_AGG_COUNT_ALL || ag.kind == LDF_AGG_COUNT_DISTINCT);
+    out[nkeys + a]            = alloc_out_column(al, ag.out_type, rows, nullable);
+    AggOut& o                 = f.a[a];
+    o.kind                    = ag.kind;
+    o.count_mode              = ag.count_mode;
+    o.col                     = agg_col[a];
+    o.in_type                 = ag.kind == LDF_AGG_COUNT_ALL ? LDF_INT64 : table[ag.in_col].type;
+    o.dst = OCol{out[nkeys + a].data, out[nkeys + a].valid, ag.out_type, type_width(ag.out_type)};
+  }
+}
+
+// Words of the records: the shared one (row count, then the distinct counts)
+// and every value column's block.
+void layout_records(GbPlan& p)
+{
+  int w = 1;
+  for (int ci = 0; ci < p.ncols; ++ci) {
+    ColPlan& c   = p.c[ci];
+    c.sum_chunks = c.fixed ? kSumChunks : 2;
+    c.mm64       = type_width(c.col.type) > 4 ? 1 : 0;
+    int cw       = 0;  // the column block
+    c.off_vcount = c.nullable ? cw++ : 0;
+    if (c.states & ST_SUM) {
+      c.off_sum = cw;
+      cw += c.fixed ? kSumChunks : 1;
+    }
+    if (c.states & ST_MIN) c.off_mn = cw++;
+    if (c.states & ST_MAX) c.off_mx = cw++;
+    c.cw = cw;
+    if (c.states & ST_NDIST) c.off_nd = w++;
+  }
+  p.stride = w;
+}
+
+// ===========================================================================
+// Small inputs: the whole aggregation in ONE kernel, a thread-block cluster
+// whose CTAs meet at hardware cluster barriers between the phases.  The
+// general plan needs some twenty stream operations and three read-backs,
+// which is all the time a call on a few thousand rows takes; here the host
+// reads back one row count.  SUM and COUNT of 1,000 rows: 222 -> 90 us a
+// call, of 50,000 rows with 5,000 groups 260 -> 100 us.
+//   1. empty key slots (and NUNIQUE pair sets)
+//   2. every row finds or inserts its key's slot; the row that inserts one
+//      takes the next dense group id and zeroes that group's records
+//   3. rows accumulate into the records of their slot's id; the lowest ids
+//      (the first keys met, so the frequent ones) in shared memory first
+//   4. group id = output row: finalized in place, outputs allocated for as
+//      many groups as rows
+// The records, exact float sums and output rules are the general plan's.
+// ===========================================================================
+constexpr int kSmallThreads = 512;
+constexpr int kSmallHot     = 256;  // ids with shared-memory records
+struct SmallArgs {
+  FinArgs f;             // f.p: columns, records, slots (slots[cap], slots[cap + 1]: null key, the empty word)
+  uint32_t* slot_id;     // [cap + 2]
+  uint32_t* row_slot;    // [n]
+  unsigned int* ngroups;
+  uint32_t* special_ids;  // [2]
+  int hot;
+  int sh_vcount[kMaxAggCols], sh_sum[kMaxAggCols], sh_mn[kMaxAggCols], sh_mx[kMaxAggCols];
+  int smem_words;
+};
+
+__device__ __forceinline__ uint32_t cluster_ctas()
+{
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
+// Every thread of the cluster; memory written before is visible after.
+__device__ __forceinline__ void cluster_sync()
+{
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Slot of row r's key, inserted when new (`won`).  At most n + 2 keys go into
+// 2n slots, so every probe sequence ends.
+template <KeyMode M>
+__device__ __forceinline__ uint32_t find_or_insert(const GbPlan& p, int64_t r, uint64_t& word, bool& won)
+{
+  won = false;
+  unsigned long long* s = p.slots;
+  if (M != KeyMode::GEN && !dvalid(p.k.c[0], r)) {
+    word = 0;
+    won  = *static_cast<volatile unsigned long long*>(s + p.cap) == kEmpty && atomicCAS(s + p.cap, kEmpty, 1ull) == kEmpty;
+    return static_cast<uint32_t>(p.cap);
+  }
+  const uint64_t kb = key_bits<M>(p.k, r);
+  if (M == KeyMode::K64 && kb == kEmpty) {  // the empty word itself: a slot of its own
+    word = kb;
+    won  = *static_cast<volatile unsigned long long*>(s + p.cap + 1) == kEmpty &&
+          atomicCAS(s + p.cap + 1, kEmpty, 1ull) == kEmpty;
+    return static_cast<uint32_t>(p.cap + 1);
+  }
+  const uint64_t h = M == KeyMode::GEN ? kb : mix64(kb);
+  word             = M == KeyMode::GEN ? static_cast<uint64_t>(r) : kb;
+  const uint64_t e = M == KeyMode::GEN ? (static_cast<uint64_t>(r) << 32) | static_cast<uint32_t>(h) : kb;
+  uint64_t i       = fastrange(h, p.cap);
+  for (;;) {
+    unsigned long long v = *static_cast<volatile unsigned long long*>(s + i);
+    if (v == kEmpty) {
+      v = atomicCAS(s + i, kEmpty, e);
+      if (v == kEmpty) {
+        won = true;
+        return static_cast<uint32_t>(i);
+      }
+    }
+    if (M == KeyMode::GEN ? (static_cast<uint32_t>(v) == static_cast<uint32_t>(h) &&
+                             keys_equal(p.k, r, p.k, static_cast<int64_t>(v >> 32)))
+                          : v == kb)
+      return static_cast<uint32_t>(i);
+    i = i + 1 == p.cap ? 0 : i + 1;
+  }
+}
+
+// One value of group `id` into its column's records.
+__device__ __forceinline__ void small_accumulate(const SmallArgs& a, uint32_t* sh, int ci, uint32_t id, int64_t r)
+{
+  const ColPlan& c = a.f.p.c[ci];
+  if (c.nullable && !dvalid(c.col, r)) return;
+  const bool hot          = id < static_cast<uint32_t>(a.hot);
+  unsigned long long* rec = c.crec + static_cast<uint64_t>(id) * c.cw;
+  if (c.nullable) {
+    if (hot) atomicAdd(sh + a.sh_vcount[ci] + id, 1u);
+    else red_add(rec + c.off_vcount, 1);
+  }
+  if (!(c.states & (ST_SUM | ST_MIN | ST_MAX))) return;
+  const uint64_t raw = dbits(c.col, r);
+  const bool sgn     = is_signed_int_dev(c.col.type);
+  uint64_t v         = raw;  // integers: sign-extended
+  if (sgn && c.col.width < 8) {
+    const int s8 = 64 - 8 * c.col.width;
+    v            = static_cast<uint64_t>(static_cast<int64_t>(raw << s8) >> s8);
+  }
+  if (c.states & ST_SUM) {
+    uint32_t* sum = sh + a.sh_sum[ci] + id * c.sum_chunks * 4;
+    if (c.fixed) {
+      const double x = c.col.width == 8 ? __longlong_as_double(static_cast<long long>(raw))
+                                        : static_cast<double>(__uint_as_float(static_cast<uint32_t>(raw)));
+      uint64_t m;
+      int s;
+      bool neg;
+      if (fixed_parts(x, m, s, neg)) {
+        const int b = s & 31;
+        if (!hot) add_fixed_chunks(rec + c.off_sum, m, s, neg);
+        else if (m) sh_add_magnitude(sum, c.sum_chunks, s >> 5, m << b, b ? (m >> (64 - b)) : 0, neg);
+      } else if (isnan(x)) {
+        atomicOr(c.special + id, SP_NAN);
+      } else if (isinf(x)) {
+        atomicOr(c.special + id, x > 0 ? SP_PINF : SP_NINF);
+      } else {
+        atomicAdd(c.fb + id, x);
+      }
+    } else if (hot) {
+      const bool neg = sgn && static_cast<int64_t>(v) < 0;
+      sh_add_magnitude(sum, c.sum_chunks, 0, neg ? 0ull - v : v, 0, neg);
+    } else {
+      red_add(rec + c.off_sum, v);
+    }
+  }
+  if (c.states & (ST_MIN | ST_MAX)) {
+    uint64_t o = sgn ? v ^ (1ull << 63) : v;
+    if (c.fixed && c.col.width == 8) o = (raw >> 63) ? ~raw : (raw | (1ull << 63));
+    if (c.fixed && c.col.width == 4) {
+      const uint32_t b = static_cast<uint32_t>(raw);
+      o                = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    }
+    if (hot) {
+      if (c.states & ST_MIN) atomicMax(reinterpret_cast<unsigned long long*>(sh + a.sh_mn[ci]) + id, ~o);
+      if (c.states & ST_MAX) atomicMax(reinterpret_cast<unsigned long long*>(sh + a.sh_mx[ci]) + id, o);
+    } else {
+      if (c.states & ST_MIN) red_max(rec + c.off_mn, ~o);
+      if (c.states & ST_MAX) red_max(rec + c.off_mx, o);
+    }
+  }
+}
+
+// Shared-memory records of one id to its global records.
+__device__ __forceinline__ void small_flush(const SmallArgs& a, const uint32_t* sh, uint32_t id)
+{
+  const uint32_t rows = sh[id];
+  if (rows == 0) return;
+  red_add(const_cast<unsigned long long*>(a.f.rec) + id, rows);
+  for (int ci = 0; ci < a.f.p.ncols; ++ci) {
+    const ColPlan& c = a.f.p.c[ci];
+    if (c.cw == 0) continue;
+    unsigned long long* rec = c.crec + static_cast<uint64_t>(id) * c.cw;
+    if (c.nullable) {
+      const uint32_t vc = sh[a.sh_vcount[ci] + id];
+      if (vc == 0) continue;
+      red_add(rec + c.off_vcount, vc);
+    }
+    if (c.states & ST_SUM) {
+      const uint32_t* sum = sh + a.sh_sum[ci] + id * c.sum_chunks * 4;
+      uint64_t tot        = 0;
+      for (int q = 0; q < c.sum_chunks; ++q) {
+        const uint64_t pos = sum[q * 4 + 0] + (static_cast<uint64_t>(sum[q * 4 + 1]) << 32);
+        const uint64_t neg = sum[q * 4 + 2] + (static_cast<uint64_t>(sum[q * 4 + 3]) << 32);
+        if (!c.fixed) tot += (pos - neg) << (32 * q);
+        else if (pos != neg) red_add(rec + c.off_sum + q, pos - neg);
+      }
+      if (tot) red_add(rec + c.off_sum, tot);
+    }
+    if (c.states & ST_MIN) red_max(rec + c.off_mn, reinterpret_cast<const unsigned long long*>(sh + a.sh_mn[ci])[id]);
+    if (c.states & ST_MAX) red_max(rec + c.off_mx, reinterpret_cast<const unsigned long long*>(sh + a.sh_mx[ci])[id]);
+  }
+}
+
+template <KeyMode M>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_groupby_kernel(const __grid_constant__ SmallArgs a)
+{
+  extern __shared__ __align__(16) uint32_t sh[];  // [hot] row counts, then the columns' arrays
+  constexpr int R      = M == KeyMode::GEN ? 1 : 4;
+  const GbPlan& p      = a.f.p;
+  const int64_t tid    = static_cast<int64_t>(blockIdx.x) * kSmallThreads + threadIdx.x;
+  const int64_t total  = static_cast<int64_t>(cluster_ctas()) * kSmallThreads;
+  const uint32_t lane  = lane_id();
+  unsigned long long* rec0 = const_cast<unsigned long long*>(a.f.rec);
+  // 1. empty slots and pair sets
+  for (int64_t i = tid; i < static_cast<int64_t>(p.cap) + 2; i += total) p.slots[i] = kEmpty;
+  for (int ci = 0; ci < p.ncols; ++ci)
+    if (p.c[ci].states & ST_NDIST)
+      for (int64_t i = tid; i < static_cast<int64_t>(p.c[ci].pair_cap); i += total) p.c[ci].pairs[i] = kEmpty;
+  if (tid == 0) {
+    *a.ngroups       = 0;
+    a.special_ids[0] = kUnsetId;
+    a.special_ids[1] = kUnsetId;
+    *p.overflow      = 0;
+  }
+  for (int i = threadIdx.x; i < a.smem_words; i += kSmallThreads) sh[i] = 0;
+  cluster_sync();
+  // 2. slots; whole warps step together (the winners' ids come from one
+  // atomic per warp and step)
+  for (int64_t base = tid - lane; base < p.n; base += total * R) {
+    uint64_t word[R];
+    uint32_t slot[R];
+    bool won[R];
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int64_t r = base + j * total + lane;
+      won[j]          = false;
+      slot[j]         = 0;
+      if (r < p.n) slot[j] = find_or_insert<M>(p, r, word[j], won[j]);
+      mine += won[j] ? 1u : 0u;
+    }
+    __syncwarp();
+    const uint32_t inc = warp_inclusive_scan(mine);
+    const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+    uint32_t first     = 0;
+    if (all != 0) {
+      if (lane == 31) first = atomicAdd(a.ngroups, all);
+      first = __shfl_sync(0xffffffffu, first, 31);
+    }
+    uint32_t id = first + inc - mine;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int64_t r = base + j * total + lane;
+      if (r < p.n) a.row_slot[r] = slot[j];
+      if (!won[j]) continue;
+      a.slot_id[slot[j]] = id;
+      p.id_key[id]       = word[j];
+      if (M != KeyMode::GEN && slot[j] == p.cap) a.special_ids[0] = id;  // the other special key is its word
+      for (int k = 0; k < p.stride; ++k) rec0[id + k * a.f.ld] = 0;
+      for (int ci = 0; ci < p.ncols; ++ci) {
+        const ColPlan& c = p.c[ci];
+        for (int k = 0; k < c.cw; ++k) c.crec[static_cast<uint64_t>(id) * c.cw + k] = 0;
+        if ((c.states & ST_SUM) && c.fixed) {
+          c.fb[id]      = 0.0;
+          c.special[id] = 0;
+        }
+      }
+      ++id;
+    }
+  }
+  cluster_sync();
+  // 3. accumulate
+  for (int64_t base = tid; base < p.n; base += total * 4) {
+    uint32_t id[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t r = base + j * total;
+      id[j]           = r < p.n ? __ldcg(a.row_slot + r) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) id[j] = base + j * total < p.n ? __ldcg(a.slot_id + id[j]) : kUnsetId;
+    for (int j = 0; j < 4; ++j) {
+      const int64_t r = base + j * total;
+      if (r >= p.n) break;
+      if (id[j] < static_cast<uint32_t>(a.hot)) atomicAdd(sh + id[j], 1u);
+      else red_add(rec0 + id[j], 1);
+      for (int ci = 0; ci < p.ncols; ++ci) {
+        const ColPlan& c = p.c[ci];
+        if (c.cw) small_accumulate(a, sh, ci, id[j], r);
+        if ((c.states & ST_NDIST) && dvalid(c.col, r) && pair_insert(p, c, id[j], r))
+          red_add(rec0 + id[j] + c.off_nd * a.f.ld, 1);
+      }
+    }
+  }
+  __syncthreads();
+  for (uint32_t id = threadIdx.x; id < static_cast<uint32_t>(a.hot); id += kSmallThreads) small_flush(a, sh, id);
+  cluster_sync();
+  // 4. output rows
+  const int64_t groups = __ldcg(a.ngroups);
+  for (int64_t i = tid; i < groups; i += total) finalize_row(a.f, i);
+}
+
+// Rows up to which one cluster takes the whole call: its 16 SMs are still
+// ahead of the general plan there (131,072 rows of one group each: 219 us
+// against 409; of 131 groups 118 against 253).
+constexpr int64_t kSmallGroupbyRows = int64_t(1) << 17;
+
+// False (nothing done): a pair set overflowed its probe limit.
+template <KeyMode M>
+bool small_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const int32_t* keys, int nkeys,
+                   const ldf_aggregation* aggs, int naggs, const std::vector<int>& agg_col, ldf_column* out)
+{
+  const Allocator& al = ctx.alloc();
+  cudaStream_t s      = ctx.stream();
+  const int64_t n     = p.n;
+  layout_records(p);
+  p.cap    = static_cast<uint64_t>(2 * n + 64);
+  p.id_cap = static_cast<uint64_t>(n);
+  // one scratch allocation, carved in 256-byte steps
+  size_t bytes = 0;
+  auto carve   = [&](size_t b) {
+    const size_t o = bytes;
+    bytes += (b + 255) & ~size_t(255);
+    return o;
+  };
+  const size_t o_slots = carve((p.cap + 2) * 8), o_sid = carve((p.cap + 2) * 4), o_rows = carve(n * 4);
+  const size_t o_key = carve(n * 8), o_rec = carve(n * 8 * p.stride), o_misc = carve(256);
+  size_t o_col[kMaxAggCols], o_fb[kMaxAggCols], o_sp[kMaxAggCols], o_pairs[kMaxAggCols];
+  for (int ci = 0; ci < p.ncols; ++ci) {
+    ColPlan& c  = p.c[ci];
+    c.pair_cap  = (c.states & ST_NDIST) ? static_cast<uint64_t>(2 * n + 64) : 0;
+    o_col[ci]   = carve(n * 8 * c.cw);
+    o_fb[ci]    = carve((c.states & ST_SUM) && c.fixed ? n * 8 : 0);
+    o_sp[ci]    = carve((c.states & ST_SUM) && c.fixed ? n * 4 : 0);
+    o_pairs[ci] = carve(c.pair_cap * 8);
+  }
+  Buffer<uint8_t> scratch(al, bytes);
+  uint8_t* base = scratch.get();
+  p.slots       = reinterpret_cast<unsigned long long*>(base + o_slots);
+  p.id_key      = reinterpret_cast<unsigned long long*>(base + o_key);
+  unsigned int* misc = reinterpret_cast<unsigned int*>(base + o_misc);
+  p.overflow         = reinterpret_cast<int*>(misc + 1);
+  SmallArgs a{};
+  a.slot_id     = reinterpret_cast<uint32_t*>(base + o_sid);
+  a.row_slot    = reinterpret_cast<uint32_t*>(base + o_rows);
+  a.ngroups     = misc;
+  a.special_ids = misc + 2;
+  // shared-memory records of the lowest ids
+  int per = 4;
+  for (int ci = 0; ci < p.ncols; ++ci) {
+    ColPlan& c = p.c[ci];
+    c.crec     = reinterpret_cast<unsigned long long*>(base + o_col[ci]);
+    c.fb       = reinterpret_cast<double*>(base + o_fb[ci]);
+    c.special  = reinterpret_cast<unsigned int*>(base + o_sp[ci]);
+    c.pairs    = reinterpret_cast<unsigned long long*>(base + o_pairs[ci]);
+    per += (c.nullable ? 4 : 0) + ((c.states & ST_SUM) ? 16 * c.sum_chunks : 0) + ((c.states & ST_MIN) ? 8 : 0) +
+           ((c.states & ST_MAX) ? 8 : 0);
+  }
+  a.hot     = static_cast<int>(std::min<int64_t>(n, std::min(kSmallHot, (200 * 1024) / per)));
+  int words = (a.hot + 3) & ~3;
+  auto take = [&](bool on, int w) {
+    const int o = words;
+    if (on) words += (w * a.hot + 3) & ~3;
+    return o;
+  };
+  for (int ci = 0; ci < p.ncols; ++ci) {
+    const ColPlan& c = p.c[ci];
+    a.sh_mn[ci]      = take(c.states & ST_MIN, 2);
+    a.sh_mx[ci]      = take(c.states & ST_MAX, 2);
+    a.sh_sum[ci]     = take(c.states & ST_SUM, 4 * c.sum_chunks);
+    a.sh_vcount[ci]  = take(c.nullable, 1);
+  }
+  a.smem_words      = words;
+  const size_t smem = static_cast<size_t>(words) * 4;
+  a.f.p             = p;
+  a.f.rec           = reinterpret_cast<unsigned long long*>(base + o_rec);
+  a.f.ld            = static_cast<uint64_t>(n);
+  a.f.key_mode      = static_cast<int>(M);
+  a.f.special_ids   = a.special_ids;
+  Buffer<int32_t> repr;
+  bind_outputs(al, table, keys, nkeys, aggs, naggs, agg_col, M == KeyMode::GEN, n, out, a.f, repr);
+  // up to 16 CTAs (the largest cluster), about four rows a thread
+  unsigned ctas = 1;
+  while (ctas < 16 && static_cast<int64_t>(ctas) * kSmallThreads * 2 < n) ctas *= 2;
+  LDF_CUDA(cudaFuncSetAttribute(small_groupby_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024));
+  LDF_CUDA(cudaFuncSetAttribute(small_groupby_kernel<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  launch_cluster("small_groupby", small_groupby_kernel<M>, ctas, kSmallThreads, smem, s, a);
+  unsigned int h[2] = {0, 0};  // groups, overflow
+  ctx.fetch(h, misc, sizeof(h));
+  ctx.finish();
+  if (h[1] != 0) {
+    for (int j = 0; j < nkeys + naggs; ++j) free_out_column(al, out[j]);
+    return false;
+  }
+  const int64_t G = h[0];
+  for (int j = 0; j < nkeys + naggs; ++j) out[j].size = G;
+  bool strings = false;
+  for (int j = 0; j < nkeys; ++j)
+    if (table[keys[j]].type == LDF_STRING) {
+      gather_strings(ctx, make_dcol(table[keys[j]]), repr.get(), G, out[j]);
+      strings = true;
+    }
+  if (strings) ctx.finish();
+  return true;
 }
 
 template <KeyMode M>
@@ -1548,7 +2048,7 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
       launch("freq_stats", freq_stats_kernel, gs_blocks(pc.pair_cap, 256), 256, 0, s, spcounts.get(),
              static_cast<int64_t>(pc.pair_cap), stats.get() + 2);
     unsigned long long h[4];
-    LDF_CUDA(cudaMemcpyAsync(h, stats.get(), 32, cudaMemcpyDeviceToHost, s));
+    ctx.fetch(h, stats.get(), 32);
     ctx.finish();
     // GEE (Charikar et al. 2000) for the groups, taken x4 below because it
     // underestimates heavy tails (a table that turns out too small overflows
@@ -1569,23 +2069,7 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
   uint64_t pair_cap = static_cast<uint64_t>(std::max<int64_t>(est_pairs + est_pairs / 2, 64));
 
   // ---- record layout and shared-memory hot set -------------------------------
-  int w = 1;  // shared record: count_all, then the distinct counts
-  for (int ci = 0; ci < p.ncols; ++ci) {
-    ColPlan& c   = p.c[ci];
-    c.sum_chunks = c.fixed ? kSumChunks : 2;
-    c.mm64       = type_width(c.col.type) > 4 ? 1 : 0;
-    int cw       = 0;  // the column block
-    c.off_vcount = c.nullable ? cw++ : 0;
-    if (c.states & ST_SUM) {
-      c.off_sum = cw;
-      cw += c.fixed ? kSumChunks : 1;
-    }
-    if (c.states & ST_MIN) c.off_mn = cw++;
-    if (c.states & ST_MAX) c.off_mx = cw++;
-    c.cw = cw;
-    if (c.states & ST_NDIST) c.off_nd = w++;
-  }
-  p.stride = w;
+  layout_records(p);
   const int kSmemBudget = 96 * 1024;
   LDF_CUDA(cudaFuncSetAttribute(assign_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
   int hot_limit = 1 << 30;
@@ -1607,7 +2091,9 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
   }
 
   for (int attempt = 0;; ++attempt) {
-    const uint64_t id_cap = cap + kIdFirst;
+    // ids: at most one per slot, and what the warps' pools leave unused
+    const uint64_t id_cap = cap + kIdFirst +
+                            static_cast<uint64_t>(std::min<int64_t>(n, int64_t(64) * 32 * num_sms()));
     const int sw          = M == KeyMode::K32 ? 1 : 2;
     Buffer<unsigned long long> slots(al, cap * sw);
     Buffer<unsigned long long> counts(al, id_cap);  // rows per assign-pass id
@@ -1673,9 +2159,13 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
       const int64_t ablocks = std::min<int64_t>(static_cast<int64_t>(num_sms()) * std::max(occ, 1),
                                                 ceil_div(n, int64_t(kGbThreads) * assign_rows<M>()));
       wait_keys();
+      const int64_t seed = std::min<int64_t>(n, kSeedRows);
+      launch("seed_keys", seed_keys_kernel<M>,
+             static_cast<unsigned>(ceil_div(seed, int64_t(kGbThreads) * assign_rows<M>())), kGbThreads, 0, s, pa, seed,
+             n / seed);
       launch("assign", assign_kernel<M>, static_cast<unsigned>(ablocks), kGbThreads, a_smem, s, pa, gid.get());
       unsigned long long hm[2];
-      LDF_CUDA(cudaMemcpyAsync(hm, misc.get(), 16, cudaMemcpyDeviceToHost, s));
+      ctx.fetch(hm, misc.get(), 16);
       ctx.finish();
       if (static_cast<int>(hm[1]) != 0) {
         if (attempt >= 4) fail(LDF_ERR_INTERNAL, "groupby hash table overflow");
@@ -1816,8 +2306,8 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
           }
           unsigned int hv[2];
           int64_t tier[kSegTiers];
-          LDF_CUDA(cudaMemcpyAsync(hv, vr, 8, cudaMemcpyDeviceToHost, s));
-          LDF_CUDA(cudaMemcpyAsync(tier, tb.get(), sizeof(tier), cudaMemcpyDeviceToHost, s));
+          ctx.fetch(hv, vr, 8);
+          ctx.fetch(tier, tb.get(), sizeof(tier));
           ctx.finish();
           Buffer<uint32_t> bits;
           if (hv[0] <= hv[1] && bitmap_budget > 0) {
@@ -1852,9 +2342,9 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
             exclusive_scan_i64(reinterpret_cast<const int64_t*>(rec.get() + hb),
                                reinterpret_cast<int64_t*>(seg_start.get()), T, seg_total.get(), ctx);
             int64_t hv2[2] = {0, 0};  // total rows of ranks >= hb, rows of ranks [hb, s0)
-            LDF_CUDA(cudaMemcpyAsync(&hv2[0], seg_total.get(), 8, cudaMemcpyDeviceToHost, s));
+            ctx.fetch(&hv2[0], seg_total.get(), 8);
             if (s0 < nid)
-              LDF_CUDA(cudaMemcpyAsync(&hv2[1], seg_start.get() + (s0 - hb), 8, cudaMemcpyDeviceToHost, s));
+              ctx.fetch(&hv2[1], seg_start.get() + (s0 - hb), 8);
             ctx.finish();
             const int64_t total = hv2[0];
             pair_rows           = s0 < nid ? hv2[1] : total;
@@ -1921,7 +2411,7 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
           if (p.c[ci].states & ST_NDIST) nunique_pass(ci);
       }
       if (ndist_col >= 0) {  // only pair-set inserts can overflow after the assign pass
-        LDF_CUDA(cudaMemcpyAsync(hm, misc.get(), 16, cudaMemcpyDeviceToHost, s));
+        ctx.fetch(hm, misc.get(), 16);
         ctx.finish();
       }
       if (ndist_col >= 0 && static_cast<int>(hm[1]) != 0) {  // the pair set overflowed
@@ -1951,29 +2441,8 @@ void run_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const 
     f.key_mode = static_cast<int>(M);
     f.groups   = groups.get();
     f.ngroups  = G;
-    f.nkeys    = nkeys;
-    for (int j = 0; j < nkeys; ++j) {
-      const ldf_column& kc = table[keys[j]];
-      out[j]               = alloc_out_column(al, kc.type, G, kc.valid != nullptr);
-      f.key_dst[j]         = OCol{out[j].data, out[j].valid, kc.type, type_width(kc.type)};
-    }
     Buffer<int32_t> repr;
-    if (M == KeyMode::GEN) {
-      repr   = Buffer<int32_t>(al, std::max<int64_t>(G, 1));
-      f.repr = repr.get();
-    }
-    f.nagg = naggs;
-    for (int a = 0; a < naggs; ++a) {
-      const ldf_aggregation& ag = aggs[a];
-      const bool nullable       = !(ag.kind == LDF_AGG_COUNT_ALL || ag.kind == LDF_AGG_COUNT_DISTINCT);
-      out[nkeys + a]            = alloc_out_column(al, ag.out_type, G, nullable);
-      AggOut& o                 = f.a[a];
-      o.kind                    = ag.kind;
-      o.count_mode              = ag.count_mode;
-      o.col                     = agg_col[a];
-      o.in_type                 = ag.kind == LDF_AGG_COUNT_ALL ? LDF_INT64 : table[ag.in_col].type;
-      o.dst = OCol{out[nkeys + a].data, out[nkeys + a].valid, ag.out_type, type_width(ag.out_type)};
-    }
+    bind_outputs(al, table, keys, nkeys, aggs, naggs, agg_col, M == KeyMode::GEN, G, out, f, repr);
     if (G > 0) launch("finalize", finalize_kernel, gs_blocks(G, 256), 256, 0, s, f);
     for (int j = 0; j < nkeys; ++j)
       if (table[keys[j]].type == LDF_STRING) gather_strings(ctx, make_dcol(table[keys[j]]), repr.get(), G, out[j]);
@@ -3264,6 +3733,13 @@ void groupby_aggregation(const ldf_column* table, int ncols, const int32_t* keys
       fail(LDF_ERR_UNSUPPORTED, "min/max of a string column is not supported");
   }
   if (try_partitioned(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out, hs, col_of_plan)) return;
+  if (n > 0 && n <= kSmallGroupbyRows && hs.staged_bytes() == 0) {
+    const KeyMode m = key_mode(k);
+    if (m == KeyMode::K32 ? small_groupby<KeyMode::K32>(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out)
+        : m == KeyMode::K64 ? small_groupby<KeyMode::K64>(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out)
+                            : small_groupby<KeyMode::GEN>(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out))
+      return;
+  }
   switch (key_mode(k)) {
     case KeyMode::K32:
       run_groupby<KeyMode::K32>(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out, hs, col_of_plan);
