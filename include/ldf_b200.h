@@ -196,6 +196,15 @@ int ldf_b200_arrow_bits_to_bytes(const uint8_t* bits, int64_t bit_offset, int64_
 int ldf_b200_arrow_offsets_to_ranges(const void* offsets, int32_t offset_bytes, int64_t n,
                                      ldf_range* ranges, void* stream);
 
+/* ---- file bytes -> pinned host memory -> device ---------------------------- */
+/* The first `nbytes` bytes of the file at `path` read into `host` (pinned) by
+ * several threads, each piece copied to `dev` on `stream` as soon as it has
+ * been read; the copies are complete when the call returns.  *os_error: 0, or
+ * the errno of the read that failed (the call itself then still returns
+ * LDF_OK). */
+int ldf_b200_read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, int32_t* os_error,
+                       void* stream);
+
 /* ---- CSV text -> columns, parsed on the device --------------------------- */
 /* Replaces cudf::io::read_csv in CSVRead::gpu_variant (csv.cu:53-139) with
  * the conversions of the reference's Arrow reader (CSVRead::cpu_variant,

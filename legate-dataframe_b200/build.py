@@ -35,6 +35,7 @@ SOURCES = [
     "distinct.cu",
     "ingest.cu",
     "csv.cu",
+    "file_read.cu",
     "parquet.cu",
 ]
 

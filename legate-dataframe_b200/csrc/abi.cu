@@ -17,6 +17,7 @@ void distinct(const ldf_column* table, int ncols, const int32_t* keys, int nkeys
               const OpContext& ctx);
 void arrow_bits_to_bytes(const uint8_t* bits, int64_t bit_offset, int64_t n, uint8_t* out, cudaStream_t s);
 void arrow_offsets_to_ranges(const void* offsets, int offset_bytes, int64_t n, ldf_range* out, cudaStream_t s);
+int read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, cudaStream_t s);
 void csv_read(const uint8_t* text, int64_t n, char delimiter, int skip_first, const int32_t* fields,
               const int32_t* types, int ncols, const char* nulls, int nulls_bytes, int n_nulls, ldf_column* out,
               int64_t* nrows, const OpContext& ctx);
@@ -146,6 +147,14 @@ int ldf_b200_arrow_offsets_to_ranges(const void* offsets, int32_t offset_bytes, 
 {
   return guarded([&] {
     ldf::arrow_offsets_to_ranges(offsets, offset_bytes, n, ranges, static_cast<cudaStream_t>(stream));
+  });
+}
+
+int ldf_b200_read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, int32_t* os_error, void* stream)
+{
+  return guarded([&] {
+    LDF_REQUIRE(os_error != nullptr, "read_file: null argument");
+    *os_error = ldf::read_file(path, nbytes, host, dev, static_cast<cudaStream_t>(stream));
   });
 }
 

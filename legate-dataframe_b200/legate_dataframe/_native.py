@@ -162,6 +162,10 @@ def lib():
             ]
             L.ldf_b200_test_stalled_lookback.argtypes = [ctypes.c_uint32, P(ldf_allocator), ctypes.c_void_p]
             L.ldf_b200_test_stalled_lookback.restype = ctypes.c_int
+            L.ldf_b200_read_file.argtypes = [
+                ctypes.c_char_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, i32p, ctypes.c_void_p,
+            ]
+            L.ldf_b200_read_file.restype = ctypes.c_int
             L.ldf_b200_csv_read.argtypes = [
                 ctypes.c_void_p, ctypes.c_int64, ctypes.c_char, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32),
                 ctypes.POINTER(ctypes.c_int32), ctypes.c_int32, ctypes.c_char_p, ctypes.c_int32, ctypes.c_int32,

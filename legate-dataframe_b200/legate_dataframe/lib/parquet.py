@@ -19,7 +19,6 @@ import ctypes
 import glob
 import os
 import pathlib
-from concurrent.futures import ThreadPoolExecutor, as_completed
 
 import numpy as np
 import pyarrow as pa
@@ -38,38 +37,18 @@ def _file_list(files) -> list[str]:
     return [str(f) for f in files]
 
 
-_READ_PIECE = 64 << 20  # bytes per read (and per host-to-device copy) of a large file
-
-
 def _file_to_device(path, dev) -> tuple[torch.Tensor, torch.Tensor, int]:
-    """The file's bytes in pinned host memory and on the device.  Large files
-    are read in 64 MB pieces by a few threads, each piece copied to the device
-    as soon as it has been read, so the reads and the copies overlap."""
+    """The file's bytes in pinned host memory and on the device, read by
+    several threads with each piece's copy queued as soon as it has been read
+    (ldf_b200_read_file)."""
     size = os.path.getsize(path)
     host = torch.empty(max(size, 16), dtype=torch.uint8, pin_memory=True)
     text = torch.empty(max(size, 16), dtype=torch.uint8, device=dev)
-    if size == 0:
-        return host, text, 0
-    mv = memoryview(host.numpy())
-    pieces = [(a, min(a + _READ_PIECE, size)) for a in range(0, size, _READ_PIECE)]
-
-    def read(piece):
-        a, b = piece
-        with open(path, "rb") as f:
-            f.seek(a)
-            got = f.readinto(mv[a:b])
-        if got != b - a:
-            raise OSError(f"short read of {path}")
-        return piece
-
-    if len(pieces) == 1:
-        read(pieces[0])
-        text[:size].copy_(host[:size], non_blocking=True)
-    else:
-        with ThreadPoolExecutor(max_workers=min(8, len(pieces))) as ex:
-            for fut in as_completed([ex.submit(read, pc) for pc in pieces]):
-                a, b = fut.result()
-                text[a:b].copy_(host[a:b], non_blocking=True)
+    err = ctypes.c_int32(0)
+    N.check(N.lib().ldf_b200_read_file(os.fsencode(path), size, host.data_ptr(), text.data_ptr(), ctypes.byref(err),
+                                       ctypes.c_void_p(N.current_stream_handle())))
+    if err.value:
+        raise OSError(err.value, os.strerror(err.value), os.fspath(path))
     return host, text, size
 
 
