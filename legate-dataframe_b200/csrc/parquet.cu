@@ -238,35 +238,24 @@ __device__ void snap_stage(SnapStage& st, SnapShared& sh, int64_t i, bool sizes)
   if (sizes) snap_sizes(st, sh);
 }
 
-// src[0, n) -> dst (at most cap bytes) by the calling warp; false when the
-// stream is malformed.  The stream is a chain of elements (literals and
-// back-references) whose boundaries are known only by parsing them in turn.
-// Per batch of up to kSnapBatch short elements: the warp walks the chain
-// through size[] (one shared load per element; the sizes of every staged
-// position were tabulated in parallel), each lane decodes one element, and
-// the batch's output bytes are produced all at once: byte r of the batch is
-// a literal's input byte, or a back-reference's source byte -- at
-// out[o - d + k % d] for byte k of a copy of offset d -- followed back
+// Elements of the stream from index i on, decoded by the calling warp until
+// output byte `total` (output bytes before `o` exist; copies may not reach
+// before `floor`); false when the stream is malformed.  The stream is a chain
+// of elements (literals and back-references) whose boundaries are known only
+// by parsing them in turn.  Per batch of up to kSnapBatch short elements: the
+// warp walks the chain through size[] (one shared load per element; the sizes
+// of every staged position were tabulated in parallel), each lane decodes one
+// element, and the batch's output bytes are produced all at once: byte r of
+// the batch is a literal's input byte, or a back-reference's source byte --
+// at out[o - d + k % d] for byte k of a copy of offset d -- followed back
 // through the batch until it reaches a literal or output written before the
 // batch (ring or global).  Long literals are copied on their own.
-__device__ bool snappy_warp(const uint8_t* src, int64_t n, uint8_t* dst, int64_t cap, int64_t& produced,
-                            SnapShared& sh)
+__device__ bool snappy_run(SnapStage& st, SnapShared& sh, uint8_t* dst, int64_t& i, int64_t& o, const int64_t total,
+                           const int64_t floor)
 {
-  const int lane = threadIdx.x % kLanes;
-  SnapStage st{src, n, 0, false};
-  snap_stage(st, sh, 0, false);
-  int64_t i    = 0;
-  uint64_t len = 0;
-  for (int sh_ = 0;; sh_ += 7) {  // preamble: the uncompressed length as a varint
-    if (i >= n || sh_ > 35) return false;
-    const uint8_t b = sh.in[i++ - st.ib];
-    len |= static_cast<uint64_t>(b & 0x7f) << sh_;
-    if (!(b & 0x80)) break;
-  }
-  if (len > static_cast<uint64_t>(cap)) return false;
-  const int64_t total = static_cast<int64_t>(len);
+  const int lane          = threadIdx.x % kLanes;
+  const int64_t n         = st.n;
   constexpr int64_t kMask = kSnapWin - 1;
-  int64_t o = 0;
   while (o < total) {
     if (i >= n) return false;
     if (i + 5 > st.ib + kSnapIn) snap_stage(st, sh, i, true);  // a tag and its extra bytes
@@ -322,7 +311,7 @@ __device__ bool snappy_warp(const uint8_t* src, int64_t n, uint8_t* dst, int64_t
         const int fl    = sh.flags[lane];
         const bool end  = at >= total;
         stop            = end || !(fl & 2) || rs + lj > kSnapBatchBytes;
-        bad             = !end && ((fl & 1) || at + lj > total || (sh.src[lane] < 0 && sh.off[lane] > at));
+        bad             = !end && ((fl & 1) || at + lj > total || (sh.src[lane] < 0 && sh.off[lane] > at - floor));
       }
       const unsigned sm = __ballot_sync(0xffffffffu, stop), bm = __ballot_sync(0xffffffffu, bad);
       cut       = sm ? __ffs(sm) - 1 : nb;
@@ -337,7 +326,7 @@ __device__ bool snappy_warp(const uint8_t* src, int64_t n, uint8_t* dst, int64_t
         const int fl     = sh.flags[j];
         const bool end   = at >= total;
         const bool stop  = end || !(fl & 2) || rs + lj > kSnapBatchBytes;
-        const bool bad   = !end && ((fl & 1) || at + lj > total || (sh.src[j] < 0 && sh.off[j] > at));
+        const bool bad   = !end && ((fl & 1) || at + lj > total || (sh.src[j] < 0 && sh.off[j] > at - floor));
         if (stop) atomicMin(&sh.cut, j);
         if (bad) atomicMin(&sh.bad, j);
       }
@@ -460,6 +449,28 @@ __device__ bool snappy_warp(const uint8_t* src, int64_t n, uint8_t* dst, int64_t
     i = st.ib + (cut < nb ? sh.epos[cut] : walk_end);
     __syncwarp();  // the next batch reads these bytes and rewrites the descriptors
   }
+  return true;
+}
+
+// src[0, n) -> dst (at most cap bytes) by the calling warp; false when the
+// stream is malformed.
+__device__ bool snappy_warp(const uint8_t* src, int64_t n, uint8_t* dst, int64_t cap, int64_t& produced,
+                            SnapShared& sh)
+{
+  SnapStage st{src, n, 0, false};
+  snap_stage(st, sh, 0, false);
+  int64_t i    = 0;
+  uint64_t len = 0;
+  for (int sh_ = 0;; sh_ += 7) {  // preamble: the uncompressed length as a varint
+    if (i >= n || sh_ > 35) return false;
+    const uint8_t b = sh.in[i++ - st.ib];
+    len |= static_cast<uint64_t>(b & 0x7f) << sh_;
+    if (!(b & 0x80)) break;
+  }
+  if (len > static_cast<uint64_t>(cap)) return false;
+  const int64_t total = static_cast<int64_t>(len);
+  int64_t o           = 0;
+  if (!snappy_run(st, sh, dst, i, o, total, 0)) return false;
   produced = o;
   return true;
 }
@@ -1274,6 +1285,276 @@ unsigned pq_blocks(int64_t work, int threads)
   return static_cast<unsigned>(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// ---- Snappy pages of several fragments --------------------------------------
+// Snappy compressors work on 64 KB of input at a time: no element crosses a
+// multiple of kFragBytes of output and no copy reaches back over one.  The
+// format does not demand it, so a page that breaks it (or is malformed) is
+// decoded again by the per-page kernels.  A page of several fragments is
+// decoded a warp per fragment:
+//  1. snap_exits: the stream in segments of kFragSeg bytes; for every position
+//     of a segment, read as a tag, where the elements from there on leave the
+//     segment and how many bytes they put out (pointer jumping in shared
+//     memory, each entry one 64-bit word, so that any mix of rounds a thread
+//     sees is a valid jump);
+//  2. snap_starts: one thread per page follows the exits, a step per segment,
+//     and notes where to start for each fragment: the last segment entry at
+//     or before it;
+//  3. snap_fragment: one warp per fragment skips to its first element and
+//     decodes it (snappy_run).
+// A page as one warp's work took 19 ms for 1 MB pages of int64 and float32
+// values (4M rows of three columns).
+constexpr int64_t kFragBytes    = 65536;
+constexpr int kFragSeg          = 4096;
+constexpr int kExitThreads      = 256;
+constexpr int64_t kFragMaxInput = int64_t(64) << 20;  // stream bytes per round (8 bytes of exits each)
+
+struct FragPage {
+  int page;
+  int nfrag;
+  int64_t file_off;  // file offset of the stream (behind a v2 page's levels)
+  int64_t n, u;      // stream bytes, output bytes
+  int64_t lv;        // v2 levels in front of the stream (copied as they are)
+  int64_t exit0;     // first of its exits (n entries)
+  int64_t seg0;      // first of its segments
+  int64_t frag0;     // first of its fragments
+  uint8_t* dst;      // output (levels included)
+};
+struct FragStart {
+  int64_t pos, out;  // stream index and output position to start from; pos < 0: none
+};
+
+__device__ __forceinline__ int frag_page_of(const FragPage* fp, int n, int64_t g, int64_t FragPage::*base)
+{
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (fp[mid].*base <= g) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(kExitThreads) snap_exits_kernel(const uint8_t* file, const FragPage* fp, int npages,
+                                                                  unsigned long long* exits)
+{
+  // entry: (next position relative to the segment, output bytes up to it)
+  __shared__ unsigned long long e[kFragSeg];
+  __shared__ uint8_t in[kFragSeg + 8];
+  const FragPage& f  = fp[frag_page_of(fp, npages, blockIdx.x, &FragPage::seg0)];
+  const int64_t s0   = (static_cast<int64_t>(blockIdx.x) - f.seg0) * kFragSeg;
+  const int m        = static_cast<int>(f.n - s0 < kFragSeg ? f.n - s0 : kFragSeg);
+  const uint8_t* src = file + f.file_off + s0;
+  for (int x = threadIdx.x; x < kFragSeg + 8; x += kExitThreads) in[x] = s0 + x < f.n ? src[x] : 0;
+  __syncthreads();
+  for (int x = threadIdx.x; x < m; x += kExitThreads) {
+    const uint32_t t = in[x];
+    uint64_t size, out;
+    if ((t & 3) != 0) {
+      size = (t & 3) == 1 ? 2 : ((t & 3) == 2 ? 3 : 5);
+      out  = (t & 3) == 1 ? 4 + ((t >> 2) & 7) : (t >> 2) + 1;
+    } else {
+      out     = (t >> 2) + 1;
+      int hdr = 1;
+      if (out > 60) {
+        const int nb = static_cast<int>(out) - 60;
+        out          = static_cast<uint64_t>(le_bytes(in + x + 1, nb)) + 1;
+        hdr += nb;
+      }
+      size = hdr + out;
+    }
+    const uint64_t nxt = x + size < 0xffffffffull ? x + size : 0xffffffffull;
+    e[x]               = nxt << 32 | (out < 0xffffffffull ? out : 0xffffffffull);
+  }
+  int more;
+  do {
+    __syncthreads();
+    more = 0;
+    for (int x = threadIdx.x; x < m; x += kExitThreads) {
+      const unsigned long long v = e[x];
+      const uint32_t nxt         = static_cast<uint32_t>(v >> 32);
+      if (nxt >= static_cast<uint32_t>(m)) continue;
+      const unsigned long long w = *static_cast<volatile unsigned long long*>(e + nxt);
+      e[x] = (w & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(v) + static_cast<uint32_t>(w));
+      more = 1;
+    }
+  } while (__syncthreads_or(more));
+  for (int x = threadIdx.x; x < m; x += kExitThreads) exits[f.exit0 + s0 + x] = e[x];
+}
+
+__global__ void snap_starts_kernel(const uint8_t* file, const FragPage* fp, const unsigned long long* exits,
+                                   FragStart* starts, int* redo)
+{
+  const FragPage f = fp[blockIdx.x];
+  if (threadIdx.x != 0) return;
+  const uint8_t* b = file + f.file_off;
+  int64_t pos = -1, i = 0, out = 0;
+  uint64_t len = 0;
+  for (int sh = 0; sh <= 35 && i < f.n; sh += 7) {
+    const uint8_t v = b[i++];
+    len |= static_cast<uint64_t>(v & 0x7f) << sh;
+    if (!(v & 0x80)) {
+      pos = i;
+      break;
+    }
+  }
+  int k = 0;
+  if (pos >= 0 && len == static_cast<uint64_t>(f.u)) {
+    while (pos < f.n && out < f.u) {
+      const unsigned long long e = exits[f.exit0 + pos];
+      const int64_t next         = pos / kFragSeg * kFragSeg + static_cast<int64_t>(e >> 32);
+      const int64_t after        = out + static_cast<int64_t>(e & 0xffffffffull);
+      while (k < f.nfrag && k * kFragBytes < after) starts[f.frag0 + k++] = FragStart{pos, out};
+      pos = next;
+      out = after;
+    }
+  }
+  if (pos != f.n || out != f.u) redo[blockIdx.x] = 1;
+  for (; k < f.nfrag; ++k) starts[f.frag0 + k] = FragStart{-1, 0};
+}
+
+__global__ void __launch_bounds__(kLanes) snap_fragment_kernel(const uint8_t* file, const FragPage* fp, int npages,
+                                                              const FragStart* starts, int* redo)
+{
+  __shared__ SnapShared sh;
+  const int q       = frag_page_of(fp, npages, blockIdx.x, &FragPage::frag0);
+  const FragPage& f = fp[q];
+  const int lane    = threadIdx.x;
+  const int64_t k   = static_cast<int64_t>(blockIdx.x) - f.frag0;
+  if (k == 0)
+    for (int64_t x = lane; x < f.lv; x += kLanes) f.dst[x] = file[f.file_off - f.lv + x];
+  const FragStart fs = starts[blockIdx.x];
+  if (fs.pos < 0) return;
+  const int64_t from = k * kFragBytes;
+  const int64_t to   = from + kFragBytes < f.u ? from + kFragBytes : f.u;
+  SnapStage st{file + f.file_off, f.n, 0, false};
+  int64_t i = fs.pos, o = fs.out;
+  snap_stage(st, sh, i, true);
+  bool ok = true;
+  while (ok && o < from) {  // skip whole elements up to the fragment
+    if (i >= f.n) {
+      ok = false;
+      break;
+    }
+    if (i + 5 > st.ib + kSnapIn) snap_stage(st, sh, i, true);
+    int nb = 0, r = static_cast<int>(i - st.ib);
+    while (nb < kLanes && st.ib + r < f.n && r + 5 <= kSnapIn) {
+      if (lane == 0) sh.epos[nb] = r;
+      ++nb;
+      r += sh.size[r];
+    }
+    __syncwarp();
+    int64_t l = 0, size = 0;
+    if (lane < nb) {
+      const SnapElem e = snap_at(sh, sh.epos[lane]);
+      l                = e.l;
+      size             = e.hdr + (e.literal ? e.l : 0);
+    }
+    const int64_t lend = warp_inclusive_scan(l), send = warp_inclusive_scan(size);
+    const unsigned in  = __ballot_sync(0xffffffffu, lane < nb && o + lend <= from);
+    const int taken    = __popc(in);
+    if (taken == 0) {
+      ok = false;  // an element that crosses into the fragment
+      break;
+    }
+    o += __shfl_sync(0xffffffffu, lend, taken - 1);
+    i += __shfl_sync(0xffffffffu, send, taken - 1);
+    __syncwarp();
+  }
+  if (ok) {
+    if (i < st.ib || i + 5 > st.ib + kSnapIn) snap_stage(st, sh, i < f.n ? i : f.n, true);
+    ok = snappy_run(st, sh, f.dst + f.lv, i, o, to, from) && o == to;
+  }
+  if (!ok && lane == 0) redo[q] = 1;
+}
+
+// Snappy pages of byte arrays that are not made of fragments, decoded by the
+// whole GPU through their element chains (chain_*); their outputs (returned)
+// replace the pages' data in dev_pages.
+Buffer<uint8_t> decode_chain_pages(const OpContext& ctx, const uint8_t* file, const ldf_parquet_page* pages,
+                                   const std::vector<int>& chain, int64_t chain_in, std::vector<PqPage>& dev_pages,
+                                   unsigned long long* err)
+{
+  const Allocator& al = ctx.alloc();
+  cudaStream_t s      = ctx.stream();
+  std::vector<ChainPage> cpages;
+  std::vector<int64_t> in_b, out_b, el_b, ck_b, cbases;  // cbases: in | out | elem | ck, one entry per page each
+  int64_t chain_elems = 0, chain_cks = 0, chain_out = 0, chain_maxu = 1, in_run = 0;
+  for (int p : chain) {
+    const ldf_parquet_page& h = pages[p];
+    const int64_t lv          = h.kind == LDF_PQ_DATA_V2 ? h.levels_bytes : 0;
+    ChainPage c{};
+    c.page     = p;
+    c.file_off = h.offset + lv;
+    c.n        = h.compressed - lv;
+    c.lv       = lv;
+    c.u        = h.uncompressed - lv;
+    c.elem_cap = c.n / 2 + 1;
+    c.ck_cap   = c.elem_cap / kChainStep + 2;
+    in_b.push_back(in_run);
+    out_b.push_back(chain_out);
+    el_b.push_back(chain_elems);
+    ck_b.push_back(chain_cks);
+    in_run += c.n;
+    chain_elems += c.elem_cap;
+    chain_cks += c.ck_cap;
+    chain_maxu = std::max(chain_maxu, h.uncompressed);
+    chain_out += (h.uncompressed + 15) & ~int64_t(15);
+    cpages.push_back(c);
+  }
+  for (auto* v : {&in_b, &out_b, &el_b, &ck_b}) cbases.insert(cbases.end(), v->begin(), v->end());
+  Buffer<uint8_t> scratch(al, chain_out);
+  for (size_t q = 0; q < chain.size(); ++q) dev_pages[chain[q]].data = scratch.get() + out_b[q];
+  const int nc          = static_cast<int>(chain.size());
+  const int64_t cin     = chain_in;
+  Buffer<ChainPage> d_cp(al, nc);
+  Buffer<ChainState> d_st(al, nc);
+  Buffer<int64_t> d_cb(al, cbases.size());
+  LDF_CUDA(cudaMemcpyAsync(d_cp.get(), cpages.data(), nc * sizeof(ChainPage), cudaMemcpyHostToDevice, s));
+  LDF_CUDA(cudaMemcpyAsync(d_cb.get(), cbases.data(), cbases.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+  const ChainBases B{d_cb.get(), d_cb.get() + nc, d_cb.get() + 2 * nc, d_cb.get() + 3 * nc, nc};
+  Buffer<int64_t> j0(al, cin), j1(al, cin), j2(al, cin);
+  launch("chain_start", chain_start_kernel, pq_blocks(nc, 128), 128, 0, s, file,
+         static_cast<const ChainPage*>(d_cp.get()), d_st.get(), nc, err);
+  launch("chain_next", chain_next_kernel, pq_blocks(cin, 256), 256, 0, s, file,
+         static_cast<const ChainPage*>(d_cp.get()), static_cast<const ChainState*>(d_st.get()), B, cin, j0.get());
+  const int64_t* jump = j0.get();
+  for (int r = 0; r < kChainLog; ++r) {
+    int64_t* out = (r % 2 == 0) ? j1.get() : j2.get();
+    launch("chain_double", chain_double_kernel, pq_blocks(cin, 256), 256, 0, s, jump, out, cin);
+    jump = out;
+  }
+  Buffer<int64_t> ck(al, chain_cks);
+  launch("chain_checkpoints", chain_checkpoints_kernel, pq_blocks(nc, 128), 128, 0, s,
+         static_cast<const ChainPage*>(d_cp.get()), d_st.get(), B, jump, ck.get());
+  Buffer<int64_t> epos(al, chain_elems), elen(al, chain_elems), emeta(al, chain_elems), eoff(al, chain_elems);
+  launch("chain_walk", chain_walk_kernel, pq_blocks(chain_cks, 128), 128, 0, s, file,
+         static_cast<const ChainPage*>(d_cp.get()), d_st.get(), B, chain_cks, static_cast<const int64_t*>(ck.get()),
+         epos.get(), err);
+  launch("chain_decode", chain_decode_kernel, pq_blocks(chain_elems, 256), 256, 0, s, file,
+         static_cast<const ChainPage*>(d_cp.get()), static_cast<const ChainState*>(d_st.get()), B, chain_elems,
+         static_cast<const int64_t*>(epos.get()), elen.get(), emeta.get());
+  Buffer<int64_t> etotal(al, 1);
+  exclusive_scan_i64(elen.get(), eoff.get(), chain_elems, etotal.get(), ctx);
+  Buffer<int64_t> p0(al, chain_out), p1(al, chain_out);
+  launch("chain_ptr", chain_ptr_kernel, pq_blocks(chain_out, 256), 256, 0, s,
+         static_cast<const ChainPage*>(d_cp.get()), static_cast<const ChainState*>(d_st.get()), B, chain_out,
+         static_cast<const int64_t*>(eoff.get()), static_cast<const int64_t*>(elen.get()),
+         static_cast<const int64_t*>(emeta.get()), p0.get(), err);
+  int rounds = 1;  // every pointer moves back one byte or more: log2 of the page size rounds reach a literal
+  while ((int64_t(1) << rounds) <= chain_maxu) ++rounds;
+  int64_t* pin = p0.get();
+  int64_t* pout = p1.get();
+  for (int r = 0; r < rounds; ++r) {
+    launch("chain_jump", chain_jump_kernel, pq_blocks(chain_out, 256), 256, 0, s,
+           static_cast<const int64_t*>(pin), pout, chain_out);
+    std::swap(pin, pout);
+  }
+  launch("chain_final", chain_final_kernel, pq_blocks(chain_out, 256), 256, 0, s, file,
+         static_cast<const ChainPage*>(d_cp.get()), B, static_cast<const int64_t*>(pin), chain_out, scratch.get(),
+         err);
+  return scratch;
+}
+
 }  // namespace
 
 void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_page* pages, int npages,
@@ -1302,9 +1583,9 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   }
   // check the page table, lay out the decompression scratch
   std::vector<int64_t> covered(ncols, 0);
-  std::vector<int> snappy, chain, dict_strings, dict_chain, data_pages;
+  std::vector<int> snappy, frag, dict_strings, dict_chain, data_pages;
   std::vector<int64_t> soff;
-  int64_t scratch_bytes = 0, nentries = 0, chain_in = 0, dict_in = 0;
+  int64_t scratch_bytes = 0, nentries = 0, dict_in = 0;
   std::vector<PqPage> dev_pages(npages);
   for (int p = 0; p < npages; ++p) {
     const ldf_parquet_page& h = pages[p];
@@ -1322,13 +1603,8 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
     dev_pages[p].data_bytes = h.codec == LDF_PQ_SNAPPY ? h.uncompressed : h.compressed;
     if (h.codec == LDF_PQ_SNAPPY) {
       const int64_t lv = h.kind == LDF_PQ_DATA_V2 ? h.levels_bytes : 0;
-      if (C.physical[h.column] == LDF_PQ_BYTE_ARRAY && h.uncompressed - lv >= kChainMinBytes &&
-          chain_in + h.compressed <= kChainMaxInput) {
-        chain.push_back(p);  // decoded by the whole GPU (scratch laid out below)
-        chain_in += h.compressed - lv;
-      } else {
-        snappy.push_back(p);
-      }
+      if (h.uncompressed - lv > kFragBytes) frag.push_back(p);  // a warp per fragment
+      else snappy.push_back(p);
     }
     if (h.kind == LDF_PQ_DICT_PAGE) {
       LDF_REQUIRE(h.encoding == 0 || h.encoding == 2, "parquet_decode: dictionary pages must be PLAIN");
@@ -1358,41 +1634,14 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   }
   for (int j = 0; j < ncols; ++j)
     LDF_REQUIRE(covered[j] == nrows, "parquet_decode: the data pages do not cover every row of a column");
-  // scratch: the chain pages' outputs first (one index space), then the others
-  std::vector<ChainPage> cpages;
-  std::vector<int64_t> cbases;  // in | out | elem | ck, one entry per chain page each
-  int64_t chain_elems = 0, chain_cks = 0, chain_out = 0, chain_maxu = 1;
-  {
-    std::vector<int64_t> in_b, out_b, el_b, ck_b;
-    int64_t in_run = 0;
-    for (int p : chain) {
-      const ldf_parquet_page& h = pages[p];
-      const int64_t lv          = h.kind == LDF_PQ_DATA_V2 ? h.levels_bytes : 0;
-      ChainPage c{};
-      c.page     = p;
-      c.file_off = h.offset + lv;
-      c.n        = h.compressed - lv;
-      c.lv       = lv;
-      c.u        = h.uncompressed - lv;
-      c.elem_cap = c.n / 2 + 1;
-      c.ck_cap   = c.elem_cap / kChainStep + 2;
-      in_b.push_back(in_run);
-      out_b.push_back(scratch_bytes);
-      el_b.push_back(chain_elems);
-      ck_b.push_back(chain_cks);
-      in_run += c.n;
-      chain_elems += c.elem_cap;
-      chain_cks += c.ck_cap;
-      chain_maxu = std::max(chain_maxu, h.uncompressed);
-      scratch_bytes += (h.uncompressed + 15) & ~int64_t(15);
-      cpages.push_back(c);
-    }
-    chain_out = scratch_bytes;
-    for (auto* v : {&in_b, &out_b, &el_b, &ck_b}) cbases.insert(cbases.end(), v->begin(), v->end());
-    for (int p : snappy) {
-      soff.push_back(scratch_bytes);
-      scratch_bytes += (pages[p].uncompressed + 15) & ~int64_t(15);
-    }
+  std::vector<int64_t> frag_off;
+  for (int p : frag) {
+    frag_off.push_back(scratch_bytes);
+    scratch_bytes += (pages[p].uncompressed + 15) & ~int64_t(15);
+  }
+  for (int p : snappy) {
+    soff.push_back(scratch_bytes);
+    scratch_bytes += (pages[p].uncompressed + 15) & ~int64_t(15);
   }
   {  // decompress the largest pages first: a page is one warp's sequential work
     std::vector<int> order(snappy.size());
@@ -1413,7 +1662,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   cudaStream_t s      = ctx.stream();
   Buffer<uint8_t> scratch(al, std::max<int64_t>(scratch_bytes, 16));
   for (size_t q = 0; q < snappy.size(); ++q) dev_pages[snappy[q]].data = scratch.get() + soff[q];
-  for (size_t q = 0; q < chain.size(); ++q) dev_pages[chain[q]].data = scratch.get() + cbases[chain.size() + q];
+  for (size_t q = 0; q < frag.size(); ++q) dev_pages[frag[q]].data = scratch.get() + frag_off[q];
   for (int p = 0; p < npages; ++p)
     if (pages[p].codec != LDF_PQ_SNAPPY) dev_pages[p].data = file + pages[p].offset;
   Buffer<PqPage> d_pages(al, std::max(npages, 1));
@@ -1446,60 +1695,98 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   Buffer<int32_t> entry_len(al, std::max<int64_t>(nentries, 1));
   const int nsn = static_cast<int>(snappy.size()), nds = static_cast<int>(dict_strings.size()),
             ndp = static_cast<int>(data_pages.size());
-  if (!chain.empty()) {  // large byte-array pages: the element chains ranked by the whole GPU
-    const int nc          = static_cast<int>(chain.size());
-    const int64_t cin     = chain_in;
-    Buffer<ChainPage> d_cp(al, nc);
-    Buffer<ChainState> d_st(al, nc);
-    Buffer<int64_t> d_cb(al, cbases.size());
-    LDF_CUDA(cudaMemcpyAsync(d_cp.get(), cpages.data(), nc * sizeof(ChainPage), cudaMemcpyHostToDevice, s));
-    LDF_CUDA(cudaMemcpyAsync(d_cb.get(), cbases.data(), cbases.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    const ChainBases B{d_cb.get(), d_cb.get() + nc, d_cb.get() + 2 * nc, d_cb.get() + 3 * nc, nc};
-    Buffer<int64_t> j0(al, cin), j1(al, cin), j2(al, cin);
-    launch("chain_start", chain_start_kernel, pq_blocks(nc, 128), 128, 0, s, file,
-           static_cast<const ChainPage*>(d_cp.get()), d_st.get(), nc, d_err.get());
-    launch("chain_next", chain_next_kernel, pq_blocks(cin, 256), 256, 0, s, file,
-           static_cast<const ChainPage*>(d_cp.get()), static_cast<const ChainState*>(d_st.get()), B, cin, j0.get());
-    const int64_t* jump = j0.get();
-    for (int r = 0; r < kChainLog; ++r) {
-      int64_t* out = (r % 2 == 0) ? j1.get() : j2.get();
-      launch("chain_double", chain_double_kernel, pq_blocks(cin, 256), 256, 0, s, jump, out, cin);
-      jump = out;
+  // pages of several fragments, kFragMaxInput stream bytes at a time
+  std::vector<FragPage> fpages;
+  std::vector<int> h_redo(frag.size(), 0);
+  Buffer<FragPage> d_fp(al, std::max<size_t>(frag.size(), 1));
+  Buffer<int> d_redo(al, std::max<size_t>(frag.size(), 1));
+  Buffer<unsigned long long> exits;
+  Buffer<FragStart> starts;
+  if (!frag.empty()) {
+    struct Round {
+      size_t first, count;
+      int64_t in, segs, frags;
+    };
+    std::vector<Round> rounds;
+    int64_t most_in = 0, most_frags = 0;
+    for (size_t q = 0; q < frag.size(); ++q) {
+      const ldf_parquet_page& h = pages[frag[q]];
+      FragPage f{};
+      f.page     = frag[q];
+      f.lv       = h.kind == LDF_PQ_DATA_V2 ? h.levels_bytes : 0;
+      f.file_off = h.offset + f.lv;
+      f.n        = h.compressed - f.lv;
+      f.u        = h.uncompressed - f.lv;
+      f.nfrag    = static_cast<int>(ceil_div(f.u, kFragBytes));
+      f.dst      = scratch.get() + frag_off[q];
+      if (rounds.empty() || (rounds.back().in > 0 && rounds.back().in + f.n > kFragMaxInput))
+        rounds.push_back(Round{q, 0, 0, 0, 0});
+      Round& r = rounds.back();
+      f.exit0  = r.in;
+      f.seg0   = r.segs;
+      f.frag0  = r.frags;
+      ++r.count;
+      r.in += f.n;
+      r.segs += ceil_div(f.n, int64_t(kFragSeg));
+      r.frags += f.nfrag;
+      most_in    = std::max(most_in, r.in);
+      most_frags = std::max(most_frags, r.frags);
+      fpages.push_back(f);
     }
-    Buffer<int64_t> ck(al, chain_cks);
-    launch("chain_checkpoints", chain_checkpoints_kernel, pq_blocks(nc, 128), 128, 0, s,
-           static_cast<const ChainPage*>(d_cp.get()), d_st.get(), B, jump, ck.get());
-    Buffer<int64_t> epos(al, chain_elems), elen(al, chain_elems), emeta(al, chain_elems), eoff(al, chain_elems);
-    launch("chain_walk", chain_walk_kernel, pq_blocks(chain_cks, 128), 128, 0, s, file,
-           static_cast<const ChainPage*>(d_cp.get()), d_st.get(), B, chain_cks, static_cast<const int64_t*>(ck.get()),
-           epos.get(), d_err.get());
-    launch("chain_decode", chain_decode_kernel, pq_blocks(chain_elems, 256), 256, 0, s, file,
-           static_cast<const ChainPage*>(d_cp.get()), static_cast<const ChainState*>(d_st.get()), B, chain_elems,
-           static_cast<const int64_t*>(epos.get()), elen.get(), emeta.get());
-    Buffer<int64_t> etotal(al, 1);
-    exclusive_scan_i64(elen.get(), eoff.get(), chain_elems, etotal.get(), ctx);
-    Buffer<int64_t> p0(al, chain_out), p1(al, chain_out);
-    launch("chain_ptr", chain_ptr_kernel, pq_blocks(chain_out, 256), 256, 0, s,
-           static_cast<const ChainPage*>(d_cp.get()), static_cast<const ChainState*>(d_st.get()), B, chain_out,
-           static_cast<const int64_t*>(eoff.get()), static_cast<const int64_t*>(elen.get()),
-           static_cast<const int64_t*>(emeta.get()), p0.get(), d_err.get());
-    int rounds = 1;  // every pointer moves back one byte or more: log2 of the page size rounds reach a literal
-    while ((int64_t(1) << rounds) <= chain_maxu) ++rounds;
-    int64_t* pin = p0.get();
-    int64_t* pout = p1.get();
-    for (int r = 0; r < rounds; ++r) {
-      launch("chain_jump", chain_jump_kernel, pq_blocks(chain_out, 256), 256, 0, s,
-             static_cast<const int64_t*>(pin), pout, chain_out);
-      std::swap(pin, pout);
+    exits  = Buffer<unsigned long long>(al, std::max<int64_t>(most_in, 1));
+    starts = Buffer<FragStart>(al, most_frags);
+    LDF_CUDA(cudaMemcpyAsync(d_fp.get(), fpages.data(), frag.size() * sizeof(FragPage), cudaMemcpyHostToDevice, s));
+    LDF_CUDA(cudaMemsetAsync(d_redo.get(), 0, frag.size() * sizeof(int), s));
+    for (const Round& r : rounds) {
+      const FragPage* fp = d_fp.get() + r.first;
+      const int np       = static_cast<int>(r.count);
+      if (r.segs > 0)
+        launch("snap_exits", snap_exits_kernel, static_cast<unsigned>(r.segs), kExitThreads, 0, s, file, fp, np,
+               exits.get());
+      launch("snap_starts", snap_starts_kernel, static_cast<unsigned>(np), 32, 0, s, file, fp,
+             static_cast<const unsigned long long*>(exits.get()), starts.get(), d_redo.get() + r.first);
+      launch("snap_fragment", snap_fragment_kernel, static_cast<unsigned>(r.frags), kLanes, 0, s, file, fp, np,
+             static_cast<const FragStart*>(starts.get()), d_redo.get() + r.first);
     }
-    launch("chain_final", chain_final_kernel, pq_blocks(chain_out, 256), 256, 0, s, file,
-           static_cast<const ChainPage*>(d_cp.get()), B, static_cast<const int64_t*>(pin), chain_out, scratch.get(),
-           d_err.get());
+    ctx.fetch(h_redo.data(), d_redo.get(), frag.size() * sizeof(int));
   }
   if (nsn > 0)
     launch("pq_snappy", pq_snappy_kernel, static_cast<unsigned>(nsn), kLanes, 0, s,
            file, d_pages.get(), static_cast<const int*>(d_lists.get()), nsn, scratch.get(),
            static_cast<const int64_t*>(d_soff.get()), d_err.get());
+  Buffer<uint8_t> chain_scratch;
+  if (!frag.empty()) {
+    ctx.finish();
+    std::vector<int> again, chain;
+    std::vector<int64_t> again_off;
+    int64_t chain_in = 0;
+    for (size_t q = 0; q < frag.size(); ++q) {
+      if (!h_redo[q]) continue;
+      const FragPage& f = fpages[q];
+      if (C.physical[pages[f.page].column] == LDF_PQ_BYTE_ARRAY && f.u >= kChainMinBytes &&
+          chain_in + pages[f.page].compressed <= kChainMaxInput) {
+        chain.push_back(f.page);  // by the whole GPU
+        chain_in += f.n;
+      } else {  // one warp a page
+        again.push_back(f.page);
+        again_off.push_back(frag_off[q]);
+      }
+    }
+    if (!again.empty()) {
+      Buffer<int> d_again(al, again.size());
+      Buffer<int64_t> d_again_off(al, again.size());
+      LDF_CUDA(cudaMemcpyAsync(d_again.get(), again.data(), again.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+      LDF_CUDA(cudaMemcpyAsync(d_again_off.get(), again_off.data(), again.size() * sizeof(int64_t),
+                               cudaMemcpyHostToDevice, s));
+      launch("pq_snappy", pq_snappy_kernel, static_cast<unsigned>(again.size()), kLanes, 0, s, file, d_pages.get(),
+             static_cast<const int*>(d_again.get()), static_cast<int>(again.size()), scratch.get(),
+             static_cast<const int64_t*>(d_again_off.get()), d_err.get());
+    }
+    if (!chain.empty()) {
+      chain_scratch = decode_chain_pages(ctx, file, pages, chain, chain_in, dev_pages, d_err.get());
+      LDF_CUDA(cudaMemcpyAsync(d_pages.get(), dev_pages.data(), npages * sizeof(PqPage), cudaMemcpyHostToDevice, s));
+    }
+  }
   if (nds > 0)
     launch("pq_dict_strings", pq_dict_strings_kernel, static_cast<unsigned>(nds), kPqThreads, 0, s,
            static_cast<const PqPage*>(d_pages.get()), static_cast<const int*>(d_lists.get()) + nsn, nds,
