@@ -5,19 +5,21 @@
 // The caller walks the footer and the page headers (Thrift, a few bytes per
 // page) and hands over one entry per page; the whole file is in device
 // memory.  Then:
-// 1. Snappy pages are decompressed, one warp per page, with the compressed
-//    stream staged and the recent output kept in shared memory; every lane
-//    parses the same element tags and the warp copies each element's bytes
-//    together.
-// 2. Dictionary pages of byte arrays get an entry table (offset, length),
-//    one block per page walking the length prefixes from shared memory.
+// 1. Snappy pages are decompressed, one warp per 64 KB fragment, with the
+//    compressed stream staged and the recent output kept in shared memory;
+//    where the fragments start in the stream is found by a parallel pass.
+//    Streams not made of fragments go a warp per page, or by chains of
+//    pointers over the whole GPU (large byte-array pages).
+// 2. Dictionary pages of byte arrays and PLAIN byte-array pages get an entry
+//    table (offset, length), their chains of length prefixes ranked in
+//    parallel (small dictionary pages: one block walks the prefixes).
 // 3. One block per data page decodes its rows in tiles of kPqTile: thread 0
 //    cuts the next tile out of the RLE / bit-packed hybrid streams (the
 //    definition levels, the dictionary indices) as a list of run segments,
 //    and every thread decodes its values from the segment it falls in; a
 //    block scan of the definition levels gives each valid row its value
 //    index; PLAIN values are read at that index, dictionary values through
-//    the decoded index, and byte arrays by a walk of their length prefixes.
+//    the decoded index, and byte arrays through the entry table.
 // 4. String columns: lengths -> offsets (scan) -> characters copied.
 #include <algorithm>
 
@@ -37,6 +39,7 @@ struct PqPage {
   const uint8_t* data;    // payload, decompressed (the file's bytes for an uncompressed page)
   int64_t data_bytes;
   int64_t dict_entry0;    // byte-array dictionary pages: first entry in the entry table
+  int64_t plain0 = -1;    // PLAIN byte-array data pages: first value in the entry table (-1: prefixes walked)
 };
 
 // Error record: (page << 8 | code), the smallest kept.
@@ -69,9 +72,11 @@ constexpr int kSnapBatchBytes = 1024;  // output bytes of a batch at most
 constexpr int kSnapShort      = 64;    // longer literals are copied on their own
 constexpr int kSnapPerLane    = 4;     // output bytes per lane per window of a batch
 
-struct alignas(16) SnapShared {
+template <int WIN>
+struct alignas(16) SnapSharedOf {
+  static constexpr int kWin = WIN;
   uint8_t in[kSnapIn];
-  uint8_t win[kSnapWin];
+  uint8_t win[WIN];
   uint16_t size[kSnapIn];         // input bytes of an element whose tag is at in[x] (0xffff: unknown)
   uint8_t elem[kSnapBatchBytes];  // batch element of each output byte
   int64_t off[kSnapBatch];        // copy: offset
@@ -82,6 +87,7 @@ struct alignas(16) SnapShared {
   int32_t flags[kSnapBatch];      // 1: malformed on its own, 2: short enough for a batch
   int32_t cut, bad;
 };
+using SnapShared = SnapSharedOf<kSnapWin>;
 
 struct SnapStage {
   const uint8_t* src;
@@ -132,7 +138,8 @@ __device__ __forceinline__ SnapElem snap_decode(uint32_t t, uint32_t x)
 }
 
 // The tag at staged index r and the four bytes after it (r + 5 <= kSnapIn).
-__device__ __forceinline__ SnapElem snap_at(const SnapShared& sh, int r)
+template <typename Sh>
+__device__ __forceinline__ SnapElem snap_at(const Sh& sh, int r)
 {
   const uint8_t* q = sh.in + r;
   const uint32_t x = static_cast<uint32_t>(q[1]) | static_cast<uint32_t>(q[2]) << 8 |
@@ -175,7 +182,8 @@ __device__ __forceinline__ uint32_t snap_size(uint32_t t, uint32_t x)
 
 // size[] of the staged bytes: every position read as a tag, in parallel,
 // four positions from two aligned words at a time.
-__device__ void snap_sizes(SnapStage& st, SnapShared& sh)
+template <typename Sh>
+__device__ void snap_sizes(SnapStage& st, Sh& sh)
 {
   const int lane = threadIdx.x % kLanes;
 #pragma unroll 2
@@ -218,7 +226,8 @@ __device__ int64_t snap_load(const SnapStage& st, int64_t i, SnapGranule (&reg)[
 }
 
 // Makes the loaded stage the staged one: in[k] = src[ib + k].
-__device__ void snap_commit(SnapStage& st, SnapShared& sh, int64_t ib, const SnapGranule (&reg)[kSnapPer])
+template <typename Sh>
+__device__ void snap_commit(SnapStage& st, Sh& sh, int64_t ib, const SnapGranule (&reg)[kSnapPer])
 {
   const int lane = threadIdx.x % kLanes;
   __syncwarp();  // every lane is done with the previous contents
@@ -230,7 +239,8 @@ __device__ void snap_commit(SnapStage& st, SnapShared& sh, int64_t ib, const Sna
 
 // Stages the stream from the 16-byte boundary at or below stream index i;
 // with `sizes`, size[] too.
-__device__ void snap_stage(SnapStage& st, SnapShared& sh, int64_t i, bool sizes)
+template <typename Sh>
+__device__ void snap_stage(SnapStage& st, Sh& sh, int64_t i, bool sizes)
 {
   SnapGranule reg[kSnapPer];
   const int64_t ib = snap_load(st, i, reg);  // all loads first, then the stores
@@ -250,12 +260,13 @@ __device__ void snap_stage(SnapStage& st, SnapShared& sh, int64_t i, bool sizes)
 // at out[o - d + k % d] for byte k of a copy of offset d -- followed back
 // through the batch until it reaches a literal or output written before the
 // batch (ring or global).  Long literals are copied on their own.
-__device__ bool snappy_run(SnapStage& st, SnapShared& sh, uint8_t* dst, int64_t& i, int64_t& o, const int64_t total,
+template <typename Sh>
+__device__ bool snappy_run(SnapStage& st, Sh& sh, uint8_t* dst, int64_t& i, int64_t& o, const int64_t total,
                            const int64_t floor)
 {
   const int lane          = threadIdx.x % kLanes;
   const int64_t n         = st.n;
-  constexpr int64_t kMask = kSnapWin - 1;
+  constexpr int64_t kMask = Sh::kWin - 1;
   while (o < total) {
     if (i >= n) return false;
     if (i + 5 > st.ib + kSnapIn) snap_stage(st, sh, i, true);  // a tag and its extra bytes
@@ -342,9 +353,9 @@ __device__ bool snappy_run(SnapStage& st, SnapShared& sh, uint8_t* dst, int64_t&
       if (body > n || body + e.l > n || o + e.l > total) return false;
       // Copied a stage at a time with four-byte stores, the next stage's
       // loads in flight meanwhile; the ring keeps only the literal's last
-      // kSnapWin bytes.
+      // Sh::kWin bytes.
       const int64_t l         = e.l;
-      const int64_t ring_from = l > kSnapWin ? l - kSnapWin : 0;
+      const int64_t ring_from = l > Sh::kWin ? l - Sh::kWin : 0;
       int64_t from_i          = body;
       if (from_i >= st.ib + kSnapIn) snap_stage(st, sh, from_i, false);
       for (int64_t done = 0; done < l;) {
@@ -388,7 +399,7 @@ __device__ bool snappy_run(SnapStage& st, SnapShared& sh, uint8_t* dst, int64_t&
     // ring included, so a source inside the batch but before the window is
     // read from the ring and only sources inside the window are followed
     // back.  A batch writes ring slots of [o, o + B), B <= kSnapBatchBytes;
-    // the slots of positions from o + kSnapBatchBytes - kSnapWin on are not
+    // the slots of positions from o + kSnapBatchBytes - Sh::kWin on are not
     // among them, so those are read from the ring and older ones from dst.
     for (int base = 0; base < B; base += kSnapPerLane * kLanes) {
       uint8_t bv[kSnapPerLane];
@@ -407,7 +418,7 @@ __device__ bool snappy_run(SnapStage& st, SnapShared& sh, uint8_t* dst, int64_t&
         const int64_t nr = si >= 0 ? 0 : r0 - d + k;
         const bool far   = si < 0 && nr < base;
         const int64_t at = o + nr;
-        bv[q]    = si >= 0 ? sh.in[si + k] : (far ? (nr >= kSnapBatchBytes - kSnapWin ? sh.win[at & kMask] : dst[at]) : 0);
+        bv[q]    = si >= 0 ? sh.in[si + k] : (far ? (nr >= kSnapBatchBytes - Sh::kWin ? sh.win[at & kMask] : dst[at]) : 0);
         chase[q] = rb < B && si < 0 && !far;
         nrq[q]   = nr;
       }
@@ -429,7 +440,7 @@ __device__ bool snappy_run(SnapStage& st, SnapShared& sh, uint8_t* dst, int64_t&
           else nr = r0 - d + static_cast<int>(rr - r0) % static_cast<int>(d);  // d < len <= 64
           if (nr < base) {
             const int64_t at = o + nr;
-            bv[q] = nr >= kSnapBatchBytes - kSnapWin ? sh.win[at & kMask] : dst[at];
+            bv[q] = nr >= kSnapBatchBytes - Sh::kWin ? sh.win[at & kMask] : dst[at];
             break;
           }
           rr = nr;
@@ -1143,7 +1154,7 @@ __global__ void __launch_bounds__(kPqThreads) pq_data_kernel(const PqPage* pages
       if (threadIdx.x == 0) nseg = rle_cut(ids, static_cast<uint32_t>(tile_valid), seg);
       __syncthreads();
       for (uint32_t k = threadIdx.x; k < tile_valid; k += blockDim.x) idx[k] = rle_value(ids, seg, nseg, k);
-    } else if (strs && threadIdx.x == 0) {
+    } else if (strs && pg.plain0 < 0 && threadIdx.x == 0) {
       int64_t pos = walk;
       for (int64_t k = 0; k < tile_valid; ++k) {
         int64_t len = -1;
@@ -1190,6 +1201,15 @@ __global__ void __launch_bounds__(kPqThreads) pq_data_kernel(const PqPage* pages
             len = entry_len[dp->dict_entry0 + e];
           } else {
             pq_error(err, p, kPqErrDictIndex);
+          }
+        } else if (pg.plain0 >= 0) {
+          const int64_t e = pg.plain0 + vbase + k;
+          len             = entry_len[e];
+          src             = vals + entry_off[e];
+          if (len < 0) {  // the prefixes end before this value
+            pq_error(err, p, kPqErrValues);
+            src = nullptr;
+            len = 0;
           }
         } else {
           src = vals + str_off[k];
@@ -1285,12 +1305,12 @@ unsigned pq_blocks(int64_t work, int threads)
   return static_cast<unsigned>(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-// ---- Snappy pages of several fragments --------------------------------------
+// ---- Snappy pages by fragments ------------------------------------------------
 // Snappy compressors work on 64 KB of input at a time: no element crosses a
 // multiple of kFragBytes of output and no copy reaches back over one.  The
 // format does not demand it, so a page that breaks it (or is malformed) is
-// decoded again by the per-page kernels.  A page of several fragments is
-// decoded a warp per fragment:
+// decoded again by the per-page kernels.  Pages are decoded a warp per
+// fragment; for those of several fragments
 //  1. snap_exits: the stream in segments of kFragSeg bytes; for every position
 //     of a segment, read as a tag, where the elements from there on leave the
 //     segment and how many bytes they put out (pointer jumping in shared
@@ -1301,12 +1321,18 @@ unsigned pq_blocks(int64_t work, int threads)
 //     or before it;
 //  3. snap_fragment: one warp per fragment skips to its first element and
 //     decodes it (snappy_run).
-// A page as one warp's work took 19 ms for 1 MB pages of int64 and float32
-// values (4M rows of three columns).
+// The bound is each warp's chain of dependent shared-memory steps (8,000
+// elements a fragment of int64 values), so what counts is warps in flight:
+// 4M rows of three columns, 95 MB, take 2.1 ms here and 1.0 ms in the two
+// passes before; a warp per page and chains of pointers took 26 ms.
 constexpr int64_t kFragBytes    = 65536;
 constexpr int kFragSeg          = 4096;
 constexpr int kExitThreads      = 256;
-constexpr int64_t kFragMaxInput = int64_t(64) << 20;  // stream bytes per round (8 bytes of exits each)
+constexpr int64_t kFragMaxInput = int64_t(128) << 20;  // stream bytes per round (8 bytes of exits each)
+// Ring of recent output of a fragment's warp.  8 KB lets 14 warps share an SM
+// where the per-page kernel's 32 KB lets 5 (4.5 ms); copies from further back
+// read the output (median offset 1 to 3 KB).
+using FragShared = SnapSharedOf<8192>;
 
 struct FragPage {
   int page;
@@ -1398,7 +1424,11 @@ __global__ void snap_starts_kernel(const uint8_t* file, const FragPage* fp, cons
     }
   }
   int k = 0;
-  if (pos >= 0 && len == static_cast<uint64_t>(f.u)) {
+  if (pos >= 0 && len == static_cast<uint64_t>(f.u) && f.nfrag == 1) {
+    starts[f.frag0 + k++] = FragStart{pos, 0};
+    pos = f.n;
+    out = f.u;
+  } else if (pos >= 0 && len == static_cast<uint64_t>(f.u)) {
     while (pos < f.n && out < f.u) {
       const unsigned long long e = exits[f.exit0 + pos];
       const int64_t next         = pos / kFragSeg * kFragSeg + static_cast<int64_t>(e >> 32);
@@ -1415,7 +1445,7 @@ __global__ void snap_starts_kernel(const uint8_t* file, const FragPage* fp, cons
 __global__ void __launch_bounds__(kLanes) snap_fragment_kernel(const uint8_t* file, const FragPage* fp, int npages,
                                                               const FragStart* starts, int* redo)
 {
-  __shared__ SnapShared sh;
+  __shared__ FragShared sh;
   const int q       = frag_page_of(fp, npages, blockIdx.x, &FragPage::frag0);
   const FragPage& f = fp[q];
   const int lane    = threadIdx.x;
@@ -1465,6 +1495,118 @@ __global__ void __launch_bounds__(kLanes) snap_fragment_kernel(const uint8_t* fi
     ok = snappy_run(st, sh, f.dst + f.lv, i, o, to, from) && o == to;
   }
   if (!ok && lane == 0) redo[q] = 1;
+}
+
+// ---- PLAIN byte-array data pages ---------------------------------------------
+// The same three steps for the chain of length prefixes of a data page's
+// values: str_exits and str_starts find the first value of every segment and
+// its index, str_entries writes the (offset, length) of every value, one warp
+// per segment.  For pages of 20,000 strings 0.8 ms and 0.7 ms in the data
+// kernel, whose thread 0 walked the prefixes in 4.3 ms.
+constexpr int kPlainChainMin     = 256;  // values from which a page takes this path
+constexpr int64_t kPlainMaxInput = int64_t(512) << 20;  // page bytes per call (8 bytes of exits each)
+struct PlainPage {
+  int page;
+  int nullable;
+  int64_t exit0, seg0, entry0;
+};
+
+// A data page's value bytes (behind its definition levels).
+__device__ __forceinline__ const uint8_t* page_values(const PqPage& pg, bool nullable, int64_t& n)
+{
+  int64_t off = 0;
+  if (pg.h.kind == LDF_PQ_DATA_V2) off = pg.h.levels_bytes;
+  else if (nullable) off = pg.data_bytes >= 4 ? 4 + static_cast<int64_t>(le_bytes(pg.data, 4)) : pg.data_bytes + 1;
+  n = off <= pg.data_bytes ? pg.data_bytes - off : 0;
+  return pg.data + off;
+}
+__device__ __forceinline__ int plain_page_of(const PlainPage* pp, int n, int64_t seg)
+{
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (pp[mid].seg0 <= seg) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(kExitThreads) str_exits_kernel(const PqPage* pages, const PlainPage* pp, int npages,
+                                                                 unsigned long long* exits)
+{
+  __shared__ unsigned long long e[kFragSeg];
+  __shared__ uint8_t in[kFragSeg + 4];
+  const PlainPage& f = pp[plain_page_of(pp, npages, blockIdx.x)];
+  const int64_t s0   = (static_cast<int64_t>(blockIdx.x) - f.seg0) * kFragSeg;
+  int64_t n;
+  const uint8_t* vals = page_values(pages[f.page], f.nullable != 0, n);
+  if (s0 >= n) return;
+  const int m = static_cast<int>(n - s0 < kFragSeg ? n - s0 : kFragSeg);
+  for (int x = threadIdx.x; x < kFragSeg + 4; x += kExitThreads) in[x] = s0 + x < n ? vals[s0 + x] : 0;
+  __syncthreads();
+  for (int x = threadIdx.x; x < m; x += kExitThreads) {
+    const int64_t end = s0 + x + 4 + static_cast<int64_t>(le_bytes(in + x, 4));
+    // (a value that runs past the page ends the chain uncounted)
+    e[x] = end <= n && s0 + x + 4 <= n ? static_cast<unsigned long long>(end - s0) << 32 | 1u : 0xffffffffull << 32;
+  }
+  int more;
+  do {
+    __syncthreads();
+    more = 0;
+    for (int x = threadIdx.x; x < m; x += kExitThreads) {
+      const unsigned long long v = e[x];
+      const uint32_t nxt         = static_cast<uint32_t>(v >> 32);
+      if (nxt >= static_cast<uint32_t>(m)) continue;
+      const unsigned long long w = *static_cast<volatile unsigned long long*>(e + nxt);
+      e[x] = (w & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(v) + static_cast<uint32_t>(w));
+      more = 1;
+    }
+  } while (__syncthreads_or(more));
+  for (int x = threadIdx.x; x < m; x += kExitThreads) exits[f.exit0 + s0 + x] = e[x];
+}
+
+// starts[segment] = position and index of its first value (preset to -1).
+__global__ void str_starts_kernel(const PqPage* pages, const PlainPage* pp, const unsigned long long* exits,
+                                  FragStart* starts)
+{
+  if (threadIdx.x != 0) return;
+  const PlainPage& f = pp[blockIdx.x];
+  int64_t n;
+  page_values(pages[f.page], f.nullable != 0, n);
+  int64_t pos = 0, count = 0;
+  while (pos < n && count < pages[f.page].h.num_values) {
+    const int64_t seg          = pos / kFragSeg;
+    const unsigned long long e = exits[f.exit0 + pos];
+    starts[f.seg0 + seg]       = FragStart{pos, count};
+    pos = seg * kFragSeg + static_cast<int64_t>(e >> 32);
+    count += static_cast<int64_t>(e & 0xffffffffull);
+  }
+}
+
+__global__ void __launch_bounds__(kLanes) str_entries_kernel(const PqPage* pages, const PlainPage* pp, int npages,
+                                                            const FragStart* starts, int64_t* entry_off,
+                                                            int32_t* entry_len)
+{
+  __shared__ uint8_t in[kFragSeg + 4];
+  const FragStart fs = starts[blockIdx.x];
+  if (fs.pos < 0) return;
+  const PlainPage& f = pp[plain_page_of(pp, npages, blockIdx.x)];
+  const int64_t s0   = (static_cast<int64_t>(blockIdx.x) - f.seg0) * kFragSeg;
+  int64_t n;
+  const uint8_t* vals = page_values(pages[f.page], f.nullable != 0, n);
+  for (int x = threadIdx.x; x < kFragSeg + 4; x += kLanes) in[x] = s0 + x < n ? vals[s0 + x] : 0;
+  __syncwarp();
+  if (threadIdx.x != 0) return;
+  int64_t pos = fs.pos, k = fs.out;
+  while (pos < s0 + kFragSeg && k < pages[f.page].h.num_values) {
+    if (pos + 4 > n) break;
+    const int64_t len = static_cast<int64_t>(le_bytes(in + (pos - s0), 4));
+    if (pos + 4 + len > n) break;
+    entry_off[f.entry0 + k] = pos + 4;
+    entry_len[f.entry0 + k] = static_cast<int32_t>(len);
+    ++k;
+    pos += 4 + len;
+  }
 }
 
 // Snappy pages of byte arrays that are not made of fragments, decoded by the
@@ -1583,9 +1725,9 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   }
   // check the page table, lay out the decompression scratch
   std::vector<int64_t> covered(ncols, 0);
-  std::vector<int> snappy, frag, dict_strings, dict_chain, data_pages;
-  std::vector<int64_t> soff;
-  int64_t scratch_bytes = 0, nentries = 0, dict_in = 0;
+  std::vector<int> frag, dict_strings, dict_chain, data_pages;
+  std::vector<PlainPage> plain;
+  int64_t scratch_bytes = 0, nentries = 0, dict_in = 0, plain_in = 0, plain_segs = 0;
   std::vector<PqPage> dev_pages(npages);
   for (int p = 0; p < npages; ++p) {
     const ldf_parquet_page& h = pages[p];
@@ -1602,9 +1744,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
     dev_pages[p].h          = h;
     dev_pages[p].data_bytes = h.codec == LDF_PQ_SNAPPY ? h.uncompressed : h.compressed;
     if (h.codec == LDF_PQ_SNAPPY) {
-      const int64_t lv = h.kind == LDF_PQ_DATA_V2 ? h.levels_bytes : 0;
-      if (h.uncompressed - lv > kFragBytes) frag.push_back(p);  // a warp per fragment
-      else snappy.push_back(p);
+      frag.push_back(p);
     }
     if (h.kind == LDF_PQ_DICT_PAGE) {
       LDF_REQUIRE(h.encoding == 0 || h.encoding == 2, "parquet_decode: dictionary pages must be PLAIN");
@@ -1628,6 +1768,24 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
                       pages[h.dict].column == h.column,
                     "parquet_decode: a dictionary-encoded page without its dictionary");
       LDF_REQUIRE(h.row0 >= 0 && h.row0 + h.num_values <= nrows, "parquet_decode: page rows out of range");
+      if (h.encoding == 0 && C.physical[h.column] == LDF_PQ_BYTE_ARRAY && h.num_values >= kPlainChainMin) {
+        PlainPage f{};
+        f.page     = p;
+        f.nullable = C.nullable[h.column];
+        f.exit0    = plain_in;
+        f.seg0     = plain_segs;
+        f.entry0   = nentries;
+        plain_in += dev_pages[p].data_bytes;
+        plain_segs += ceil_div(dev_pages[p].data_bytes, int64_t(kFragSeg));
+        if (plain_in > kPlainMaxInput) {  // its bytes' exits would take too much room: walked by the data kernel
+          plain_in   = f.exit0;
+          plain_segs = f.seg0;
+        } else {
+          dev_pages[p].plain0 = nentries;
+          nentries += h.num_values;
+          plain.push_back(f);
+        }
+      }
       covered[h.column] += h.num_values;
       data_pages.push_back(p);
     }
@@ -1639,43 +1797,20 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
     frag_off.push_back(scratch_bytes);
     scratch_bytes += (pages[p].uncompressed + 15) & ~int64_t(15);
   }
-  for (int p : snappy) {
-    soff.push_back(scratch_bytes);
-    scratch_bytes += (pages[p].uncompressed + 15) & ~int64_t(15);
-  }
-  {  // decompress the largest pages first: a page is one warp's sequential work
-    std::vector<int> order(snappy.size());
-    for (size_t q = 0; q < order.size(); ++q) order[q] = static_cast<int>(q);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-      return pages[snappy[a]].uncompressed > pages[snappy[b]].uncompressed;
-    });
-    std::vector<int> sp(order.size());
-    std::vector<int64_t> so(order.size());
-    for (size_t q = 0; q < order.size(); ++q) {
-      sp[q] = snappy[order[q]];
-      so[q] = soff[order[q]];
-    }
-    snappy.swap(sp);
-    soff.swap(so);
-  }
   const Allocator& al = ctx.alloc();
   cudaStream_t s      = ctx.stream();
   Buffer<uint8_t> scratch(al, std::max<int64_t>(scratch_bytes, 16));
-  for (size_t q = 0; q < snappy.size(); ++q) dev_pages[snappy[q]].data = scratch.get() + soff[q];
   for (size_t q = 0; q < frag.size(); ++q) dev_pages[frag[q]].data = scratch.get() + frag_off[q];
   for (int p = 0; p < npages; ++p)
     if (pages[p].codec != LDF_PQ_SNAPPY) dev_pages[p].data = file + pages[p].offset;
   Buffer<PqPage> d_pages(al, std::max(npages, 1));
-  std::vector<int> lists;  // snappy | dict strings | data pages
-  lists.insert(lists.end(), snappy.begin(), snappy.end());
+  std::vector<int> lists;  // dict strings | data pages
   lists.insert(lists.end(), dict_strings.begin(), dict_strings.end());
   lists.insert(lists.end(), data_pages.begin(), data_pages.end());
   Buffer<int> d_lists(al, std::max<size_t>(lists.size(), 1));
-  Buffer<int64_t> d_soff(al, std::max<size_t>(soff.size(), 1));
   Buffer<unsigned long long> d_err(al, 1);
   LDF_CUDA(cudaMemcpyAsync(d_pages.get(), dev_pages.data(), npages * sizeof(PqPage), cudaMemcpyHostToDevice, s));
   LDF_CUDA(cudaMemcpyAsync(d_lists.get(), lists.data(), lists.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-  LDF_CUDA(cudaMemcpyAsync(d_soff.get(), soff.data(), soff.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
   LDF_CUDA(cudaMemsetAsync(d_err.get(), 0xff, sizeof(unsigned long long), s));
   // outputs
   std::vector<Buffer<const uint8_t*>> src_bufs;
@@ -1693,8 +1828,8 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   }
   Buffer<int64_t> entry_off(al, std::max<int64_t>(nentries, 1));
   Buffer<int32_t> entry_len(al, std::max<int64_t>(nentries, 1));
-  const int nsn = static_cast<int>(snappy.size()), nds = static_cast<int>(dict_strings.size()),
-            ndp = static_cast<int>(data_pages.size());
+  if (!plain.empty()) LDF_CUDA(cudaMemsetAsync(entry_len.get(), 0xff, nentries * sizeof(int32_t), s));
+  const int nds = static_cast<int>(dict_strings.size()), ndp = static_cast<int>(data_pages.size());
   // pages of several fragments, kFragMaxInput stream bytes at a time
   std::vector<FragPage> fpages;
   std::vector<int> h_redo(frag.size(), 0);
@@ -1717,17 +1852,18 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
       f.file_off = h.offset + f.lv;
       f.n        = h.compressed - f.lv;
       f.u        = h.uncompressed - f.lv;
-      f.nfrag    = static_cast<int>(ceil_div(f.u, kFragBytes));
+      f.nfrag    = static_cast<int>(std::max<int64_t>(1, ceil_div(f.u, kFragBytes)));
+      const int64_t exits_n = f.nfrag > 1 ? f.n : 0;
       f.dst      = scratch.get() + frag_off[q];
-      if (rounds.empty() || (rounds.back().in > 0 && rounds.back().in + f.n > kFragMaxInput))
+      if (rounds.empty() || (rounds.back().in > 0 && rounds.back().in + exits_n > kFragMaxInput))
         rounds.push_back(Round{q, 0, 0, 0, 0});
       Round& r = rounds.back();
       f.exit0  = r.in;
       f.seg0   = r.segs;
       f.frag0  = r.frags;
       ++r.count;
-      r.in += f.n;
-      r.segs += ceil_div(f.n, int64_t(kFragSeg));
+      r.in += exits_n;
+      r.segs += ceil_div(exits_n, int64_t(kFragSeg));
       r.frags += f.nfrag;
       most_in    = std::max(most_in, r.in);
       most_frags = std::max(most_frags, r.frags);
@@ -1750,10 +1886,6 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
     }
     ctx.fetch(h_redo.data(), d_redo.get(), frag.size() * sizeof(int));
   }
-  if (nsn > 0)
-    launch("pq_snappy", pq_snappy_kernel, static_cast<unsigned>(nsn), kLanes, 0, s,
-           file, d_pages.get(), static_cast<const int*>(d_lists.get()), nsn, scratch.get(),
-           static_cast<const int64_t*>(d_soff.get()), d_err.get());
   Buffer<uint8_t> chain_scratch;
   if (!frag.empty()) {
     ctx.finish();
@@ -1789,7 +1921,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   }
   if (nds > 0)
     launch("pq_dict_strings", pq_dict_strings_kernel, static_cast<unsigned>(nds), kPqThreads, 0, s,
-           static_cast<const PqPage*>(d_pages.get()), static_cast<const int*>(d_lists.get()) + nsn, nds,
+           static_cast<const PqPage*>(d_pages.get()), static_cast<const int*>(d_lists.get()), nds,
            entry_off.get(), entry_len.get(), d_err.get());
   if (!dict_chain.empty()) {  // large dictionary pages: the length-prefix chains ranked by the whole GPU
     const int nc = static_cast<int>(dict_chain.size());
@@ -1832,9 +1964,27 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
            static_cast<const DictChain*>(d_dc.get()), B, ck_run, static_cast<const int64_t*>(ck.get()),
            static_cast<const int64_t*>(d_nck.get()), entry_off.get(), entry_len.get(), d_err.get());
   }
+  if (!plain.empty()) {
+    const int np = static_cast<int>(plain.size());
+    Buffer<PlainPage> d_pp(al, np);
+    if (static_cast<int64_t>(exits.size()) < plain_in) exits = Buffer<unsigned long long>(al, plain_in);
+    if (static_cast<int64_t>(starts.size()) < plain_segs) starts = Buffer<FragStart>(al, std::max<int64_t>(plain_segs, 1));
+    LDF_CUDA(cudaMemcpyAsync(d_pp.get(), plain.data(), np * sizeof(PlainPage), cudaMemcpyHostToDevice, s));
+    if (plain_segs > 0) LDF_CUDA(cudaMemsetAsync(starts.get(), 0xff, plain_segs * sizeof(FragStart), s));
+    const PqPage* dp = d_pages.get();
+    if (plain_segs > 0)
+      launch("str_exits", str_exits_kernel, static_cast<unsigned>(plain_segs), kExitThreads, 0, s, dp,
+             static_cast<const PlainPage*>(d_pp.get()), np, exits.get());
+    launch("str_starts", str_starts_kernel, static_cast<unsigned>(np), 32, 0, s, dp,
+           static_cast<const PlainPage*>(d_pp.get()), static_cast<const unsigned long long*>(exits.get()), starts.get());
+    if (plain_segs > 0)
+      launch("str_entries", str_entries_kernel, static_cast<unsigned>(plain_segs), kLanes, 0, s, dp,
+             static_cast<const PlainPage*>(d_pp.get()), np, static_cast<const FragStart*>(starts.get()),
+             entry_off.get(), entry_len.get());
+  }
   if (ndp > 0)
     launch("pq_data", pq_data_kernel, static_cast<unsigned>(ndp), kPqThreads, 0, s,
-           static_cast<const PqPage*>(d_pages.get()), static_cast<const int*>(d_lists.get()) + nsn + nds, C,
+           static_cast<const PqPage*>(d_pages.get()), static_cast<const int*>(d_lists.get()) + nds, C,
            static_cast<const int64_t*>(entry_off.get()), static_cast<const int32_t*>(entry_len.get()), d_err.get());
   unsigned long long h_err = ~0ull;
   ctx.fetch(&h_err, d_err.get(), sizeof(h_err));

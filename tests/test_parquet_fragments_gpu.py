@@ -134,3 +134,35 @@ def test_malformed_stream_of_several_fragments(how):
         bad = varint(n + 8) + fine[len(varint(n)):]
     with pytest.raises(ValueError, match="Parquet page 1: a Snappy stream is malformed"):
         decode([fine, bad], [n // 8] * 2, N.LDF_PQ_INT64, N.LDF_INT64, [n] * 2)
+
+
+@pytest.mark.parametrize("version", ["1.0", "2.0"])
+@pytest.mark.parametrize("compression", ["snappy", "none"])
+@pytest.mark.parametrize("nulls", [False, True])
+@pytest.mark.parametrize("n", [255, 256, 20_000, 100_003])
+def test_plain_strings(tmp_path, n, nulls, compression, version):
+    """PLAIN byte-array pages (length prefixes ranked per 4 KB segment): empty
+    strings, strings of several segments, strings that end at a segment."""
+    import pyarrow.parquet as pq
+
+    from legate_dataframe.lib.parquet import parquet_read
+
+    rng = np.random.default_rng(n)
+    words = ["", "a", "xyz" * 7, "s" * 4088, "q" * 4092, "long " * 2500] + [f"w{i}" * (i % 9) for i in range(500)]
+    w = rng.integers(0, len(words), n)
+    w[rng.random(n) < 0.995] %= 3
+    t = pa.table({"s": pa.array([words[i] for i in w], mask=rng.random(n) < 0.3 if nulls else None), "i": np.arange(n)})
+    path = tmp_path / "t.parquet"
+    pq.write_table(t, path, use_dictionary=False, compression=compression, data_page_version=version,
+                   data_page_size=200_000)
+    assert parquet_read(str(path)).to_arrow().equals(t)
+
+
+def test_truncated_plain_strings():
+    from legate_dataframe import _native as N
+
+    data = b"".join(len(w).to_bytes(4, "little") + w for w in [b"value"] * 20_000)
+    for cut in (1, 5, 9_000):
+        st = pa.compress(data[:-cut], codec="snappy", asbytes=True)
+        with pytest.raises(ValueError, match="Parquet page 0: the page's values are truncated"):
+            decode([st], [20_000], N.LDF_PQ_BYTE_ARRAY, N.LDF_STRING, [len(data) - cut])
