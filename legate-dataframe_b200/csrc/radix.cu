@@ -12,9 +12,25 @@ namespace ldf {
 namespace {
 
 constexpr int RT    = kRadixThreads;
-constexpr int RI    = kRadixItems;
-constexpr int RTILE = kRadixTile;
 constexpr int RW    = RT / 32;
+
+// Rows per thread of a onesweep tile, and the resident CTAs per SM its
+// registers are sized for.  A pass on carried words gains from large tiles
+// (fewer look-backs and barriers per row): when first measured, one carried pass
+// over 100M rows took 0.94 / 0.84 / 0.82 ms with 12 / 16 / 20 rows of 4-byte
+// words (0.65 ms now, with 4-byte status words and full tiles loaded without
+// bounds), and 8-byte words were fastest with 16 (20 spill).  Passes that load their word from the
+// columns hold more per row and stay at 12.
+template <bool GATHER, typename KT>
+__host__ __device__ constexpr int radix_items()
+{
+  return GATHER ? kRadixItems : sizeof(KT) == 4 ? 20 : 16;
+}
+template <bool GATHER>
+__host__ __device__ constexpr int radix_min_blocks()
+{
+  return GATHER ? kRadixMinBlocks : 3;
+}
 
 __device__ __forceinline__ uint64_t bucket_word(const RadixPass& p, int64_t row)
 {
@@ -41,6 +57,25 @@ __device__ __forceinline__ void fused_add(uint64_t v, int off, uint64_t& c, uint
   }
 }
 
+__device__ __forceinline__ bool is_nan_raw(int type, uint64_t raw)
+{
+  if (type == LDF_FLOAT64)
+    return (raw & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (raw & 0x000fffffffffffffull) != 0;
+  if (type == LDF_FLOAT32) return (raw & 0x7f800000u) == 0x7f800000u && (raw & 0x007fffffu) != 0;
+  return false;
+}
+
+// code_k of a row from its raw value: values in order, NaNs next to them and
+// nulls outermost, both behind (nulls_at_end) or before the values.
+__device__ __forceinline__ uint64_t fused_code(const FusedKey& f, int k, uint64_t raw, bool valid)
+{
+  const SortKeyDesc& d = f.key[k];
+  if (!f.has_class[k]) return sort_word_of(d, raw, true) - f.min[k];
+  if (!valid) return d.nulls_at_end ? f.span[k] + 2 : 0;
+  if (is_nan_raw(d.col.type, raw)) return d.nulls_at_end ? f.span[k] + 1 : 1;
+  return sort_word_of(d, raw, true) - f.min[k] + (d.nulls_at_end ? 0 : 2);
+}
+
 // C = W >> 8 of the fused word W of a row (FusedKey); *low = W's low byte.
 __device__ __forceinline__ uint64_t fused_word(const FusedKey& f, int64_t row, uint32_t& low)
 {
@@ -48,7 +83,7 @@ __device__ __forceinline__ uint64_t fused_word(const FusedKey& f, int64_t row, u
   low        = 0;
 #pragma unroll
   for (int k = 0; k < kFuseMax; ++k)
-    if (k < f.n) fused_add(sort_word(f.key[k], row) - f.min[k], f.off[k], c, low);
+    if (k < f.n) fused_add(fused_code(f, k, dbits(f.key[k].col, row), dvalid(f.key[k].col, row)), f.off[k], c, low);
   return c;
 }
 
@@ -144,12 +179,12 @@ __global__ void __launch_bounds__(RT) histogram_kernel(HistArgs a)
 struct PassArgs {
   RadixPass p;
   int64_t n;
-  const uint64_t* keys_in;
-  uint64_t* keys_out;
+  const void* keys_in;  // carried words, KT each
+  void* keys_out;
   const int32_t* vals_in;  // null: identity
   int32_t* vals_out;
   const uint64_t* digit_base;  // [256]
-  uint64_t* status;            // [tiles * 256]
+  uint32_t* status;            // [tiles * 256] (tile_status)
   unsigned long long* counter;
   int32_t* inv_out;  // != null: inv_out[row] = the row's output position
   RadixPayload pay;  // columns moved by this pass (payload_empty: none)
@@ -284,25 +319,39 @@ __device__ __forceinline__ void move_payload_rows(const RadixPayload& p, const i
 }
 
 // Predecessor tiles whose status words one look-back round trip loads.
-constexpr int kLookback = 8;
+constexpr int kLookback = 4;
+
+// Status word of one digit of a tile: 0 not ready; a tile's own count + 1 (top
+// bit clear); the count of the tile and all before it, with the top bit set
+// (fewer than 2^31 rows).
+constexpr uint32_t kTilePrefix = 0x80000000u;
+__device__ __forceinline__ uint32_t ld_status(const uint32_t* p)
+{
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// Each word stands for itself (no other data is read on the strength of it).
+__device__ __forceinline__ void st_status(uint32_t* p, uint32_t v)
+{
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
 // Shared state of one onesweep tile.
 struct OsShared {
-  uint32_t whist[RW][256];  // per-warp digit counts, then per-warp digit prefixes
-  uint32_t tile_start[256];  // tile-local start of each digit
+  uint32_t whist[RW][256];  // per-warp digit counts, then tile-local positions
   int32_t delta[256];        // output position of staged row j of digit d: delta[d] + j
   uint32_t scan[RW + 1];
   int64_t tile[2];
 };
 
-// Lanes of the warp whose digit equals this lane's (d <= 256; 256 marks an
-// item without a row): one ballot per digit bit, each lane keeping the lanes
-// that agree with it on that bit.
+// Lanes of the warp whose digit equals this lane's: one ballot per digit bit,
+// each lane keeping the lanes that agree with it on that bit.
 __device__ __forceinline__ uint32_t digit_peers(uint32_t d)
 {
   uint32_t peers = 0xffffffffu;
 #pragma unroll
-  for (int b = 0; b < 9; ++b) {
+  for (int b = 0; b < 8; ++b) {
     const uint32_t bit = (d >> b) & 1u;
     const uint32_t set = __ballot_sync(0xffffffffu, bit);
     peers &= bit ? set : ~set;
@@ -311,86 +360,94 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d)
 }
 
 // Everything of one pass over one tile after its rows are in registers:
-// key[i] / val[i] / dr[i] (digit, 256 = no row) of item i of this thread,
-// item order (warp, i, lane).  Stable warp-level ranking, tile-local scan, the
-// tile's digit counts published at once, rows staged in digit order into
-// s_keys / s_vals / s_dig (tile-local positions need no look-back), per-digit
-// decoupled look-back, then coalesced runs written out.  sh.whist must be zero
-// on entry.  Ends with every thread past its reads of the staging arrays.
-template <bool WRITE_KEYS, bool MOVE>
-__device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile, uint64_t (&key)[RI],
+// key[i] / val[i] / dr[i] (digit) of item i of this thread, item order (warp,
+// i, lane).  Items past the last row, at the end of the last tile, count as
+// rows of digit 255: they land behind the tile's rows and are not written.
+// Stable warp-level ranking, the tile's digit counts published at once,
+// tile-local scan, rows staged in digit order into s_keys / s_vals / s_dig
+// (tile-local positions need no look-back), per-digit decoupled look-back, then
+// coalesced runs written out.  sh.whist must be zero on entry.  Ends with every
+// thread past its reads of the staging arrays.
+//
+// The bound of a pass on carried words is its instructions (about 140 per row
+// and warp, half the issue slots; DRAM 25 %), most of them the ranking.
+template <bool WRITE_KEYS, bool MOVE, typename KT, int RI>
+__device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile, KT (&key)[RI],
                                                  int32_t (&val)[RI], uint32_t (&dr)[RI], OsShared& sh,
-                                                 uint64_t* s_keys, int32_t* s_vals, uint8_t* s_dig)
+                                                 KT* s_keys, int32_t* s_vals, uint8_t* s_dig)
 {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t lt_mask = (1u << lane) - 1u;
   // stable warp-level ranking, items in (i, lane) order
+  uint32_t* whist = sh.whist[warp];
 #pragma unroll
   for (int i = 0; i < RI; ++i) {
     const uint32_t d     = dr[i];
     const uint32_t peers = digit_peers(d);
     const uint32_t rank  = __popc(peers & lt_mask);
-    uint32_t base        = 0;
-    if (d < 256) base = sh.whist[warp][d];
+    const uint32_t base  = whist[d];
     __syncwarp();
-    if (d < 256 && rank == 0) sh.whist[warp][d] = base + __popc(peers);
+    if (rank == 0) whist[d] = base + __popc(peers);
     __syncwarp();
-    dr[i] = d | ((base + rank) << 9);
+    dr[i] = d | ((base + rank) << 8);
   }
   __syncthreads();
-  // per-digit warp prefixes and tile counts (thread t owns digit t)
+  // per-digit warp prefixes and tile counts (thread t owns digit t); the
+  // counts are published before anything else, so that the tiles after this one
+  // can finish their look-back while it stages its rows
   const int t = threadIdx.x;
-  uint32_t run = 0;
+  uint32_t run = 0, count[RW];
 #pragma unroll
   for (int w = 0; w < RW; ++w) {
-    uint32_t c       = sh.whist[w][t];
-    sh.whist[w][t]   = run;
-    run += c;
+    count[w] = sh.whist[w][t];
+    run += count[w];
   }
+  uint32_t* st = a.status;
+  if (tile == 0) st_status(&st[t], kTilePrefix | run);
+  else st_status(&st[tile * 256 + t], run + 1);
   uint32_t tile_total;
   const uint32_t start = block_exclusive_scan<uint32_t, RT>(run, sh.scan, &tile_total);
-  sh.tile_start[t]     = start;
-  // publish this tile's digit counts before anything else, so the tiles
-  // after it can finish their look-back while this one stages its rows
-  uint64_t* st = a.status;
-  if (tile == 0) st_release_u64(&st[t], kFlagPrefix | run);
-  else st_release_u64(&st[tile * 256 + t], kFlagAgg | run);
+  {
+    uint32_t at = start;
+#pragma unroll
+    for (int w = 0; w < RW; ++w) {
+      sh.whist[w][t] = at;  // tile-local position of the warp's first row of the digit
+      at += count[w];
+    }
+  }
   __syncthreads();
   // stage the tile in digit order
 #pragma unroll
   for (int i = 0; i < RI; ++i) {
-    const uint32_t d = dr[i] & 0x1ffu;
-    if (d < 256) {
-      const uint32_t lp = sh.tile_start[d] + sh.whist[warp][d] + (dr[i] >> 9);
-      if (WRITE_KEYS) s_keys[lp] = key[i];
-      s_vals[lp] = val[i];
-      s_dig[lp]  = static_cast<uint8_t>(d);
-    }
+    const uint32_t d  = dr[i] & 0xffu;
+    const uint32_t lp = whist[d] + (dr[i] >> 8);
+    if (WRITE_KEYS) s_keys[lp] = key[i];
+    s_vals[lp] = val[i];
+    s_dig[lp]  = static_cast<uint8_t>(d);
   }
   // per-digit decoupled look-back, kLookback predecessors' status words
   // loaded together per round trip
   {
-    uint64_t excl = 0;
+    uint32_t excl = 0;
     if (tile > 0) {
       int64_t j      = tile - 1;  // next predecessor to fold in
       uint32_t spins = 0;
       while (j >= 0) {
-        uint64_t sv[kLookback];
+        uint32_t sv[kLookback];
 #pragma unroll
-        for (int w = 0; w < kLookback; ++w) sv[w] = j - w >= 0 ? ld_volatile_u64(&st[(j - w) * 256 + t]) : kFlagPrefix;
+        for (int w = 0; w < kLookback; ++w) sv[w] = j - w >= 0 ? ld_status(&st[(j - w) * 256 + t]) : kTilePrefix;
         int used  = 0;
         bool done = false, stall = false;
 #pragma unroll
         for (int w = 0; w < kLookback; ++w) {
           if (done || stall) continue;
-          const uint64_t f = sv[w] & ~kValueMask;
-          if (f == 0) {
+          if (sv[w] == 0) {
             stall = true;
             continue;
           }
-          excl += sv[w] & kValueMask;
+          done = (sv[w] & kTilePrefix) != 0;
+          excl += done ? sv[w] & ~kTilePrefix : sv[w] - 1;
           ++used;
-          if (f == kFlagPrefix) done = true;
         }
         if (done) break;
         j -= used;
@@ -402,18 +459,20 @@ __device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile
           __nanosleep(32);
         }
       }
-      st_release_u64(&st[tile * 256 + t], kFlagPrefix | (excl + run));
+      st_status(&st[tile * 256 + t], kTilePrefix | (excl + run));
     }
     // positions fit 32 bits (fewer than 2^31 rows)
     sh.delta[t] = static_cast<int32_t>(a.digit_base[t] + excl) - static_cast<int32_t>(start);
   }
   __syncthreads();
+  constexpr int RTILE = RT * RI;
   const int64_t tbase = tile * RTILE;
   const int cnt       = static_cast<int>(a.n - tbase < RTILE ? a.n - tbase : RTILE);
   if constexpr (!MOVE) {
+#pragma unroll 4
     for (int j = threadIdx.x; j < cnt; j += RT) {
       const int32_t pos = sh.delta[s_dig[j]] + j;
-      if (WRITE_KEYS) a.keys_out[pos] = s_keys[j];
+      if (WRITE_KEYS) static_cast<KT*>(a.keys_out)[pos] = s_keys[j];
       a.vals_out[pos] = s_vals[j];
       if (a.inv_out) a.inv_out[s_vals[j]] = static_cast<int32_t>(pos);
     }
@@ -444,12 +503,29 @@ __device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile
 // the columns at the row, the first pass of a word; otherwise the carried key).
 // In a pass on the carried word, all row ids and then all words are loaded
 // before any digit is taken, so that the thread's loads are in flight together.
-template <bool GATHER, bool FUSEDG = false>
-__device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, uint64_t (&key)[RI],
+template <bool GATHER, bool FUSEDG, typename KT, int RI>
+__device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, KT (&key)[RI],
                                                int32_t (&val)[RI], uint32_t (&dr)[RI])
 {
+  constexpr int RTILE = RT * RI;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t wbase = tile * RTILE + warp * (32 * RI) + lane;
+  if (!GATHER && a.p.src != DigitSrc::CLASS && (tile + 1) * RTILE <= a.n) {  // a full tile: no bounds
+    const KT* k = static_cast<const KT*>(a.keys_in) + wbase;
+    if (a.vals_in) {
+      const int32_t* v = a.vals_in + wbase;
+#pragma unroll
+      for (int i = 0; i < RI; ++i) val[i] = __ldg(v + i * 32);
+    } else {
+#pragma unroll
+      for (int i = 0; i < RI; ++i) val[i] = static_cast<int32_t>(wbase) + i * 32;
+    }
+#pragma unroll
+    for (int i = 0; i < RI; ++i) key[i] = __ldg(k + i * 32);
+#pragma unroll
+    for (int i = 0; i < RI; ++i) dr[i] = static_cast<uint32_t>(key[i] >> a.p.shift) & 0xffu;
+    return;
+  }
   if (!GATHER && a.p.src != DigitSrc::CLASS) {
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -459,26 +535,28 @@ __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, 
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const int64_t idx = wbase + i * 32;
-      key[i] = idx < a.n ? __ldg(reinterpret_cast<const unsigned long long*>(a.keys_in) + idx) : 0ull;
+      key[i] = idx < a.n ? __ldg(static_cast<const KT*>(a.keys_in) + idx) : KT(0);
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i)
-      dr[i] = wbase + i * 32 < a.n ? static_cast<uint32_t>(key[i] >> a.p.shift) & 0xffu : 256u;
+      dr[i] = wbase + i * 32 < a.n ? static_cast<uint32_t>(key[i] >> a.p.shift) & 0xffu : 255u;
     return;
   }
   if (FUSEDG) {
     // the fused word from its key columns, one column at a time with the
     // items' loads in flight together; dr[i] gathers W's low byte
+    uint64_t c[RI];
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const int64_t idx = wbase + i * 32;
       val[i] = idx < a.n ? (a.vals_in ? __ldg(a.vals_in + idx) : static_cast<int32_t>(idx)) : -1;
-      key[i] = 0;
+      c[i]   = 0;
       dr[i]  = 0;
     }
     for (int k = 0; k < a.fused.n; ++k) {
       const SortKeyDesc& kk = a.fused.key[k];
       uint64_t raw[RI];
+      uint32_t ok = 0;
 #pragma unroll
       for (int i = 0; i < RI; ++i) {
         raw[i] = 0;
@@ -489,18 +567,20 @@ __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, 
           case 4: raw[i] = __ldg(static_cast<const uint32_t*>(kk.col.data) + val[i]); break;
           default: raw[i] = __ldg(static_cast<const unsigned long long*>(kk.col.data) + val[i]); break;
         }
+        if (dvalid(kk.col, val[i])) ok |= 1u << i;
       }
 #pragma unroll
       for (int i = 0; i < RI; ++i)
-        if (val[i] >= 0) fused_add(sort_word_of(kk, raw[i], true) - a.fused.min[k], a.fused.off[k], key[i], dr[i]);
+        if (val[i] >= 0) fused_add(fused_code(a.fused, k, raw[i], (ok >> i) & 1u), a.fused.off[k], c[i], dr[i]);
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
+      key[i] = static_cast<KT>(c[i]);
       if (val[i] < 0) {
         val[i] = 0;
-        dr[i]  = 256;
+        dr[i]  = 255;
       } else if (!a.p.fused_low) {
-        dr[i] = static_cast<uint32_t>(key[i] >> a.p.shift) & 0xffu;
+        dr[i] = static_cast<uint32_t>(c[i] >> a.p.shift) & 0xffu;
       }
     }
     return;
@@ -510,29 +590,29 @@ __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, 
     const int64_t idx = wbase + i * 32;
     key[i]            = 0;
     val[i]            = 0;
-    dr[i]             = 256;
+    dr[i]             = 255;
     if (idx < a.n) {
       const int64_t row = a.vals_in ? a.vals_in[idx] : idx;
       val[i]            = static_cast<int32_t>(row);
       if (a.p.src == DigitSrc::CLASS) {
         dr[i] = class_digit(a.p.key, row);
       } else {
-        key[i] = GATHER ? pass_word(a.p, row) : a.keys_in[idx];
+        key[i] = static_cast<KT>(GATHER ? pass_word(a.p, row) : static_cast<const KT*>(a.keys_in)[idx]);
         dr[i]  = static_cast<uint32_t>(key[i] >> a.p.shift) & 0xffu;
       }
     }
   }
 }
 
-// Tiles ahead that a onesweep tile prefetches into L2 (one wave of resident
-// CTAs); LDF_B200_L2_PREFETCH=0 turns the prefetch off.
-int64_t prefetch_tiles()
+// Whether a onesweep tile prefetches the rows of the tile one wave of resident
+// CTAs ahead into L2 (LDF_B200_L2_PREFETCH=0 turns it off).
+bool prefetch_ahead()
 {
-  static const bool off = [] {
+  static const bool on = [] {
     const char* e = std::getenv("LDF_B200_L2_PREFETCH");
-    return e != nullptr && std::atoi(e) == 0;
+    return e == nullptr || std::atoi(e) != 0;
   }();
-  return off ? 0 : static_cast<int64_t>(num_sms()) * kRadixMinBlocks;
+  return on;
 }
 // Whether a first pass over rows in input order prefetches its key columns
 // (LDF_B200_L2_PREFETCH_FIRST=0 turns it off).
@@ -578,23 +658,27 @@ bool pass_columns_on_device(const RadixPass& p, const FusedKey* fused)
   return column_on_device(p.key.col);
 }
 
-// One tile per CTA.  WRITE_KEYS: later passes of the same word follow, so
-// carry the word along.  MOVE: the pass also moves a.pay's columns (the last
-// pass only, which carries no word).
-template <bool GATHER, bool WRITE_KEYS, bool MOVE = false, bool FUSEDG = false>
-__global__ void __launch_bounds__(RT, kRadixMinBlocks) onesweep_kernel(PassArgs a)
+// One tile per CTA.  WRITE_KEYS: later passes of the same word follow (or the
+// sorted words are wanted), so carry the word along.  MOVE: the pass also
+// moves a.pay's columns (the last pass only, which carries no word).  KT: the
+// carried word, 4 bytes when that holds it: 8 instead of 12 bytes a row read
+// and written in every pass.
+template <bool GATHER, bool WRITE_KEYS, bool MOVE, bool FUSEDG, typename KT>
+__global__ void __launch_bounds__(RT, radix_min_blocks<GATHER>()) onesweep_kernel(PassArgs a)
 {
+  constexpr int RI    = radix_items<GATHER, KT>();
+  constexpr int RTILE = RT * RI;
   __shared__ OsShared sh;
-  // staged tile (dynamic): [keys u64 x RTILE when carried][rows i32 x RTILE][digits u8 x RTILE]
+  // staged tile (dynamic): [keys KT x RTILE when carried][rows i32 x RTILE][digits u8 x RTILE]
   extern __shared__ __align__(16) unsigned char s_stage[];
-  uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_stage);
-  int32_t* s_vals  = reinterpret_cast<int32_t*>(s_stage + (WRITE_KEYS ? RTILE * sizeof(uint64_t) : 0));
-  uint8_t* s_dig   = reinterpret_cast<uint8_t*>(s_vals + RTILE);
+  KT* s_keys      = reinterpret_cast<KT*>(s_stage);
+  int32_t* s_vals = reinterpret_cast<int32_t*>(s_stage + (WRITE_KEYS ? RTILE * sizeof(KT) : 0));
+  uint8_t* s_dig  = reinterpret_cast<uint8_t*>(s_vals + RTILE);
 
   const int64_t tile = next_tile_id(a.counter, &sh.tile[0]);
   for (int i = threadIdx.x; i < RW * 256; i += RT) (&sh.whist[0][0])[i] = 0;
   __syncthreads();
-  uint64_t key[RI];
+  KT key[RI];
   int32_t val[RI];
   uint32_t dr[RI];
   if (a.pf_ahead > 0 && threadIdx.x == 0 && (tile + a.pf_ahead) * RTILE < a.n) {
@@ -602,7 +686,8 @@ __global__ void __launch_bounds__(RT, kRadixMinBlocks) onesweep_kernel(PassArgs 
     const int64_t hi = min(lo + static_cast<int64_t>(RTILE), a.n);
     if (!GATHER) {
       if (a.vals_in) l2_prefetch_bulk(a.vals_in, lo * 4, hi * 4);
-      if (a.p.src != DigitSrc::CLASS) l2_prefetch_bulk(a.keys_in, lo * 8, hi * 8);
+      if (a.p.src != DigitSrc::CLASS)
+        l2_prefetch_bulk(a.keys_in, lo * static_cast<int64_t>(sizeof(KT)), hi * static_cast<int64_t>(sizeof(KT)));
     } else if (a.pf_columns && a.vals_in == nullptr) {  // rows in input order: the key columns are read in order
       if (FUSEDG) {
         for (int k = 0; k < a.fused.n; ++k) prefetch_column(a.fused.key[k].col, lo, hi);
@@ -613,27 +698,32 @@ __global__ void __launch_bounds__(RT, kRadixMinBlocks) onesweep_kernel(PassArgs 
       }
     }
   }
-  load_tile_rows<GATHER, FUSEDG>(a, tile, key, val, dr);
-  rank_and_scatter<WRITE_KEYS, MOVE>(a, tile, key, val, dr, sh, s_keys, s_vals, s_dig);
+  load_tile_rows<GATHER, FUSEDG, KT, RI>(a, tile, key, val, dr);
+  rank_and_scatter<WRITE_KEYS, MOVE, KT, RI>(a, tile, key, val, dr, sh, s_keys, s_vals, s_dig);
 }
 
-constexpr size_t onesweep_smem(bool write_keys)
-{
-  return (write_keys ? RTILE * sizeof(uint64_t) : 0) + RTILE * (sizeof(int32_t) + 1);
-}
-
-template <bool GATHER, bool WRITE_KEYS, bool MOVE = false, bool FUSEDG = false>
-void launch_onesweep(cudaStream_t s, unsigned tiles, const PassArgs& a)
+// Runs the pass over a.n rows; clears the status words and the tile counter
+// behind them first.
+template <bool GATHER, bool WRITE_KEYS, bool MOVE = false, bool FUSEDG = false, typename KT = uint64_t>
+void launch_onesweep(cudaStream_t s, PassArgs& a)
 {
   static_assert(!(MOVE && WRITE_KEYS), "the pass that moves columns is the last one");
-  constexpr size_t smem = onesweep_smem(WRITE_KEYS);
-  LDF_CUDA(cudaFuncSetAttribute(onesweep_kernel<GATHER, WRITE_KEYS, MOVE, FUSEDG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
+  constexpr int64_t tile_rows = RT * radix_items<GATHER, KT>();
+  constexpr size_t smem = (WRITE_KEYS ? tile_rows * sizeof(KT) : 0) + tile_rows * (sizeof(int32_t) + 1);
+  const int64_t tiles   = ceil_div(a.n, tile_rows);
+  auto kernel           = onesweep_kernel<GATHER, WRITE_KEYS, MOVE, FUSEDG, KT>;
+  a.counter             = reinterpret_cast<unsigned long long*>(a.status + tiles * 256);
+  a.pf_ahead            = prefetch_ahead() ? int64_t(num_sms()) * radix_min_blocks<GATHER>() : 0;
+  LDF_CUDA(cudaMemsetAsync(a.status, 0, (tiles * 256 + 2) * sizeof(uint32_t), s));
+  LDF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   // profile names: a pass that loads its word from the columns, one that
   // moves the payload columns, the others
   const char* name = MOVE ? "onesweep_move" : (GATHER ? "onesweep_gather" : "onesweep");
-  launch(name, onesweep_kernel<GATHER, WRITE_KEYS, MOVE, FUSEDG>, tiles, RT, smem, s, a);
+  launch(name, kernel, static_cast<unsigned>(tiles), RT, smem, s, a);
 }
+
+// Status words of a pass, of the smallest tiles (the counter's included).
+int64_t status_words(int64_t n) { return ceil_div(n, int64_t(kRadixTile)) * 256 + 2; }
 
 // Identity order: the payload columns copied as they are.
 __global__ void copy_payload_kernel(RadixPayload p, int64_t n)
@@ -668,7 +758,7 @@ unsigned hist_blocks(int64_t n)
 bool same_word(const RadixPass& a, const RadixPass& b)
 {
   if (a.src != b.src || a.src == DigitSrc::CLASS) return false;
-  if (a.src == DigitSrc::BUCKET || a.src == DigitSrc::FUSED) return true;
+  if (a.src == DigitSrc::BUCKET || a.src == DigitSrc::FUSED || a.src == DigitSrc::CARRIED) return true;
   return a.key.col.data == b.key.col.data && a.key.descending == b.key.descending;
 }
 
@@ -692,6 +782,7 @@ __global__ void __launch_bounds__(256) word_range_kernel(WordRangeArgs a, int64_
       if (k >= a.n) continue;
       const DCol& c = a.key[k].col;
       uint64_t raw[kRangeRows];
+      uint32_t ok = 0;
 #pragma unroll
       for (int j = 0; j < kRangeRows; ++j) {
         const int64_t r = base + j * blockDim.x + threadIdx.x;
@@ -703,10 +794,12 @@ __global__ void __launch_bounds__(256) word_range_kernel(WordRangeArgs a, int64_
           case 4: raw[j] = __ldg(static_cast<const uint32_t*>(c.data) + r); break;
           default: raw[j] = __ldg(static_cast<const unsigned long long*>(c.data) + r); break;
         }
+        if (dvalid(c, r)) ok |= 1u << j;
       }
 #pragma unroll
       for (int j = 0; j < kRangeRows; ++j) {
         if (base + j * blockDim.x + threadIdx.x >= n) continue;
+        if (!((ok >> j) & 1u) || is_nan_raw(c.type, raw[j])) continue;
         const unsigned long long w = sort_word_of(a.key[k], raw[j], true);
         lo[k]                      = w < lo[k] ? w : lo[k];
         hi[k]                      = w > hi[k] ? w : hi[k];
@@ -743,7 +836,10 @@ void sort_word_ranges(const OpContext& ctx, const SortKeyDesc* keys, int nkeys, 
   WordRangeArgs a{};
   a.n = nkeys;
   for (int k = 0; k < nkeys; ++k) a.key[k] = keys[k];
-  if (n > 0) launch("word_range", word_range_kernel, hblocks(n), 256, 0, s, a, n, mm.get());
+  if (n > 0)
+    launch("word_range", word_range_kernel,
+           static_cast<unsigned>(std::min<int64_t>(ceil_div(n, int64_t(256) * kRangeRows), 8 * num_sms())), 256, 0, s, a,
+           n, mm.get());
   ctx.fetch(h.data(), mm.get(), h.size() * 8);
   ctx.finish();
   for (int k = 0; k < nkeys; ++k) {
@@ -773,38 +869,68 @@ void radix_histograms(const OpContext& ctx, const std::vector<RadixPass>& passes
   }
 }
 
-void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
-                     int32_t* perm, std::vector<uint32_t>* hist_out, int32_t* inv, const RadixPayload* payload,
-                     const FusedKey* fused)
+namespace {
+
+// Writes the word W >> drop (KT) of every row and counts all its digits: one
+// read of the key columns, kWordRows rows a thread with a column's loads in
+// flight together.
+constexpr int kWordRows = 4;
+struct WordArgs {
+  FusedKey f;
+  int64_t n;
+  int npasses;
+  void* words;
+  uint32_t* hist;  // [npasses][256]
+};
+template <typename KT>
+__global__ void __launch_bounds__(RT) fused_words_kernel(WordArgs a)
+{
+  __shared__ uint32_t sh[sizeof(KT) * 256];
+  for (int i = threadIdx.x; i < a.npasses * 256; i += RT) sh[i] = 0;
+  __syncthreads();
+  const int64_t per_iter = static_cast<int64_t>(RT) * kWordRows;
+  for (int64_t base = blockIdx.x * per_iter; base < a.n; base += static_cast<int64_t>(gridDim.x) * per_iter) {
+    uint64_t c[kWordRows];
+    uint32_t low[kWordRows];
+#pragma unroll
+    for (int j = 0; j < kWordRows; ++j) c[j] = 0, low[j] = 0;
+    for (int k = 0; k < a.f.n; ++k) {
+      const DCol& col = a.f.key[k].col;
+      uint64_t raw[kWordRows];
+      bool ok[kWordRows];
+#pragma unroll
+      for (int j = 0; j < kWordRows; ++j) {
+        const int64_t r = base + j * RT + threadIdx.x;
+        raw[j]          = r < a.n ? dbits_stream(col, r) : 0;
+        ok[j]           = r < a.n && dvalid_stream(col, r);
+      }
+#pragma unroll
+      for (int j = 0; j < kWordRows; ++j)
+        if (base + j * RT + threadIdx.x < a.n) fused_add(fused_code(a.f, k, raw[j], ok[j]), a.f.off[k], c[j], low[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kWordRows; ++j) {
+      const int64_t r = base + j * RT + threadIdx.x;
+      if (r >= a.n) continue;
+      const KT w = static_cast<KT>(a.f.drop ? c[j] >> (a.f.drop - 8) : c[j] << 8 | low[j]);
+      static_cast<KT*>(a.words)[r] = w;
+      for (int q = 0; q < a.npasses; ++q) atomicAdd(&sh[q * 256 + (static_cast<uint32_t>(w >> (8 * q)) & 0xffu)], 1u);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < a.npasses * 256; i += RT)
+    if (sh[i]) atomicAdd(&a.hist[i], sh[i]);
+}
+
+// The passes `run` (none of a constant digit) of `passes`, in order; hist: all
+// passes' digit counts.  first_words: the word that the first pass carries
+// (null: it is loaded from the columns), kb bytes.
+void run_passes(const OpContext& ctx, const std::vector<RadixPass>& passes, const std::vector<int>& run,
+                const std::vector<uint32_t>& hist, int64_t n, int32_t* perm, int32_t* inv, const RadixPayload* payload,
+                const FusedKey* fused, Buffer<uint8_t>* first_words, size_t kb, Buffer<uint8_t>* words)
 {
   const Allocator& al = ctx.alloc();
   cudaStream_t s      = ctx.stream();
-  const size_t P      = passes.size();
-  std::vector<uint32_t> hist(P * 256, 0);
-  if (P > 0 && n > 0) {
-    Buffer<uint32_t> d_hist(al, P * 256);
-    radix_histograms(ctx, passes, n, d_hist.get(), fused);
-    ctx.fetch(hist.data(), d_hist.get(), P * 256 * sizeof(uint32_t));
-    ctx.finish();
-  }
-  if (hist_out) *hist_out = hist;
-  // schedule: skip constant-digit passes; the first executed pass of a word
-  // gathers it, later passes of the same word read it carried
-  std::vector<int> run;
-  for (size_t q = 0; q < P; ++q) {
-    bool constant = false;
-    for (int d = 0; d < 256; ++d)
-      if (hist[q * 256 + d] == static_cast<uint32_t>(n)) constant = true;
-    if (!constant && n > 0) run.push_back(static_cast<int>(q));
-  }
-  if (run.empty()) {
-    if (n > 0) launch("iota", iota_kernel, hblocks(n), RT, 0, s, perm, n);
-    if (n > 0 && inv) launch("iota", iota_kernel, hblocks(n), RT, 0, s, inv, n);
-    if (n > 0 && payload && !payload_empty(*payload))
-      launch("copy_payload", copy_payload_kernel, hblocks(n), RT, 0, s, *payload, n);
-    LDF_CHECK_LAUNCH();
-    return;
-  }
   std::vector<uint64_t> bases(run.size() * 256);
   for (size_t k = 0; k < run.size(); ++k) {
     uint64_t acc = 0;
@@ -816,9 +942,8 @@ void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes,
   Buffer<uint64_t> d_bases(al, bases.size());
   LDF_CUDA(cudaMemcpyAsync(d_bases.get(), bases.data(), bases.size() * 8, cudaMemcpyHostToDevice, s));
 
-  const int64_t tiles = ceil_div(n, RTILE);
-  Buffer<uint64_t> status(al, tiles * 256 + 2);
-  Buffer<uint64_t> keys[2] = {Buffer<uint64_t>(al, n), Buffer<uint64_t>(al, n)};
+  Buffer<uint32_t> status(al, status_words(n));
+  Buffer<uint8_t> keys[2] = {Buffer<uint8_t>(al, n * kb), first_words ? std::move(*first_words) : Buffer<uint8_t>(al, n * kb)};
   Buffer<int32_t> vals_tmp(al, n);
   // ping-pong so that the last pass writes into `perm`
   int32_t* vbuf[2];
@@ -826,12 +951,12 @@ void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes,
   vbuf[0]        = odd ? perm : vals_tmp.get();
   vbuf[1]        = odd ? vals_tmp.get() : perm;
   const int32_t* vin = nullptr;
-  const uint64_t* kin = nullptr;
+  const void* kin    = first_words ? keys[1].get() : nullptr;
   for (size_t k = 0; k < run.size(); ++k) {
-    const RadixPass& p = passes[run[k]];
-    const bool gather  = k == 0 || !same_word(passes[run[k - 1]], p);
-    const bool write_keys = p.src != DigitSrc::CLASS && k + 1 < run.size() && same_word(p, passes[run[k + 1]]);
-    LDF_CUDA(cudaMemsetAsync(status.get(), 0, (tiles * 256 + 2) * 8, s));
+    const RadixPass& p    = passes[run[k]];
+    const bool last       = k + 1 == run.size();
+    const bool gather     = p.src != DigitSrc::CARRIED && (k == 0 || !same_word(passes[run[k - 1]], p));
+    const bool write_keys = p.src != DigitSrc::CLASS && (last ? words != nullptr : same_word(p, passes[run[k + 1]]));
     PassArgs a{};
     a.p          = p;
     a.n          = n;
@@ -841,29 +966,345 @@ void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes,
     a.vals_out   = vbuf[k % 2];
     a.digit_base = d_bases.get() + k * 256;
     a.status     = status.get();
-    a.counter    = reinterpret_cast<unsigned long long*>(status.get() + tiles * 256);
-    a.inv_out    = k + 1 == run.size() ? inv : nullptr;
-    if (k + 1 == run.size() && payload) a.pay = *payload;
+    a.inv_out    = last ? inv : nullptr;
+    if (last && payload) a.pay = *payload;
     if (fused) a.fused = *fused;
     a.err        = ctx.err();
-    a.pf_ahead   = prefetch_tiles();
     a.pf_columns = gather && k == 0 && prefetch_first_pass() && pass_columns_on_device(p, fused) ? 1 : 0;
-    const unsigned g = static_cast<unsigned>(tiles);
     const bool move = !payload_empty(a.pay);
-    if (gather && p.src == DigitSrc::FUSED) {  // the fused word's first pass
-      if (move) launch_onesweep<true, false, true, true>(s, g, a);
-      else if (write_keys) launch_onesweep<true, true, false, true>(s, g, a);
-      else launch_onesweep<true, false, false, true>(s, g, a);
-    } else if (move && gather) launch_onesweep<true, false, true>(s, g, a);
-    else if (move) launch_onesweep<false, false, true>(s, g, a);
-    else if (gather && write_keys) launch_onesweep<true, true>(s, g, a);
-    else if (gather) launch_onesweep<true, false>(s, g, a);
-    else if (write_keys) launch_onesweep<false, true>(s, g, a);
-    else launch_onesweep<false, false>(s, g, a);
-    LDF_CHECK_LAUNCH();
+    if (kb == 4) {
+      if (move) launch_onesweep<false, false, true, false, uint32_t>(s, a);
+      else if (write_keys) launch_onesweep<false, true, false, false, uint32_t>(s, a);
+      else launch_onesweep<false, false, false, false, uint32_t>(s, a);
+    } else if (gather && p.src == DigitSrc::FUSED) {  // the fused word's first pass
+      if (move) launch_onesweep<true, false, true, true>(s, a);
+      else if (write_keys) launch_onesweep<true, true, false, true>(s, a);
+      else launch_onesweep<true, false, false, true>(s, a);
+    } else if (move && gather) launch_onesweep<true, false, true>(s, a);
+    else if (move) launch_onesweep<false, false, true>(s, a);
+    else if (gather && write_keys) launch_onesweep<true, true>(s, a);
+    else if (gather) launch_onesweep<true, false>(s, a);
+    else if (write_keys) launch_onesweep<false, true>(s, a);
+    else launch_onesweep<false, false>(s, a);
     vin = vbuf[k % 2];
     kin = keys[k % 2].get();
+    if (words && last) *words = std::move(keys[k % 2]);
   }
+}
+
+// Passes whose digit is not the same in every row.
+std::vector<int> varying_passes(const std::vector<uint32_t>& hist, size_t P, int64_t n)
+{
+  std::vector<int> run;
+  for (size_t q = 0; q < P; ++q) {
+    bool constant = false;
+    for (int d = 0; d < 256; ++d)
+      if (hist[q * 256 + d] == static_cast<uint32_t>(n)) constant = true;
+    if (!constant && n > 0) run.push_back(static_cast<int>(q));
+  }
+  return run;
+}
+
+// The identity order.
+void identity_order(const OpContext& ctx, int64_t n, int32_t* perm, int32_t* inv, const RadixPayload* payload)
+{
+  cudaStream_t s = ctx.stream();
+  if (n > 0) launch("iota", iota_kernel, hblocks(n), RT, 0, s, perm, n);
+  if (n > 0 && inv) launch("iota", iota_kernel, hblocks(n), RT, 0, s, inv, n);
+  if (n > 0 && payload && !payload_empty(*payload))
+    launch("copy_payload", copy_payload_kernel, hblocks(n), RT, 0, s, *payload, n);
+}
+
+}  // namespace
+
+void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
+                     int32_t* perm, std::vector<uint32_t>* hist_out, int32_t* inv, const RadixPayload* payload,
+                     const FusedKey* fused)
+{
+  const size_t P = passes.size();
+  std::vector<uint32_t> hist(P * 256, 0);
+  if (P > 0 && n > 0) {
+    Buffer<uint32_t> d_hist(ctx.alloc(), P * 256);
+    radix_histograms(ctx, passes, n, d_hist.get(), fused);
+    ctx.fetch(hist.data(), d_hist.get(), P * 256 * sizeof(uint32_t));
+    ctx.finish();
+  }
+  if (hist_out) *hist_out = hist;
+  // skip constant-digit passes; the first executed pass of a word gathers it,
+  // later passes of the same word read it carried
+  const std::vector<int> run = varying_passes(hist, P, n);
+  if (run.empty()) identity_order(ctx, n, perm, inv, payload);
+  else run_passes(ctx, passes, run, hist, n, perm, inv, payload, fused, nullptr, 8, nullptr);
+}
+
+void radix_sort_words(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, int32_t* perm,
+                      const RadixPayload* payload, Buffer<uint8_t>* words, int* word_bytes)
+{
+  cudaStream_t s = ctx.stream();
+  const int P    = (bits - f.drop + 7) / 8;
+  const int kb   = P <= 4 ? 4 : 8;
+  if (word_bytes) *word_bytes = kb;
+  std::vector<uint32_t> hist(static_cast<size_t>(P) * 256, 0);
+  Buffer<uint8_t> first;
+  if (P > 0 && n > 0) {
+    first = Buffer<uint8_t>(ctx.alloc(), static_cast<size_t>(n) * kb);
+    Buffer<uint32_t> d_hist(ctx.alloc(), hist.size());
+    LDF_CUDA(cudaMemsetAsync(d_hist.get(), 0, hist.size() * sizeof(uint32_t), s));
+    WordArgs a{};
+    a.f       = f;
+    a.n       = n;
+    a.npasses = P;
+    a.words   = first.get();
+    a.hist    = d_hist.get();
+    const unsigned g =
+      static_cast<unsigned>(std::min<int64_t>(ceil_div(n, int64_t(RT) * kWordRows), 8 * num_sms()));
+    launch("fused_words", kb == 4 ? fused_words_kernel<uint32_t> : fused_words_kernel<uint64_t>, g, RT, 0, s, a);
+    ctx.fetch(hist.data(), d_hist.get(), hist.size() * sizeof(uint32_t));
+    ctx.finish();
+  }
+  std::vector<RadixPass> passes(P);
+  for (int q = 0; q < P; ++q) {
+    passes[q].src   = DigitSrc::CARRIED;
+    passes[q].shift = 8 * q;
+  }
+  const std::vector<int> run = varying_passes(hist, P, n);
+  if (run.empty()) {
+    identity_order(ctx, n, perm, nullptr, payload);
+    if (words) *words = std::move(first);  // equal words are in order
+  } else {
+    run_passes(ctx, passes, run, hist, n, perm, nullptr, payload, &f, &first, kb, words);
+  }
+}
+
+// ---- sorting on the leading bits -----------------------------------------------
+namespace {
+
+constexpr int kSampleTies     = 1 << 17;        // sampled rows
+constexpr int kDropCands      = 7;              // passes 2 .. 8
+
+struct TieSampleArgs {
+  FusedKey f;
+  int64_t n, stride;
+  int ncand;
+  int drop[kDropCands];
+  unsigned long long* slots;  // [ncand][2 * kSampleTies]
+  unsigned int* ties;         // [ncand]
+};
+
+// ties[c] += sampled rows whose W >> drop[c] another sampled row has.
+__global__ void tie_sample_kernel(TieSampleArgs a)
+{
+  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t r = i * a.stride;
+  uint32_t low;
+  const uint64_t w = r < a.n ? fused_word(a.f, r, low) : 0;
+  for (int c = 0; c < a.ncand; ++c) {
+    bool tie = false;
+    if (r < a.n) {
+      const unsigned long long key = w >> (a.drop[c] - 8);
+      unsigned long long* s        = a.slots + static_cast<int64_t>(c) * 2 * kSampleTies;
+      uint32_t at                  = static_cast<uint32_t>(fastrange(mix64(key), 2 * kSampleTies));
+      for (int probe = 0; key != ~0ull; ++probe) {
+        unsigned long long v = *static_cast<volatile unsigned long long*>(s + at);
+        if (v == ~0ull) v = atomicCAS(s + at, ~0ull, key);
+        if (v == ~0ull) break;
+        if (v == key) {
+          tie = true;
+          break;
+        }
+        at = at + 1 == 2 * kSampleTies ? 0 : at + 1;
+      }
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, tie);
+    if (m && (threadIdx.x & 31) == 0) atomicAdd(a.ties + c, static_cast<unsigned>(__popc(m)));
+  }
+}
+
+// The bits of a row's W below f.drop.
+__device__ __forceinline__ uint64_t dropped_bits(const FusedKey& f, int64_t row)
+{
+  uint32_t low;
+  const uint64_t c = fused_word(f, row, low);
+  const int d      = f.drop - 8;  // of C; f.drop <= 64
+  return (d ? (c & (~0ull >> (64 - d))) << 8 : 0ull) | low;
+}
+
+constexpr int kTieThread = 12;  // longest run a thread orders by itself
+struct TieRun {
+  int32_t start, len;
+};
+
+// A thread per run of equal words: short runs are ordered in place by
+// insertion, longer ones listed (count[0]; count[1]: a run over kTieRunMax).
+template <typename KT>
+__global__ void __launch_bounds__(256) order_ties_kernel(FusedKey f, const KT* w, int64_t n, int32_t* perm, TieRun* runs,
+                                                         unsigned int* count)
+{
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i + 1 < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const KT x = __ldg(w + i);
+    if (x != __ldg(w + i + 1) || (i > 0 && __ldg(w + i - 1) == x)) continue;
+    int len = 2;
+    while (i + len < n && len <= kTieRunMax && __ldg(w + i + len) == x) ++len;
+    if (len > kTieThread) {
+      if (len > kTieRunMax) atomicExch(count + 1, 1u);
+      else runs[atomicAdd(count, 1u)] = TieRun{static_cast<int32_t>(i), len};
+      continue;
+    }
+    int32_t row[kTieThread];
+    uint64_t low[kTieThread];
+    for (int k = 0; k < len; ++k) {
+      const int32_t r  = perm[i + k];
+      const uint64_t l = dropped_bits(f, r);
+      int at           = k;
+      for (; at > 0 && low[at - 1] > l; --at) {
+        low[at] = low[at - 1];
+        row[at] = row[at - 1];
+      }
+      low[at] = l;
+      row[at] = r;
+    }
+    for (int k = 0; k < len; ++k) perm[i + k] = row[k];
+  }
+}
+
+// A block per listed run: each row's place counted among the run's rows.
+__global__ void __launch_bounds__(256) order_runs_kernel(FusedKey f, const TieRun* runs, int32_t* perm)
+{
+  __shared__ uint64_t low[kTieRunMax];
+  const TieRun t = runs[blockIdx.x];
+  int32_t row[kTieRunMax / 256];
+#pragma unroll
+  for (int q = 0; q < kTieRunMax / 256; ++q) {
+    const int k = q * 256 + threadIdx.x;
+    row[q]      = 0;
+    if (k < t.len) {
+      row[q] = perm[t.start + k];
+      low[k] = dropped_bits(f, row[q]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kTieRunMax / 256; ++q) {
+    const int k = q * 256 + threadIdx.x;
+    if (k >= t.len) continue;
+    const uint64_t x = low[k];
+    int at           = 0;
+    for (int j = 0; j < t.len; ++j) at += low[j] < x || (low[j] == x && j < k) ? 1 : 0;
+    perm[t.start + at] = row[q];
+  }
+}
+
+// Random reads of one 16-byte record a row: as many in flight per thread as
+// the registers hold.
+constexpr int kPermRows = 8;
+__global__ void __launch_bounds__(256) move_records_kernel(RadixPayload pay, const int32_t* perm, int64_t n)
+{
+  const int64_t per = static_cast<int64_t>(blockDim.x) * kPermRows;
+  for (int64_t base = blockIdx.x * per + threadIdx.x; base < n; base += static_cast<int64_t>(gridDim.x) * per) {
+    int32_t row[kPermRows];
+    ulonglong2 v[kPermRows];
+#pragma unroll
+    for (int k = 0; k < kPermRows; ++k) row[k] = base + k * blockDim.x < n ? __ldcs(perm + base + k * blockDim.x) : -1;
+#pragma unroll
+    for (int k = 0; k < kPermRows; ++k) v[k] = row[k] >= 0 ? __ldg(pay.packed + row[k]) : make_ulonglong2(0, 0);
+#pragma unroll
+    for (int q = 0; q < kPassPayload; ++q) {
+      if (q >= pay.nparts) break;
+#pragma unroll
+      for (int k = 0; k < kPermRows; ++k)
+        if (row[k] >= 0) st_fixed(pay.pdst[q], pay.pwidth[q], base + k * blockDim.x, record_part(v[k], pay.poff[q]));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) move_by_perm_kernel(RadixPayload pay, const int32_t* perm, int64_t n)
+{
+  const int64_t per = static_cast<int64_t>(blockDim.x) * kMoveBatch;
+  for (int64_t base = blockIdx.x * per; base < n; base += static_cast<int64_t>(gridDim.x) * per) {
+    int32_t pos[kMoveBatch], row[kMoveBatch];
+#pragma unroll
+    for (int k = 0; k < kMoveBatch; ++k) {
+      const int64_t i = base + k * blockDim.x + threadIdx.x;
+      pos[k]          = i < n ? static_cast<int32_t>(i) : -1;
+      row[k]          = i < n ? __ldg(perm + i) : 0;
+    }
+    move_payload_rows(pay, pos, row);
+  }
+}
+
+}  // namespace
+
+int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n)
+{
+  TieSampleArgs a{};
+  a.f      = f;
+  a.n      = n;
+  a.stride = ceil_div(n, kSampleTies);
+  // two passes fewer than the whole word takes, at least, and a prefix that
+  // could tell n rows apart
+  const int full = (bits + 7) / 8;
+  for (int k = 2; k <= full - 2 && k <= 8; ++k)
+    if (bits - 8 * k >= 8 && (int64_t(1) << std::min(8 * k, 62)) >= n / 16) a.drop[a.ncand++] = bits - 8 * k;
+  if (n < kDropMinRows || a.ncand == 0) return 0;
+  cudaStream_t s = ctx.stream();
+  Buffer<unsigned long long> slots(ctx.alloc(), static_cast<size_t>(a.ncand) * 2 * kSampleTies);
+  Buffer<unsigned int> ties(ctx.alloc(), kDropCands);
+  LDF_CUDA(cudaMemsetAsync(slots.get(), 0xff, slots.bytes(), s));
+  LDF_CUDA(cudaMemsetAsync(ties.get(), 0, kDropCands * sizeof(unsigned int), s));
+  a.slots = slots.get();
+  a.ties  = ties.get();
+  launch("tie_sample", tie_sample_kernel, static_cast<unsigned>(kSampleTies / 256), 256, 0, s, a);
+  unsigned int h[kDropCands];
+  ctx.fetch(h, ties.get(), sizeof(h));
+  ctx.finish();
+  // t tying rows in the sample stand for about t (n / sample)^2 tying pairs
+  // of rows; ties of a 64th of the rows or so cost less than a pass does.  A
+  // single group of rows behind up to 8 sampled ties has some 4 (n / sample)
+  // rows, which order_ties still takes at 100M rows.
+  const double pairs = static_cast<double>(a.stride) * static_cast<double>(a.stride);
+  const double most  = std::min(8.0, std::max(2.0, static_cast<double>(n) / 64 / pairs));
+  for (int c = 0; c < a.ncand; ++c)
+    if (h[c] <= most) return a.drop[c];
+  return 0;
+}
+
+bool order_ties(const OpContext& ctx, const FusedKey& f, const void* words, int word_bytes, int64_t n, int32_t* perm)
+{
+  cudaStream_t s = ctx.stream();
+  Buffer<TieRun> runs(ctx.alloc(), static_cast<size_t>(n / kTieThread + 1));
+  Buffer<unsigned int> count(ctx.alloc(), 2);
+  LDF_CUDA(cudaMemsetAsync(count.get(), 0, 2 * sizeof(unsigned int), s));
+  const unsigned g = static_cast<unsigned>(std::min<int64_t>(ceil_div(n, 256), 16 * num_sms()));
+  if (word_bytes == 4)
+    launch("order_ties", order_ties_kernel<uint32_t>, g, 256, 0, s, f, static_cast<const uint32_t*>(words), n, perm,
+           runs.get(), count.get());
+  else
+    launch("order_ties", order_ties_kernel<unsigned long long>, g, 256, 0, s, f,
+           static_cast<const unsigned long long*>(words), n, perm, runs.get(), count.get());
+  unsigned int h[2];
+  ctx.fetch(h, count.get(), sizeof(h));
+  ctx.finish();
+  if (h[1]) return false;
+  if (h[0])
+    launch("order_runs", order_runs_kernel, h[0], 256, 0, s, f, static_cast<const TieRun*>(runs.get()), perm);
+  return true;
+}
+
+void move_by_perm(const OpContext& ctx, const RadixPayload& payload, const int32_t* perm, int64_t n)
+{
+  if (n == 0 || payload_empty(payload)) return;
+  RadixPayload rest = payload;
+  if (payload.nparts) {
+    launch("move_records", move_records_kernel,
+           static_cast<unsigned>(std::min<int64_t>(ceil_div(n, int64_t(256) * kPermRows), 16 * num_sms())), 256, 0,
+           ctx.stream(), payload, perm, n);
+    rest.nparts = 0;
+  }
+  if (!payload_empty(rest))
+    launch("move_by_perm", move_by_perm_kernel,
+           static_cast<unsigned>(std::min<int64_t>(ceil_div(n, int64_t(256) * kMoveBatch), 16 * num_sms())), 256, 0,
+           ctx.stream(), rest, perm, n);
 }
 
 }  // namespace ldf
@@ -883,13 +1324,12 @@ void radix_histogram_raw(cudaStream_t s, const RadixPass& p, int64_t n, uint32_t
   launch("histogram", histogram_kernel<false>, hist_blocks(n), RT, 0, s, h);
 }
 
-int64_t radix_status_words(int64_t n) { return ceil_div(n, RTILE) * 256 + 2; }
+int64_t radix_status_words(int64_t n) { return ceil_div(status_words(n), int64_t(2)); }
 
 void onesweep_gather_pass_raw(cudaStream_t s, const RadixPass& p, int64_t n, int32_t* rows_out,
                               const uint64_t* d_bases, uint64_t* status, int* err)
 {
   if (n <= 0) return;
-  const int64_t tiles = ceil_div(n, RTILE);
   PassArgs a{};
   a.p          = p;
   a.n          = n;
@@ -898,10 +1338,9 @@ void onesweep_gather_pass_raw(cudaStream_t s, const RadixPass& p, int64_t n, int
   a.vals_in    = nullptr;
   a.vals_out   = rows_out;
   a.digit_base = d_bases;
-  a.status     = status;
-  a.counter    = reinterpret_cast<unsigned long long*>(status + tiles * 256);
+  a.status     = reinterpret_cast<uint32_t*>(status);
   a.err        = err;
-  launch_onesweep<true, false>(s, static_cast<unsigned>(tiles), a);
+  launch_onesweep<true, false>(s, a);
 }
 
 }  // namespace ldf

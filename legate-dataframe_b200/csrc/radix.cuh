@@ -15,7 +15,7 @@ constexpr int kRadixMinBlocks = 4;
 
 // How a pass obtains the digit of a row.
 enum class DigitSrc : int {
-  CARRIED = 0,  // byte `shift/8` of the carried key word
+  CARRIED = 0,  // byte `shift/8` of the carried key word (written beforehand: radix_sort_words)
   COLUMN  = 1,  // load the key column at the row, transform, then byte
   CLASS   = 2,  // 0/1/2 class of the row: value / NaN / null, ordered by nulls_at_end
   BUCKET  = 3,  // hash of the key columns % nparts (then byte)
@@ -99,26 +99,50 @@ struct RadixPass {
   uint32_t nparts;    // BUCKET
 };
 
-// Several sort keys without nulls or floating-point values packed into one
-// word, least significant key first: W = sum_k (word_k - min_k) << off_k,
-// word_k the key's order-preserving word (inverted when descending) and
-// min_k its minimum over the rows, at most kFusedMaxBits bits in all.  The
-// pass of W's low byte loads every key at the row and carries C = W >> 8
-// (64 bits); the later passes take byte shift / 8 of C.  One word for all
-// the keys means that no pass gathers a key column through the permutation.
+// Several sort keys packed into one word, least significant key first: W =
+// sum_k code_k << off_k, at most kFusedMaxBits bits in all.  code_k is
+// word_k - min_k, word_k the key's order-preserving word (inverted when
+// descending) and min_k its minimum over the rows; a key with nulls or NaNs
+// takes two codes more, before or behind its values (fused_code).  With `drop`
+// (0, or 8 and more) the low `drop` bits are left out and W >> drop sorted.
+// A word of at most 64 bits is written by one pass over the key columns, which
+// counts all its digits too (radix_sort_words).  Of a wider one the pass of
+// the low byte loads every key at the row and carries C = W >> 8; the later
+// passes take byte shift / 8 of C.  One word for all the keys means that no
+// pass gathers a key column through the permutation.
 constexpr int kFuseMax      = 4;
 constexpr int kFusedMaxBits = 72;
 struct FusedKey {
   int n;
   SortKeyDesc key[kFuseMax];
   uint64_t min[kFuseMax];
+  uint64_t span[kFuseMax];  // largest word - min
   int off[kFuseMax];
+  int has_class[kFuseMax];
+  int drop;
 };
 
-// Minimum and maximum of the order-preserving words of `keys` (no nulls)
-// over n rows, one read of each column.
+// Minimum and maximum of the order-preserving words of `keys` over n rows,
+// nulls and NaNs aside (~0 and 0 when there are no others), one read of each
+// column.
 void sort_word_ranges(const OpContext& ctx, const SortKeyDesc* keys, int nkeys, int64_t n, uint64_t* mn,
                       uint64_t* mx);
+
+// Fewest rows for which bits are dropped: below, the sample and its read-back
+// cost what they save.
+constexpr int64_t kDropMinRows = int64_t(1) << 21;
+
+// Dropped bits (0: none) with which sorting on the rest of the fused word of
+// `bits` bits, and then ordering the few rows that tie on it, takes fewest
+// passes: from the ties among a sample of the rows.
+int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n);
+
+// Orders the rows of every run of equal `words` (the sorted W >> f.drop, 4 or
+// 8 bytes each) in `perm` by the dropped bits, equal rows in the order they
+// have.  False when a run is longer than kTieRunMax (perm is then no longer
+// useful).
+constexpr int kTieRunMax = 4096;
+bool order_ties(const OpContext& ctx, const FusedKey& f, const void* words, int word_bytes, int64_t n, int32_t* perm);
 
 // Stable sort of rows by a list of passes (least significant first).
 // Returns the permutation (row ids) in `perm` (n entries, caller allocated).
@@ -162,6 +186,16 @@ inline bool payload_empty(const RadixPayload& p) { return p.n == 0 && p.nparts =
 void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
                      int32_t* perm, std::vector<uint32_t>* hist_out = nullptr, int32_t* inv = nullptr,
                      const RadixPayload* payload = nullptr, const FusedKey* fused = nullptr);
+
+// The same on the fused word W >> f.drop of at most 64 bits (W has `bits`).
+// `words` (optional, instead of a payload): the sorted words, *word_bytes each
+// (4 when they have at most 32 bits, else 8).
+void radix_sort_words(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, int32_t* perm,
+                      const RadixPayload* payload, Buffer<uint8_t>* words = nullptr, int* word_bytes = nullptr);
+
+// The payload's columns gathered through `perm` (payload.dst[position] =
+// src[perm[position]]).
+void move_by_perm(const OpContext& ctx, const RadixPayload& payload, const int32_t* perm, int64_t n);
 
 // ---- small inputs (rank_sort.cu) -----------------------------------------
 // The whole sort of a table of at most kRankSortRows rows in one or two

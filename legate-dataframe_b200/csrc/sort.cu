@@ -615,9 +615,10 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
   std::vector<Buffer<int32_t>> reps;                   // representative rows of string keys
   std::vector<const int32_t*> rep_of(ncols, nullptr);  // per table column
   std::vector<RadixPass> passes;
+  int fused_bits = 0;
   std::vector<SortKeyDesc> kd;  // least significant key first
   std::vector<int64_t> ndistinct;  // string keys: distinct strings (their ranks' range); -1 otherwise
-  bool fusable = nkeys >= 2 && nkeys <= kFuseMax;
+  bool fusable = nkeys >= 2 || n >= kDropMinRows;
   for (int j = nkeys - 1; j >= 0; --j) {
     const ldf_column& c = table[keys[j]];
     SortKeyDesc k{};
@@ -640,16 +641,19 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
       ndistinct.push_back(-1);
     }
     k.key_bytes = k.col.width;
-    if (c.valid != nullptr || is_float(c.type)) fusable = false;  // those need CLASS passes
+    if (c.valid != nullptr || is_float(c.type)) fusable = true;  // instead of a CLASS pass
     kd.push_back(k);
   }
+  if (nkeys > kFuseMax) fusable = false;
   if (rank_sort(ctx, table, ncols, kd, n, first, rows, out)) {
     ctx.finish();
     return;
   }
-  // Keys without nulls or floats whose value ranges fit one word of at most
-  // kFusedMaxBits bits are sorted on that word: its first pass loads every key
-  // in input order, and no pass gathers a key through the permutation.
+  // Keys whose value ranges fit one word of at most kFusedMaxBits bits are
+  // sorted on that word: its first pass loads every key in input order, and no
+  // pass gathers a key through the permutation and none orders the nulls.  A
+  // single key without nulls or NaNs gains from it only by dropping bits, so
+  // small inputs skip the range.
   FusedKey fk{};
   bool fused = false;
   if (fusable && n > 0) {
@@ -672,24 +676,30 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
       uint64_t smn[kFuseMax], smx[kFuseMax];
       sort_word_ranges(ctx, scan.data(), static_cast<int>(scan.size()), n, smn, smx);
       for (size_t q = 0; q < scan.size(); ++q) {
-        mn[scan_of[q]] = smn[q];
+        mn[scan_of[q]] = std::min(smn[q], smx[q]);  // no values at all: (~0, 0)
         mx[scan_of[q]] = smx[q];
       }
     }
     int bits = 0;
-    fk.n     = static_cast<int>(kd.size());
+    bool fits = true;
+    fk.n      = static_cast<int>(kd.size());
     for (int k = 0; k < fk.n; ++k) {
-      const uint64_t span = mx[k] - mn[k];
-      int b               = 0;
-      while (b < 64 && (span >> b) != 0) ++b;
-      fk.key[k] = kd[k];
-      fk.min[k] = mn[k];
+      fk.key[k]       = kd[k];
+      fk.min[k]       = mn[k];
+      fk.span[k]      = mx[k] - mn[k];
+      fk.has_class[k] = kd[k].col.valid != nullptr || is_float(kd[k].col.type) ? 1 : 0;
+      if (fk.has_class[k] && fk.span[k] > ~0ull - 2) fits = false;  // no room for the two codes
+      const uint64_t top = fk.span[k] + (fk.has_class[k] ? 2 : 0);
+      int b              = 0;
+      while (b < 64 && (top >> b) != 0) ++b;
       fk.off[k] = bits;
       bits += b;
     }
-    if (bits <= kFusedMaxBits) {
-      fused = true;
-      for (int q = 0; 8 * q < bits; ++q) {
+    if (fits && bits <= kFusedMaxBits) {
+      fused       = true;
+      fk.drop    = choose_drop(ctx, fk, bits, n);
+      fused_bits = bits;
+      for (int q = 0; bits > 64 && 8 * q < bits; ++q) {  // a wider word: pass by pass (FusedKey)
         RadixPass p{};
         p.src       = DigitSrc::FUSED;
         p.fused_low = q == 0 ? 1 : 0;
@@ -710,10 +720,23 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
       }
     }
   }
-  const FusedKey* fkp = fused ? &fk : nullptr;
   Buffer<int32_t> perm(al, std::max<int64_t>(n, 1));
+  // the leading bits, then the ties among them; true when `perm` is done
+  auto sort_leading = [&]() {
+    if (!fused || fk.drop == 0) return false;
+    Buffer<uint8_t> words;
+    int word_bytes = 0;
+    radix_sort_words(ctx, fk, fused_bits, n, perm.get(), nullptr, &words, &word_bytes);
+    if (order_ties(ctx, fk, words.get(), word_bytes, n, perm.get())) return true;
+    fk.drop = 0;  // too many rows tie: the whole word after all
+    return false;
+  };
+  auto sort_all = [&](const RadixPayload* pay) {
+    if (fused && fused_bits <= 64) radix_sort_words(ctx, fk, fused_bits, n, perm.get(), pay);
+    else radix_sort_rows(ctx, passes, n, perm.get(), nullptr, nullptr, pay, fused ? &fk : nullptr);
+  };
   if (!whole) {
-    radix_sort_rows(ctx, passes, n, perm.get(), nullptr, nullptr, nullptr, fkp);
+    if (!sort_leading()) sort_all(nullptr);
     gather_table(ctx, table, ncols, perm.get() + first, rows, out);
     ctx.finish();
     return;
@@ -726,7 +749,8 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
   plan_pass_move(al, table, ncols, n, out, mv, &rep_of);
   Buffer<ulonglong2> rec;
   const RadixPayload pay = pack_payload(ctx, mv.pay, n, rec);
-  radix_sort_rows(ctx, passes, n, perm.get(), nullptr, nullptr, &pay, fkp);
+  if (sort_leading()) move_by_perm(ctx, pay, perm.get(), n);
+  else sort_all(&pay);
   move_strings_in_order(ctx, table, mv, n, out);
   std::vector<DCol> fsrc;
   std::vector<ldf_column*> fdst;
