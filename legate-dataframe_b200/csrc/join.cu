@@ -515,17 +515,25 @@ constexpr int probe_min_blocks()
 // (unique build keys, semi and anti joins): a tile claims its output range
 // with one atomic on the running total, so no tile waits on another and
 // output rows come in tile completion order.
+// A tile's output rows are in the order of its probe rows (item i of all
+// threads, then item i + 1), so that the lanes of a store write side by side;
+// with each thread's rows side by side instead, a store of 32 lanes touched
+// three times the sectors.
 template <KeyMode M>
 __global__ void __launch_bounds__(kProbeThreads, (probe_min_blocks<M>()))
 probe_kernel(ProbeArgs a)
 {
-  __shared__ int64_t s_scan[kProbeThreads / 32 + 1];
+  constexpr int kWarps = kProbeThreads / 32;
+  static_assert(kProbeItems * kWarps == 32, "one warp scans the counts of all items and warps");
+  __shared__ uint32_t s_count[32];  // output rows of item i of warp w at [i * kWarps + w], then the rows before
   __shared__ uint64_t s_prefix;
   const int64_t tile = static_cast<int64_t>(blockIdx.x);
   const int64_t base = tile * kProbeTile;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int jt   = a.join_type;
 
   int64_t first[kProbeItems];
-  int64_t cnt = 0;
+  uint32_t emits[kProbeItems];  // lanes with an output row
   if (M != KeyMode::GEN) {
     // touch every item's first slot before resolving any: the loads overlap
     // and the resolving walks below mostly hit L1
@@ -539,36 +547,36 @@ probe_kernel(ProbeArgs a)
   for (int i = 0; i < kProbeItems; ++i) {
     const int64_t r = base + i * kProbeThreads + threadIdx.x;
     first[i]        = -1;
-    if (r < a.n_probe) {
-      find_slot<M>(a.t, a.pk, r, &first[i]);
-      cnt += out_rows(a.join_type, first[i] >= 0 ? 1 : 0);
-    }
+    if (r < a.n_probe) find_slot<M>(a.t, a.pk, r, &first[i]);
+    __syncwarp();
+    emits[i] = __ballot_sync(0xffffffffu, r < a.n_probe && out_rows(jt, first[i] >= 0 ? 1 : 0) != 0);
+    if (lane == 0) s_count[i * kWarps + warp] = __popc(emits[i]);
   }
-  int64_t tile_total;
-  int64_t excl = block_exclusive_scan<int64_t, kProbeThreads>(cnt, s_scan, &tile_total);
-  if (threadIdx.x == 0)
-    s_prefix = tile_total > 0 ? atomicAdd(reinterpret_cast<unsigned long long*>(a.total),
-                                          static_cast<unsigned long long>(tile_total))
-                              : 0;
   __syncthreads();
-  int64_t pos  = static_cast<int64_t>(s_prefix) + excl;
-  const int jt = a.join_type;
+  if (warp == 0) {
+    const uint32_t c   = s_count[lane];
+    const uint32_t inc = warp_inclusive_scan(c);
+    s_count[lane]      = inc - c;
+    if (lane == 31)
+      s_prefix = inc > 0 ? atomicAdd(reinterpret_cast<unsigned long long*>(a.total), static_cast<unsigned long long>(inc))
+                         : 0;
+  }
+  __syncthreads();
   const bool semi = jt == LDF_JOIN_SEMI || jt == LDF_JOIN_ANTI;
+  int64_t opos[kProbeItems];
+#pragma unroll
+  for (int i = 0; i < kProbeItems; ++i)
+    opos[i] = (emits[i] >> lane) & 1u ? static_cast<int64_t>(s_prefix) + s_count[i * kWarps + warp] +
+                                          __popc(emits[i] & ((1u << lane) - 1u))
+                                      : -1;
   if (M != KeyMode::GEN && a.lmap == nullptr) {
     // batched, column-wise emit
-    int64_t opos[kProbeItems], lrow[kProbeItems], brow[kProbeItems];
+    int64_t lrow[kProbeItems], brow[kProbeItems];
 #pragma unroll
     for (int i = 0; i < kProbeItems; ++i) {
-      const int64_t r = base + i * kProbeThreads + threadIdx.x;
-      opos[i]         = -1;
-      lrow[i]         = r;
-      brow[i]         = -1;
-      if (r >= a.n_probe) continue;
-      if (!semi && first[i] >= 0) {
-        brow[i] = first[i];
-        if (a.matched && !a.matched[first[i]]) a.matched[first[i]] = 1;  // hot rows: read, no write
-      }
-      if (out_rows(jt, first[i] >= 0 ? 1 : 0) != 0) opos[i] = pos++;
+      lrow[i] = base + i * kProbeThreads + threadIdx.x;
+      brow[i] = semi || opos[i] < 0 ? -1 : first[i];
+      if (brow[i] >= 0 && a.matched && !a.matched[brow[i]]) a.matched[brow[i]] = 1;  // hot rows: read, no write
     }
     emit_batch(a.lo, opos, lrow);
     emit_build_batch(a, opos, lrow, brow);
@@ -576,9 +584,8 @@ probe_kernel(ProbeArgs a)
   }
 #pragma unroll
   for (int i = 0; i < kProbeItems; ++i) {
-    const int64_t r = base + i * kProbeThreads + threadIdx.x;
-    if (r >= a.n_probe || out_rows(jt, first[i] >= 0 ? 1 : 0) == 0) continue;
-    emit(a, pos++, r, semi ? -1 : first[i]);
+    if (opos[i] < 0) continue;
+    emit(a, opos[i], base + i * kProbeThreads + threadIdx.x, semi ? -1 : first[i]);
     if (!semi && first[i] >= 0 && a.matched && !a.matched[first[i]]) a.matched[first[i]] = 1;
   }
 }
