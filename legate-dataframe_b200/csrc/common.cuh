@@ -102,12 +102,12 @@ inline void launch_cluster(const char* name, void (*kernel)(KArgs...), unsigned 
 // Device memory of one call.  allocate/deallocate go straight to the
 // caller's allocator (outputs use them: the caller owns what they return).
 // Scratch buffers (Buffer<T>) of at most kSmallScratch bytes are carved from
-// kScratchChunk-byte chunks instead, which are handed back when the Allocator
-// is destroyed at the end of the call: one allocator round trip per chunk
-// rather than per buffer.
+// chunks of kScratchChunk bytes (four times that from the second on) instead,
+// which are handed back when the Allocator is destroyed at the end of the call:
+// one allocator round trip per chunk rather than per buffer.
 class Allocator {
  public:
-  static constexpr size_t kSmallScratch = size_t(1) << 20;
+  static constexpr size_t kSmallScratch = size_t(8) << 20;
   static constexpr size_t kScratchChunk = size_t(16) << 20;
 
   Allocator(const ldf_allocator* a, cudaStream_t s) : a_(a), s_(s) {}
@@ -123,7 +123,7 @@ class Allocator {
  private:
   const ldf_allocator* a_;
   cudaStream_t s_;
-  mutable std::vector<void*> chunks_;
+  mutable std::vector<std::pair<void*, size_t>> chunks_;
   mutable char* bump_  = nullptr;
   mutable size_t left_ = 0;
 };

@@ -130,9 +130,10 @@ void* Allocator::allocate_scratch(size_t nbytes) const
   nbytes = (nbytes + 255) & ~size_t(255);
   if (nbytes > kSmallScratch) return allocate(nbytes);
   if (left_ < nbytes) {
-    bump_ = static_cast<char*>(allocate(kScratchChunk));
-    chunks_.push_back(bump_);
-    left_ = kScratchChunk;
+    const size_t chunk = chunks_.empty() ? kScratchChunk : 4 * kScratchChunk;
+    bump_              = static_cast<char*>(allocate(chunk));
+    chunks_.emplace_back(bump_, chunk);
+    left_ = chunk;
   }
   void* p = bump_;
   bump_ += nbytes;
@@ -151,7 +152,7 @@ void Allocator::deallocate_scratch(void* p, size_t nbytes) const
 
 Allocator::~Allocator()
 {
-  for (void* c : chunks_) deallocate(c, kScratchChunk);
+  for (auto& c : chunks_) deallocate(c.first, c.second);
 }
 
 // ---------------------------------------------------------------------------

@@ -775,11 +775,14 @@ __global__ void bucket_ids_kernel(KeyCols k, int64_t n, uint32_t nparts, uint32_
 {
   extern __shared__ unsigned int sc[];
   const bool use_smem = nparts <= 8192;
+  const bool pow2     = (nparts & (nparts - 1)) == 0;
   if (use_smem)
     for (uint32_t i = threadIdx.x; i < nparts; i += blockDim.x) sc[i] = 0;
   __syncthreads();
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t b = static_cast<uint32_t>(key_bits<KeyMode::GEN>(k, r) % nparts);
+    const uint64_t h = key_bits<KeyMode::GEN>(k, r);
+    // a 64-bit division is about a third of the work of a string row
+    const uint32_t b = static_cast<uint32_t>(pow2 ? h & (nparts - 1) : h % nparts);
     ids[r]           = b;
     if (use_smem) atomicAdd(&sc[b], 1u);
     else atomicAdd(&counts[b], 1ull);
