@@ -8,6 +8,8 @@
 // the histograms.
 #include "radix.cuh"
 
+#include <algorithm>
+
 namespace ldf {
 namespace {
 
@@ -21,10 +23,10 @@ constexpr int RW    = RT / 32;
 // words (0.65 ms now, with 4-byte status words and full tiles loaded without
 // bounds), and 8-byte words were fastest with 16 (20 spill).  Passes that load their word from the
 // columns hold more per row and stay at 12.
-template <bool GATHER, typename KT>
+template <bool GATHER, typename KT, typename VT>
 __host__ __device__ constexpr int radix_items()
 {
-  return GATHER ? kRadixItems : sizeof(KT) == 4 ? 20 : 16;
+  return GATHER || sizeof(VT) == 8 ? kRadixItems : sizeof(KT) == 4 ? 20 : 16;
 }
 template <bool GATHER>
 __host__ __device__ constexpr int radix_min_blocks()
@@ -181,8 +183,8 @@ struct PassArgs {
   int64_t n;
   const void* keys_in;  // carried words, KT each
   void* keys_out;
-  const int32_t* vals_in;  // null: identity
-  int32_t* vals_out;
+  const void* vals_in;  // VT each: row ids (null: identity), or the rows' other values (radix_sort_pairs)
+  void* vals_out;
   const uint64_t* digit_base;  // [256]
   uint32_t* status;            // [tiles * 256] (tile_status)
   unsigned long long* counter;
@@ -371,10 +373,10 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d)
 //
 // The bound of a pass on carried words is its instructions (about 140 per row
 // and warp, half the issue slots; DRAM 25 %), most of them the ranking.
-template <bool WRITE_KEYS, bool MOVE, typename KT, int RI>
+template <bool WRITE_KEYS, bool MOVE, typename KT, typename VT, int RI>
 __device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile, KT (&key)[RI],
-                                                 int32_t (&val)[RI], uint32_t (&dr)[RI], OsShared& sh,
-                                                 KT* s_keys, int32_t* s_vals, uint8_t* s_dig)
+                                                 VT (&val)[RI], uint32_t (&dr)[RI], OsShared& sh,
+                                                 KT* s_keys, VT* s_vals, uint8_t* s_dig)
 {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t lt_mask = (1u << lane) - 1u;
@@ -473,7 +475,7 @@ __device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile
     for (int j = threadIdx.x; j < cnt; j += RT) {
       const int32_t pos = sh.delta[s_dig[j]] + j;
       if (WRITE_KEYS) static_cast<KT*>(a.keys_out)[pos] = s_keys[j];
-      a.vals_out[pos] = s_vals[j];
+      static_cast<VT*>(a.vals_out)[pos] = s_vals[j];
       if (a.inv_out) a.inv_out[s_vals[j]] = static_cast<int32_t>(pos);
     }
   } else {
@@ -489,8 +491,8 @@ __device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile
         row[k]      = 0;
         if (j < cnt) {
           pos[k]           = sh.delta[s_dig[j]] + j;
-          row[k]           = s_vals[j];
-          a.vals_out[pos[k]] = row[k];
+          row[k]           = static_cast<int32_t>(s_vals[j]);
+          static_cast<int32_t*>(a.vals_out)[pos[k]] = row[k];
           if (a.inv_out) a.inv_out[row[k]] = pos[k];
         }
       }
@@ -503,22 +505,23 @@ __device__ __forceinline__ void rank_and_scatter(const PassArgs& a, int64_t tile
 // the columns at the row, the first pass of a word; otherwise the carried key).
 // In a pass on the carried word, all row ids and then all words are loaded
 // before any digit is taken, so that the thread's loads are in flight together.
-template <bool GATHER, bool FUSEDG, typename KT, int RI>
+template <bool GATHER, bool FUSEDG, typename KT, typename VT, int RI>
 __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, KT (&key)[RI],
-                                               int32_t (&val)[RI], uint32_t (&dr)[RI])
+                                               VT (&val)[RI], uint32_t (&dr)[RI])
 {
+  const VT* vals_in = static_cast<const VT*>(a.vals_in);
   constexpr int RTILE = RT * RI;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t wbase = tile * RTILE + warp * (32 * RI) + lane;
   if (!GATHER && a.p.src != DigitSrc::CLASS && (tile + 1) * RTILE <= a.n) {  // a full tile: no bounds
     const KT* k = static_cast<const KT*>(a.keys_in) + wbase;
-    if (a.vals_in) {
-      const int32_t* v = a.vals_in + wbase;
+    if (vals_in) {
+      const VT* v = vals_in + wbase;
 #pragma unroll
       for (int i = 0; i < RI; ++i) val[i] = __ldg(v + i * 32);
     } else {
 #pragma unroll
-      for (int i = 0; i < RI; ++i) val[i] = static_cast<int32_t>(wbase) + i * 32;
+      for (int i = 0; i < RI; ++i) val[i] = static_cast<VT>(wbase) + i * 32;
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) key[i] = __ldg(k + i * 32);
@@ -530,7 +533,7 @@ __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, 
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const int64_t idx = wbase + i * 32;
-      val[i] = idx < a.n ? (a.vals_in ? __ldg(a.vals_in + idx) : static_cast<int32_t>(idx)) : 0;
+      val[i] = idx < a.n ? (vals_in ? __ldg(vals_in + idx) : static_cast<VT>(idx)) : 0;
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -549,7 +552,7 @@ __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, 
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const int64_t idx = wbase + i * 32;
-      val[i] = idx < a.n ? (a.vals_in ? __ldg(a.vals_in + idx) : static_cast<int32_t>(idx)) : -1;
+      val[i] = idx < a.n ? (vals_in ? __ldg(vals_in + idx) : static_cast<VT>(idx)) : -1;
       c[i]   = 0;
       dr[i]  = 0;
     }
@@ -592,8 +595,8 @@ __device__ __forceinline__ void load_tile_rows(const PassArgs& a, int64_t tile, 
     val[i]            = 0;
     dr[i]             = 255;
     if (idx < a.n) {
-      const int64_t row = a.vals_in ? a.vals_in[idx] : idx;
-      val[i]            = static_cast<int32_t>(row);
+      const int64_t row = vals_in ? vals_in[idx] : idx;
+      val[i]            = static_cast<VT>(row);
       if (a.p.src == DigitSrc::CLASS) {
         dr[i] = class_digit(a.p.key, row);
       } else {
@@ -663,29 +666,30 @@ bool pass_columns_on_device(const RadixPass& p, const FusedKey* fused)
 // moves a.pay's columns (the last pass only, which carries no word).  KT: the
 // carried word, 4 bytes when that holds it: 8 instead of 12 bytes a row read
 // and written in every pass.
-template <bool GATHER, bool WRITE_KEYS, bool MOVE, bool FUSEDG, typename KT>
+template <bool GATHER, bool WRITE_KEYS, bool MOVE, bool FUSEDG, typename KT, typename VT>
 __global__ void __launch_bounds__(RT, radix_min_blocks<GATHER>()) onesweep_kernel(PassArgs a)
 {
-  constexpr int RI    = radix_items<GATHER, KT>();
+  constexpr int RI    = radix_items<GATHER, KT, VT>();
   constexpr int RTILE = RT * RI;
   __shared__ OsShared sh;
-  // staged tile (dynamic): [keys KT x RTILE when carried][rows i32 x RTILE][digits u8 x RTILE]
+  // staged tile (dynamic): [keys KT x RTILE when carried][values VT x RTILE][digits u8 x RTILE]
   extern __shared__ __align__(16) unsigned char s_stage[];
   KT* s_keys      = reinterpret_cast<KT*>(s_stage);
-  int32_t* s_vals = reinterpret_cast<int32_t*>(s_stage + (WRITE_KEYS ? RTILE * sizeof(KT) : 0));
+  VT* s_vals      = reinterpret_cast<VT*>(s_stage + (WRITE_KEYS ? RTILE * sizeof(KT) : 0));
   uint8_t* s_dig  = reinterpret_cast<uint8_t*>(s_vals + RTILE);
 
   const int64_t tile = next_tile_id(a.counter, &sh.tile[0]);
   for (int i = threadIdx.x; i < RW * 256; i += RT) (&sh.whist[0][0])[i] = 0;
   __syncthreads();
   KT key[RI];
-  int32_t val[RI];
+  VT val[RI];
   uint32_t dr[RI];
   if (a.pf_ahead > 0 && threadIdx.x == 0 && (tile + a.pf_ahead) * RTILE < a.n) {
     const int64_t lo = (tile + a.pf_ahead) * RTILE;
     const int64_t hi = min(lo + static_cast<int64_t>(RTILE), a.n);
     if (!GATHER) {
-      if (a.vals_in) l2_prefetch_bulk(a.vals_in, lo * 4, hi * 4);
+      constexpr int64_t vb = sizeof(VT);
+      if (a.vals_in) l2_prefetch_bulk(a.vals_in, lo * vb, hi * vb);
       if (a.p.src != DigitSrc::CLASS)
         l2_prefetch_bulk(a.keys_in, lo * static_cast<int64_t>(sizeof(KT)), hi * static_cast<int64_t>(sizeof(KT)));
     } else if (a.pf_columns && a.vals_in == nullptr) {  // rows in input order: the key columns are read in order
@@ -698,20 +702,21 @@ __global__ void __launch_bounds__(RT, radix_min_blocks<GATHER>()) onesweep_kerne
       }
     }
   }
-  load_tile_rows<GATHER, FUSEDG, KT, RI>(a, tile, key, val, dr);
-  rank_and_scatter<WRITE_KEYS, MOVE, KT, RI>(a, tile, key, val, dr, sh, s_keys, s_vals, s_dig);
+  load_tile_rows<GATHER, FUSEDG, KT, VT, RI>(a, tile, key, val, dr);
+  rank_and_scatter<WRITE_KEYS, MOVE, KT, VT, RI>(a, tile, key, val, dr, sh, s_keys, s_vals, s_dig);
 }
 
 // Runs the pass over a.n rows; clears the status words and the tile counter
 // behind them first.
-template <bool GATHER, bool WRITE_KEYS, bool MOVE = false, bool FUSEDG = false, typename KT = uint64_t>
+template <bool GATHER, bool WRITE_KEYS, bool MOVE = false, bool FUSEDG = false, typename KT = uint64_t,
+          typename VT = int32_t>
 void launch_onesweep(cudaStream_t s, PassArgs& a)
 {
   static_assert(!(MOVE && WRITE_KEYS), "the pass that moves columns is the last one");
-  constexpr int64_t tile_rows = RT * radix_items<GATHER, KT>();
-  constexpr size_t smem = (WRITE_KEYS ? tile_rows * sizeof(KT) : 0) + tile_rows * (sizeof(int32_t) + 1);
+  constexpr int64_t tile_rows = RT * radix_items<GATHER, KT, VT>();
+  constexpr size_t smem = (WRITE_KEYS ? tile_rows * sizeof(KT) : 0) + tile_rows * (sizeof(VT) + 1);
   const int64_t tiles   = ceil_div(a.n, tile_rows);
-  auto kernel           = onesweep_kernel<GATHER, WRITE_KEYS, MOVE, FUSEDG, KT>;
+  auto kernel           = onesweep_kernel<GATHER, WRITE_KEYS, MOVE, FUSEDG, KT, VT>;
   a.counter             = reinterpret_cast<unsigned long long*>(a.status + tiles * 256);
   a.pf_ahead            = prefetch_ahead() ? int64_t(num_sms()) * radix_min_blocks<GATHER>() : 0;
   LDF_CUDA(cudaMemsetAsync(a.status, 0, (tiles * 256 + 2) * sizeof(uint32_t), s));
@@ -924,10 +929,12 @@ __global__ void __launch_bounds__(RT) fused_words_kernel(WordArgs a)
 
 // The passes `run` (none of a constant digit) of `passes`, in order; hist: all
 // passes' digit counts.  first_words: the word that the first pass carries
-// (null: it is loaded from the columns), kb bytes.
+// (null: it is loaded from the columns), kb bytes.  first_vals: the rows' values
+// of vb bytes (null: their ids), which go to `perm` in the end.
 void run_passes(const OpContext& ctx, const std::vector<RadixPass>& passes, const std::vector<int>& run,
-                const std::vector<uint32_t>& hist, int64_t n, int32_t* perm, int32_t* inv, const RadixPayload* payload,
-                const FusedKey* fused, Buffer<uint8_t>* first_words, size_t kb, Buffer<uint8_t>* words)
+                const std::vector<uint32_t>& hist, int64_t n, void* perm, int32_t* inv, const RadixPayload* payload,
+                const FusedKey* fused, Buffer<uint8_t>* first_words, size_t kb, Buffer<uint8_t>* words,
+                const void* first_vals = nullptr, size_t vb = 4)
 {
   const Allocator& al = ctx.alloc();
   cudaStream_t s      = ctx.stream();
@@ -944,13 +951,13 @@ void run_passes(const OpContext& ctx, const std::vector<RadixPass>& passes, cons
 
   Buffer<uint32_t> status(al, status_words(n));
   Buffer<uint8_t> keys[2] = {Buffer<uint8_t>(al, n * kb), first_words ? std::move(*first_words) : Buffer<uint8_t>(al, n * kb)};
-  Buffer<int32_t> vals_tmp(al, n);
+  Buffer<uint8_t> vals_tmp(al, n * vb);
   // ping-pong so that the last pass writes into `perm`
-  int32_t* vbuf[2];
+  void* vbuf[2];
   const bool odd = run.size() % 2 == 1;
   vbuf[0]        = odd ? perm : vals_tmp.get();
   vbuf[1]        = odd ? vals_tmp.get() : perm;
-  const int32_t* vin = nullptr;
+  const void* vin = first_vals;
   const void* kin    = first_words ? keys[1].get() : nullptr;
   for (size_t k = 0; k < run.size(); ++k) {
     const RadixPass& p    = passes[run[k]];
@@ -972,7 +979,9 @@ void run_passes(const OpContext& ctx, const std::vector<RadixPass>& passes, cons
     a.err        = ctx.err();
     a.pf_columns = gather && k == 0 && prefetch_first_pass() && pass_columns_on_device(p, fused) ? 1 : 0;
     const bool move = !payload_empty(a.pay);
-    if (kb == 4) {
+    if (vb == 8) {
+      launch_onesweep<false, true, false, false, uint64_t, int64_t>(s, a);
+    } else if (kb == 4) {
       if (move) launch_onesweep<false, false, true, false, uint32_t>(s, a);
       else if (write_keys) launch_onesweep<false, true, false, false, uint32_t>(s, a);
       else launch_onesweep<false, false, false, false, uint32_t>(s, a);
@@ -1088,10 +1097,15 @@ struct TieSampleArgs {
   int ncand;
   int drop[kDropCands];
   unsigned long long* slots;  // [ncand][2 * kSampleTies]
+  unsigned int* same;         // [ncand][2 * kSampleTies], or null: sampled rows of the slot's word after the first
   unsigned int* ties;         // [ncand]
+  unsigned int* most;         // [ncand]
 };
 
-// ties[c] += sampled rows whose W >> drop[c] another sampled row has.
+// ties[c] += sampled rows whose W >> drop[c] another sampled row has.  With
+// `same`, pairs of such rows, and most[c] the most rows that share one (both
+// no longer exact past kSameMax rows, which no rule accepts).
+constexpr unsigned int kSameMax = 256;
 __global__ void tie_sample_kernel(TieSampleArgs a)
 {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -1099,7 +1113,7 @@ __global__ void tie_sample_kernel(TieSampleArgs a)
   uint32_t low;
   const uint64_t w = r < a.n ? fused_word(a.f, r, low) : 0;
   for (int c = 0; c < a.ncand; ++c) {
-    bool tie = false;
+    unsigned int tie = 0;
     if (r < a.n) {
       const unsigned long long key = w >> (a.drop[c] - 8);
       unsigned long long* s        = a.slots + static_cast<int64_t>(c) * 2 * kSampleTies;
@@ -1109,14 +1123,22 @@ __global__ void tie_sample_kernel(TieSampleArgs a)
         if (v == ~0ull) v = atomicCAS(s + at, ~0ull, key);
         if (v == ~0ull) break;
         if (v == key) {
-          tie = true;
+          tie = 1;
+          if (a.same) {
+            unsigned int* q = a.same + static_cast<int64_t>(c) * 2 * kSampleTies + at;
+            tie             = *static_cast<volatile unsigned int*>(q) >= kSameMax ? kSameMax : atomicAdd(q, 1u) + 1;
+          }
           break;
         }
         at = at + 1 == 2 * kSampleTies ? 0 : at + 1;
       }
     }
-    const uint32_t m = __ballot_sync(0xffffffffu, tie);
-    if (m && (threadIdx.x & 31) == 0) atomicAdd(a.ties + c, static_cast<unsigned>(__popc(m)));
+    const unsigned int sum = __reduce_add_sync(0xffffffffu, tie);
+    const unsigned int top = __reduce_max_sync(0xffffffffu, tie);
+    if (sum && (threadIdx.x & 31) == 0) {
+      atomicAdd(a.ties + c, sum);
+      if (a.same) atomicMax(a.most + c, top + 1);
+    }
   }
 }
 
@@ -1218,6 +1240,147 @@ __global__ void __launch_bounds__(256) move_records_kernel(RadixPayload pay, con
   }
 }
 
+// ---- rows that travel whole ---------------------------------------------------
+// One integer key as its whole word W = (raw ^ flip) - min, and at most 8
+// bytes of other columns V (radix_sort_pairs).
+
+// Writes W of every row and counts the digits that the passes sort on, from
+// bit `drop` up: one read and one write (100M int64 keys: 281 us, 5.7 TB/s;
+// fused_words' general codes took 508 us for the same bytes).
+constexpr int kPairRows = 4;
+template <typename T, typename KT>
+__global__ void __launch_bounds__(RT) pair_words_kernel(const T* raw, T flip, T min, int64_t n, int drop, int npasses,
+                                                        KT* words, uint32_t* hist)
+{
+  __shared__ uint32_t sh[8 * 256];
+  for (int i = threadIdx.x; i < npasses * 256; i += RT) sh[i] = 0;
+  __syncthreads();
+  const int64_t per_iter = static_cast<int64_t>(RT) * kPairRows;
+  for (int64_t base = blockIdx.x * per_iter + threadIdx.x; base < n; base += static_cast<int64_t>(gridDim.x) * per_iter) {
+    T x[kPairRows];
+#pragma unroll
+    for (int j = 0; j < kPairRows; ++j) x[j] = base + j * RT < n ? __ldcs(raw + base + j * RT) : T(0);
+#pragma unroll
+    for (int j = 0; j < kPairRows; ++j) {
+      if (base + j * RT >= n) break;
+      const KT w             = static_cast<KT>(static_cast<T>((x[j] ^ flip) - min));
+      words[base + j * RT] = w;
+      uint64_t d             = static_cast<uint64_t>(w) >> drop;
+      for (int q = 0; q < npasses; ++q, d >>= 8) atomicAdd(&sh[q * 256 + (static_cast<uint32_t>(d) & 0xffu)], 1u);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < npasses * 256; i += RT)
+    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+}
+
+struct PairCols {
+  uint64_t flip, min;  // the key: raw = (W + min) ^ flip
+  int width;
+  void* key;
+  int n;  // columns packed into V (0: V is one column)
+  int part_width[kPassPayload];
+  int off[kPassPayload];  // byte offset in V, a multiple of the width
+  const void* src[kPassPayload];
+  void* dst[kPassPayload];
+};
+
+template <typename KT, typename VT>
+__device__ __forceinline__ void store_pair(const PairCols& c, int64_t pos, KT w, VT v, VT* vout)
+{
+  st_fixed(c.key, c.width, pos, (static_cast<uint64_t>(w) + c.min) ^ c.flip);
+  if (vout) vout[pos] = v;
+  for (int q = 0; q < c.n; ++q) st_fixed(c.dst[q], c.part_width[q], pos, static_cast<uint64_t>(v) >> (8 * c.off[q]));
+}
+
+template <typename VT>
+__global__ void __launch_bounds__(256) pack_pairs_kernel(PairCols c, int64_t n, VT* v)
+{
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    uint64_t x = 0;
+    for (int q = 0; q < c.n; ++q) {
+      DCol d{};
+      d.data  = c.src[q];
+      d.width = c.part_width[q];
+      x |= dbits_stream(d, i) << (8 * c.off[q]);
+    }
+    v[i] = static_cast<VT>(x);
+  }
+}
+
+// Rows sorted on W >> drop to their final places and out of W.  A row's place
+// among the rows that agree with it in W >> drop is counted: with up to
+// kPairRun of them (6 on average when a 100M-row sort drops all but 24 bits)
+// each row compares itself with its neighbours in shared memory; longer runs
+// are listed for order_pair_runs (count[0]; count[1]: one over kTieRunMax).
+// Bound by those compares: 1.0 ms at 100M rows, for 2.4 GB of traffic; a
+// bitmap of the runs' first rows and one loop over a run took 1.17 ms.
+// vout: where V goes as it is (null: nowhere).  drop 0: nothing is left to order.
+constexpr int kPairRun  = 32;
+constexpr int kPairTile = 8;  // rows per thread
+template <typename KT, typename VT>
+__global__ void __launch_bounds__(256) finish_pairs_kernel(PairCols c, const KT* w, const VT* vin, VT* vout, int64_t n,
+                                                           int drop, TieRun* runs, unsigned int* count)
+{
+  constexpr int T = 256 * kPairTile;
+  __shared__ KT s[T + 2 * kPairRun];
+  const int64_t base = blockIdx.x * static_cast<int64_t>(T);
+  VT v[kPairTile];
+#pragma unroll
+  for (int j = 0; j < kPairTile; ++j) {
+    const int64_t i = base + j * 256 + threadIdx.x;
+    v[j]            = i < n && vin ? __ldcs(vin + i) : VT(0);
+  }
+  for (int j = threadIdx.x; j < T + 2 * kPairRun; j += 256) {
+    const int64_t i = base - kPairRun + j;
+    if (i >= 0 && i < n) s[j] = __ldg(w + i);
+  }
+  __syncthreads();
+  const KT below = drop ? (KT(1) << drop) - 1 : KT(0);
+#pragma unroll
+  for (int j = 0; j < kPairTile; ++j) {
+    const int64_t i = base + j * 256 + threadIdx.x;
+    if (i >= n) break;
+    const KT* at = s + kPairRun + j * 256 + threadIdx.x;
+    const KT x   = *at;
+    int64_t pos  = i;
+    if (drop) {
+      const int left  = i < kPairRun ? static_cast<int>(i) : kPairRun;
+      const int right = n - 1 - i < kPairRun ? static_cast<int>(n - 1 - i) : kPairRun;
+      int l = 0, r = 0, before = 0;
+      for (; l < left && at[-1 - l] >= (x & ~below); ++l) before += at[-1 - l] <= x ? 1 : 0;
+      for (; r < right && at[1 + r] <= (x | below); ++r) before += at[1 + r] < x ? 1 : 0;
+      if (l + r >= kPairRun) {
+        if (l > 0) continue;
+        int len = r + 1;  // the run's first row
+        while (i + len < n && len <= kTieRunMax && __ldg(w + i + len) <= (x | below)) ++len;
+        if (len > kTieRunMax) atomicExch(count + 1, 1u);
+        else runs[atomicAdd(count, 1u)] = TieRun{static_cast<int32_t>(i), len};
+        continue;
+      }
+      pos = i - l + before;
+    }
+    store_pair(c, pos, x, v[j], vout);
+  }
+}
+
+template <typename KT, typename VT>
+__global__ void __launch_bounds__(256) order_pair_runs_kernel(PairCols c, const KT* w, const VT* vin, VT* vout,
+                                                              const TieRun* runs)
+{
+  __shared__ KT key[kTieRunMax];
+  const TieRun t = runs[blockIdx.x];
+  for (int k = threadIdx.x; k < t.len; k += 256) key[k] = w[t.start + k];
+  __syncthreads();
+  for (int k = threadIdx.x; k < t.len; k += 256) {
+    const KT x = key[k];
+    int at     = 0;
+    for (int j = 0; j < t.len; ++j) at += key[j] < x || (key[j] == x && j < k) ? 1 : 0;
+    store_pair(c, t.start + at, x, vin[t.start + k], vout);
+  }
+}
+
 __global__ void __launch_bounds__(256) move_by_perm_kernel(RadixPayload pay, const int32_t* perm, int64_t n)
 {
   const int64_t per = static_cast<int64_t>(blockDim.x) * kMoveBatch;
@@ -1235,29 +1398,180 @@ __global__ void __launch_bounds__(256) move_by_perm_kernel(RadixPayload pay, con
 
 }  // namespace
 
-int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n)
+namespace {
+// sort_word_of of an integer key: its raw bits ^ int_flip.
+uint64_t int_flip(const SortKeyDesc& k)
+{
+  const uint64_t all = k.key_bytes >= 8 ? ~0ull : (1ull << (8 * k.key_bytes)) - 1;
+  return (is_signed_int(k.col.type) ? all ^ (all >> 1) : 0) ^ (k.descending ? all : 0);
+}
+
+template <typename T, typename KT>
+void pair_words(const OpContext& ctx, const FusedKey& f, const PairCols& c, int64_t n, int npasses, void* words,
+                uint32_t* hist)
+{
+  launch("pair_words", pair_words_kernel<T, KT>,
+         static_cast<unsigned>(std::min<int64_t>(ceil_div(n, int64_t(RT) * kPairRows), 8 * num_sms())), RT, 0, ctx.stream(),
+         static_cast<const T*>(f.key[0].col.data), static_cast<T>(c.flip), static_cast<T>(c.min), n, f.drop, npasses,
+         static_cast<KT*>(words), hist);
+}
+
+// vals: V of every row; vout: its column in sorted order (null: packed).
+template <typename KT, typename VT>
+bool sort_pairs(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, const PairCols& cols, const VT* vals, VT* vout)
+{
+  cudaStream_t s = ctx.stream();
+  const int P    = std::max(1, (bits - f.drop + 7) / 8);
+  std::vector<uint32_t> hist(static_cast<size_t>(P) * 256, 0);
+  Buffer<uint8_t> words(ctx.alloc(), static_cast<size_t>(n) * sizeof(KT));
+  {
+    Buffer<uint32_t> d_hist(ctx.alloc(), hist.size());
+    LDF_CUDA(cudaMemsetAsync(d_hist.get(), 0, hist.size() * sizeof(uint32_t), s));
+    switch (cols.width) {
+      case 1: pair_words<uint8_t, KT>(ctx, f, cols, n, P, words.get(), d_hist.get()); break;
+      case 2: pair_words<uint16_t, KT>(ctx, f, cols, n, P, words.get(), d_hist.get()); break;
+      case 4: pair_words<uint32_t, KT>(ctx, f, cols, n, P, words.get(), d_hist.get()); break;
+      default: pair_words<uint64_t, KT>(ctx, f, cols, n, P, words.get(), d_hist.get()); break;
+    }
+    ctx.fetch(hist.data(), d_hist.get(), hist.size() * sizeof(uint32_t));
+    ctx.finish();
+  }
+  std::vector<RadixPass> passes(P);
+  for (int q = 0; q < P; ++q) {
+    passes[q].src   = DigitSrc::CARRIED;
+    passes[q].shift = f.drop + 8 * q;
+  }
+  std::vector<int> run = varying_passes(hist, P, n);
+  if (run.empty()) run.push_back(P - 1);  // some pass has to write the rows
+  const bool direct = f.drop == 0 && vout != nullptr;  // the last pass's order is final
+  Buffer<VT> sorted;
+  if (!direct) sorted = Buffer<VT>(ctx.alloc(), static_cast<size_t>(n));
+  run_passes(ctx, passes, run, hist, n, direct ? vout : sorted.get(), nullptr, nullptr, &f, &words, sizeof(KT), &words,
+             vals, sizeof(VT));
+  const KT* w  = reinterpret_cast<const KT*>(words.get());
+  const VT* v  = sorted.get();
+  VT* vo       = direct ? nullptr : vout;
+  Buffer<TieRun> runs(ctx.alloc(), f.drop ? static_cast<size_t>(n / kPairRun + 1) : 1);
+  Buffer<unsigned int> count(ctx.alloc(), 2);
+  LDF_CUDA(cudaMemsetAsync(count.get(), 0, 2 * sizeof(unsigned int), s));
+  launch("finish_pairs", finish_pairs_kernel<KT, VT>, static_cast<unsigned>(ceil_div(n, 256 * kPairTile)), 256, 0, s, cols,
+         w, v, vo, n, f.drop, runs.get(), count.get());
+  if (f.drop == 0) return true;
+  unsigned int h[2];
+  ctx.fetch(h, count.get(), sizeof(h));
+  ctx.finish();
+  if (h[1]) return false;
+  if (h[0])
+    launch("order_pair_runs", order_pair_runs_kernel<KT, VT>, h[0], 256, 0, s, cols, w, v, vo,
+           static_cast<const TieRun*>(runs.get()));
+  return true;
+}
+
+template <typename VT>
+void sort_pairs_of(const OpContext& ctx, FusedKey f, int bits, int64_t n, PairCols c)
+{
+  const VT* vals = static_cast<const VT*>(c.src[0]);
+  VT* vout       = static_cast<VT*>(c.dst[0]);
+  Buffer<VT> packed;
+  if (c.n > 1 || c.part_width[0] != static_cast<int>(sizeof(VT))) {
+    packed = Buffer<VT>(ctx.alloc(), static_cast<size_t>(n));
+    launch("pack_pairs", pack_pairs_kernel<VT>,
+           static_cast<unsigned>(std::min<int64_t>(ceil_div(n, 256), 16 * num_sms())), 256, 0, ctx.stream(), c, n, packed.get());
+    vals = packed.get();
+    vout = nullptr;
+  } else {
+    c.n = 0;
+  }
+  auto sort = [&] {
+    if constexpr (sizeof(VT) == 4)
+      if (bits <= 32) return sort_pairs<uint32_t, VT>(ctx, f, bits, n, c, vals, vout);
+    return sort_pairs<uint64_t, VT>(ctx, f, bits, n, c, vals, vout);
+  };
+  if (sort()) return;
+  f.drop = 0;  // too many rows tie: the whole word
+  sort();
+}
+}  // namespace
+
+bool radix_pairs_fit(const FusedKey& f, int64_t n, const ldf_column* table, int ncols, int key)
+{
+  if (n < kDropMinRows || f.n != 1 || f.has_class[0] || table[key].type == LDF_STRING) return false;
+  int bytes = 0;
+  for (int j = 0; j < ncols; ++j) {
+    if (j == key) continue;
+    if (table[j].type == LDF_STRING || table[j].valid != nullptr) return false;
+    bytes += type_width(table[j].type);
+  }
+  return bytes > 0 && bytes <= 8 && ncols - 1 <= kPassPayload;
+}
+
+void radix_sort_pairs(const OpContext& ctx, FusedKey f, int bits, int64_t n, const ldf_column* table, int ncols, int key,
+                      ldf_column* out)
+{
+  PairCols c{};
+  int order[kPassPayload], bytes = 0;
+  for (int j = 0; j < ncols; ++j) {
+    if (j == key) continue;
+    order[c.n++] = j;
+    bytes += type_width(table[j].type);
+  }
+  std::stable_sort(order, order + c.n, [&](int x, int y) { return type_width(table[x].type) > type_width(table[y].type); });
+  for (int q = 0, off = 0; q < c.n; ++q) {
+    c.part_width[q] = type_width(table[order[q]].type);
+    c.off[q]        = off;
+    c.src[q]        = table[order[q]].data;
+    c.dst[q]        = out[order[q]].data;
+    off += c.part_width[q];
+  }
+  c.flip  = int_flip(f.key[0]);
+  c.min   = f.min[0];
+  c.width = f.key[0].col.width;
+  c.key   = out[key].data;
+  f.drop  = choose_drop(ctx, f, bits, n, true);
+  if (bytes <= 4) sort_pairs_of<int32_t>(ctx, f, bits, n, c);
+  else sort_pairs_of<int64_t>(ctx, f, bits, n, c);
+}
+
+int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, bool whole_rows)
 {
   TieSampleArgs a{};
   a.f      = f;
   a.n      = n;
   a.stride = ceil_div(n, kSampleTies);
-  // two passes fewer than the whole word takes, at least, and a prefix that
+  // two passes fewer than the whole word takes, at least (whole rows: one, as
+  // they are written once more after the passes anyhow), and a prefix that
   // could tell n rows apart
   const int full = (bits + 7) / 8;
-  for (int k = 2; k <= full - 2 && k <= 8; ++k)
+  for (int k = 2; k <= full - (whole_rows ? 1 : 2) && k <= 8; ++k)
     if (bits - 8 * k >= 8 && (int64_t(1) << std::min(8 * k, 62)) >= n / 16) a.drop[a.ncand++] = bits - 8 * k;
   if (n < kDropMinRows || a.ncand == 0) return 0;
   cudaStream_t s = ctx.stream();
   Buffer<unsigned long long> slots(ctx.alloc(), static_cast<size_t>(a.ncand) * 2 * kSampleTies);
-  Buffer<unsigned int> ties(ctx.alloc(), kDropCands);
+  Buffer<unsigned int> ties(ctx.alloc(), 2 * kDropCands), same;
   LDF_CUDA(cudaMemsetAsync(slots.get(), 0xff, slots.bytes(), s));
-  LDF_CUDA(cudaMemsetAsync(ties.get(), 0, kDropCands * sizeof(unsigned int), s));
+  LDF_CUDA(cudaMemsetAsync(ties.get(), 0, 2 * kDropCands * sizeof(unsigned int), s));
+  if (whole_rows) {
+    same = Buffer<unsigned int>(ctx.alloc(), static_cast<size_t>(a.ncand) * 2 * kSampleTies);
+    LDF_CUDA(cudaMemsetAsync(same.get(), 0, same.bytes(), s));
+  }
   a.slots = slots.get();
+  a.same  = same.get();
   a.ties  = ties.get();
+  a.most  = ties.get() + kDropCands;
   launch("tie_sample", tie_sample_kernel, static_cast<unsigned>(kSampleTies / 256), 256, 0, s, a);
-  unsigned int h[kDropCands];
+  unsigned int h[2 * kDropCands];
   ctx.fetch(h, ties.get(), sizeof(h));
   ctx.finish();
+  if (whole_rows) {
+    // p sampled pairs of rows that tie stand for p (n / sample)^2: up to 4 a
+    // row (8 neighbours each) are ordered for less than another pass takes.  A
+    // group of kTieRunMax rows shows 2^12 / stride of its rows.
+    const double fits   = 4.0 * static_cast<double>(n) / static_cast<double>(a.stride) / static_cast<double>(a.stride);
+    const unsigned rows = static_cast<unsigned>(std::min<int64_t>(std::max<int64_t>(4, kTieRunMax / 2 / a.stride), kSameMax));
+    for (int c = 0; c < a.ncand; ++c)
+      if (h[c] <= fits && h[kDropCands + c] <= rows) return a.drop[c];
+    return 0;
+  }
   // t tying rows in the sample stand for about t (n / sample)^2 tying pairs
   // of rows; ties of a 64th of the rows or so cost less than a pass does.  A
   // single group of rows behind up to 8 sampled ties has some 4 (n / sample)

@@ -134,8 +134,9 @@ constexpr int64_t kDropMinRows = int64_t(1) << 21;
 
 // Dropped bits (0: none) with which sorting on the rest of the fused word of
 // `bits` bits, and then ordering the few rows that tie on it, takes fewest
-// passes: from the ties among a sample of the rows.
-int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n);
+// passes: from the ties among a sample of the rows.  whole_rows: for
+// radix_sort_pairs, which orders many ties cheaply.
+int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, bool whole_rows = false);
 
 // Orders the rows of every run of equal `words` (the sorted W >> f.drop, 4 or
 // 8 bytes each) in `perm` by the dropped bits, equal rows in the order they
@@ -192,6 +193,19 @@ void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes,
 // (4 when they have at most 32 bits, else 8).
 void radix_sort_words(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, int32_t* perm,
                       const RadixPayload* payload, Buffer<uint8_t>* words = nullptr, int* word_bytes = nullptr);
+
+// Sort of a whole table (outputs allocated) whose rows fit in the passes
+// themselves (radix_pairs_fit): one integer key, at most 8 bytes of up to
+// kPassPayload other fixed-width columns, no nulls.  The passes carry the whole word and those
+// columns instead of row ids, so nothing is gathered afterwards, and the key
+// column is the word turned back.  100M rows of an int64 key and an int32
+// column: 4.0 ms (three passes of 0.79, the last step 1.0), against 7.2 ms with row
+// ids and one random 16-byte read a row.
+// From kDropMinRows rows, as for the bits dropped: the passes of smaller
+// tables stay in L2 with row ids too.
+bool radix_pairs_fit(const FusedKey& f, int64_t n, const ldf_column* table, int ncols, int key);
+void radix_sort_pairs(const OpContext& ctx, FusedKey f, int bits, int64_t n, const ldf_column* table, int ncols, int key,
+                      ldf_column* out);
 
 // The payload's columns gathered through `perm` (payload.dst[position] =
 // src[perm[position]]).

@@ -697,7 +697,6 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
     }
     if (fits && bits <= kFusedMaxBits) {
       fused       = true;
-      fk.drop    = choose_drop(ctx, fk, bits, n);
       fused_bits = bits;
       for (int q = 0; bits > 64 && 8 * q < bits; ++q) {  // a wider word: pass by pass (FusedKey)
         RadixPass p{};
@@ -720,6 +719,13 @@ void sort_table(const ldf_column* table, int ncols, const int32_t* keys, const u
       }
     }
   }
+  if (whole && fused && nkeys == 1 && radix_pairs_fit(fk, n, table, ncols, keys[0])) {
+    for (int j = 0; j < ncols; ++j) out[j] = alloc_out_column(al, table[j].type, n, table[j].valid != nullptr);
+    radix_sort_pairs(ctx, fk, fused_bits, n, table, ncols, keys[0], out);
+    ctx.finish();
+    return;
+  }
+  if (fused) fk.drop = choose_drop(ctx, fk, fused_bits, n);
   Buffer<int32_t> perm(al, std::max<int64_t>(n, 1));
   // the leading bits, then the ties among them; true when `perm` is done
   auto sort_leading = [&]() {
