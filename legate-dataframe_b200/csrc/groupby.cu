@@ -560,8 +560,11 @@ __global__ void __launch_bounds__(kGbThreads) assign_kernel(GbPlan p, uint32_t* 
 // the pass counts in shared memory (left to the race of its first wave, a key
 // holding an eighth of the rows could get any id, and 24M reductions on one
 // word took assign from 2.8 to 5-8 ms on 200M rows), and their slots are
-// complete before the wave starts.
+// complete before the wave starts.  A string or multi-column key is compared at
+// the row that inserted it: those are sampled in runs of kSeedRun rows, so that
+// frequent keys' strings share cache lines (100M string rows: 4.63 -> 4.52 ms).
 constexpr int64_t kSeedRows = 16384;
+constexpr int64_t kSeedRun  = 512;
 template <KeyMode M>
 __global__ void __launch_bounds__(kGbThreads) seed_keys_kernel(GbPlan p, int64_t rows, int64_t stride)
 {
@@ -574,8 +577,9 @@ __global__ void __launch_bounds__(kGbThreads) seed_keys_kernel(GbPlan p, int64_t
     uint32_t id[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const int64_t i = base + j * 32 + lane_id();
-      r[j]            = i < rows ? i * stride : p.n;
+      const int64_t i  = base + j * 32 + lane_id();
+      const int64_t at = M == KeyMode::GEN ? i / kSeedRun * kSeedRun * stride + i % kSeedRun : i * stride;
+      r[j]             = i < rows ? at : p.n;
     }
     group_ids<M, R>(p, pool, r, id);
   }
