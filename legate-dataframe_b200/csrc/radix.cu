@@ -1027,18 +1027,19 @@ void identity_order(const OpContext& ctx, int64_t n, int32_t* perm, int32_t* inv
 }  // namespace
 
 void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
-                     int32_t* perm, std::vector<uint32_t>* hist_out, int32_t* inv, const RadixPayload* payload,
+                     int32_t* perm, const std::vector<uint32_t>* counted, int32_t* inv, const RadixPayload* payload,
                      const FusedKey* fused)
 {
   const size_t P = passes.size();
   std::vector<uint32_t> hist(P * 256, 0);
-  if (P > 0 && n > 0) {
+  if (counted) {
+    hist = *counted;
+  } else if (P > 0 && n > 0) {
     Buffer<uint32_t> d_hist(ctx.alloc(), P * 256);
     radix_histograms(ctx, passes, n, d_hist.get(), fused);
     ctx.fetch(hist.data(), d_hist.get(), P * 256 * sizeof(uint32_t));
     ctx.finish();
   }
-  if (hist_out) *hist_out = hist;
   // skip constant-digit passes; the first executed pass of a word gathers it,
   // later passes of the same word read it carried
   const std::vector<int> run = varying_passes(hist, P, n);

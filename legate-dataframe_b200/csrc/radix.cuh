@@ -184,8 +184,10 @@ inline bool payload_empty(const RadixPayload& p) { return p.n == 0 && p.nparts =
 // `inv` (optional, n entries): inv[row] = the row's position in the sorted
 // order, written by the last pass.  `payload` (optional): columns the last
 // pass writes in sorted order.  `fused`: the FusedKey of FUSED passes.
+// `counted` (optional): the digit counts of all passes ([pass][256]), when the
+// caller has them; otherwise one read of the keys counts them.
 void radix_sort_rows(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
-                     int32_t* perm, std::vector<uint32_t>* hist_out = nullptr, int32_t* inv = nullptr,
+                     int32_t* perm, const std::vector<uint32_t>* counted = nullptr, int32_t* inv = nullptr,
                      const RadixPayload* payload = nullptr, const FusedKey* fused = nullptr);
 
 // The same on the fused word W >> f.drop of at most 64 bits (W has `bits`).
