@@ -598,7 +598,7 @@ struct Matches {
   const int32_t* list;
   uint32_t* pstart;  // per probe row, kProbeTile entries per tile
   uint32_t* pcount;
-  uint32_t* tile_counts;
+  int64_t* tile_counts;
   const int64_t* tile_offsets;
 };
 
@@ -633,7 +633,24 @@ __global__ void __launch_bounds__(kProbeThreads) match_count_kernel(ProbeArgs a,
   }
   int64_t total;
   block_exclusive_scan<int64_t, kProbeThreads>(cnt, s_scan, &total);
-  if (threadIdx.x == 0) m.tile_counts[tile] = static_cast<uint32_t>(total);
+  if (threadIdx.x == 0) m.tile_counts[tile] = total;
+}
+
+// Output rows are counted within a tile in 32 bits unless the probe's output
+// rows in all do not fit them: 1,024 probe rows on one key of 2^22 build rows
+// are 2^32 rows of one tile.
+inline bool wide_tile_rows(int64_t probe_rows) { return probe_rows > int64_t(0xffffffff); }
+
+// The last of a tile's rows whose output rows start at or before output row j
+// of the tile; excl: the output rows before each of them.
+template <typename T>
+__host__ __device__ __forceinline__ int tile_row(const T* excl, T j)
+{
+  int lo = 0;
+#pragma unroll
+  for (int step = kProbeTile / 2; step > 0; step >>= 1)
+    if (excl[lo + step] <= j) lo += step;
+  return lo;
 }
 
 // Pass 2: a tile's output rows, shared out evenly over its threads whatever
@@ -642,10 +659,13 @@ __global__ void __launch_bounds__(kProbeThreads) match_count_kernel(ProbeArgs a,
 // tiles are shared by several blocks (gridDim.y).  Whole joins with ten build
 // rows per int64 key, walking clusters of equal keys a row per thread -> this:
 // 20,000 x 20,000 rows 884 -> 212 us, 4M x 4M rows 11.6 -> 1.5 ms.
+// T: a tile's output rows (wide_tile_rows).
+template <typename T>
 __global__ void __launch_bounds__(kProbeThreads) match_write_kernel(ProbeArgs a, Matches m)
 {
   __shared__ int64_t s_scan[kProbeThreads / 32 + 1];
-  __shared__ uint32_t s_excl[kProbeTile], s_start[kProbeTile];
+  __shared__ T s_excl[kProbeTile];
+  __shared__ uint32_t s_start[kProbeTile];
   const int64_t tile = static_cast<int64_t>(blockIdx.x);
   const int64_t base = tile * kProbeTile;
   const int t0       = threadIdx.x * kProbeItems;
@@ -663,7 +683,7 @@ __global__ void __launch_bounds__(kProbeThreads) match_write_kernel(ProbeArgs a,
   int64_t excl = block_exclusive_scan<int64_t, kProbeThreads>(cnt, s_scan, &total);
 #pragma unroll
   for (int i = 0; i < kProbeItems; ++i) {
-    s_excl[t0 + i]  = static_cast<uint32_t>(excl);
+    s_excl[t0 + i]  = static_cast<T>(excl);
     s_start[t0 + i] = c[i] > 0 ? ps[i] : 0xffffffffu;  // build rows number fewer than 2^31
     excl += rows[i];
   }
@@ -677,13 +697,10 @@ __global__ void __launch_bounds__(kProbeThreads) match_write_kernel(ProbeArgs a,
       const int64_t j = j0 + i * kProbeThreads;
       pos[i] = lrow[i] = brow[i] = -1;
       if (j >= total) continue;
-      int lo = 0;  // the last row whose outputs start at or before j
-#pragma unroll
-      for (int step = kProbeTile / 2; step > 0; step >>= 1)
-        if (s_excl[lo + step] <= static_cast<uint32_t>(j)) lo += step;
+      const int lo = tile_row(s_excl, static_cast<T>(j));
       pos[i]  = out0 + j;
       lrow[i] = base + lo;
-      if (s_start[lo] != 0xffffffffu) brow[i] = __ldg(m.list + s_start[lo] + (static_cast<uint32_t>(j) - s_excl[lo]));
+      if (s_start[lo] != 0xffffffffu) brow[i] = __ldg(m.list + s_start[lo] + (static_cast<T>(j) - s_excl[lo]));
     }
     emit_batch(a.lo, pos, lrow);
     emit_build_batch(a, pos, lrow, brow);
@@ -1130,14 +1147,14 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
     mt.start = sstart.get();
     mt.list  = list.get();
     if (tiles > 0) {
-      Buffer<uint32_t> counts(al, tiles);
+      Buffer<int64_t> counts(al, tiles);
       tile_offsets   = Buffer<int64_t>(al, tiles);
       pmatch         = Buffer<uint32_t>(al, 2 * tiles * kProbeTile);
       mt.pstart      = pmatch.get();
       mt.pcount      = pmatch.get() + tiles * kProbeTile;
       mt.tile_counts = counts.get();
       launch("match_count", match_count_kernel<M>, static_cast<unsigned>(tiles), kProbeThreads, 0, s, a, mt);
-      exclusive_scan_u32(counts.get(), tile_offsets.get(), tiles, d_total.get(), ctx);
+      exclusive_scan_i64(counts.get(), tile_offsets.get(), tiles, d_total.get(), ctx);
       probe_rows      = ctx.read_i64(d_total.get());
       mt.tile_offsets = tile_offsets.get();
     }
@@ -1212,7 +1229,8 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
       // about four blocks per SM, as far as a tile's output rows go round
       const int64_t share = std::min<int64_t>(4 * num_sms() / tiles, probe_rows / tiles / (kProbeThreads * kProbeItems));
       const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(share, 64))));
-      launch("match_write", match_write_kernel, grid, kProbeThreads, 0, s, a, mt);
+      launch("match_write", wide_tile_rows(probe_rows) ? match_write_kernel<uint64_t> : match_write_kernel<uint32_t>, grid,
+             kProbeThreads, 0, s, a, mt);
     }
   }
   int64_t rows = 0;
