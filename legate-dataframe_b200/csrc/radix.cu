@@ -213,6 +213,9 @@ __device__ __forceinline__ void prefetch_column(const DCol& c, int64_t lo, int64
 // moves columns.
 constexpr int kMoveBatch = 3;
 
+// First 8-byte word of a row's string range; rows from 2^30 on pass 32 bits.
+__host__ __device__ __forceinline__ int64_t range_word(int32_t row) { return 2 * static_cast<int64_t>(row); }
+
 // dst[pos[k]] = src[row[k]] for 16-byte string ranges (8-byte aligned at the
 // source: two 8-byte loads; the scratch destination is 16-byte aligned), every
 // load issued before the first store.  pos < 0: no row.
@@ -223,7 +226,10 @@ __device__ __forceinline__ void move_ranges(const void* src, void* dst, const in
   ulonglong2 v[kMoveBatch];
 #pragma unroll
   for (int k = 0; k < kMoveBatch; ++k)
-    if (pos[k] >= 0) v[k] = make_ulonglong2(__ldg(sp + 2 * row[k]), __ldg(sp + 2 * row[k] + 1));
+    if (pos[k] >= 0) {
+      const unsigned long long* r = sp + range_word(row[k]);
+      v[k]                        = make_ulonglong2(__ldg(r), __ldg(r + 1));
+    }
 #pragma unroll
   for (int k = 0; k < kMoveBatch; ++k)
     if (pos[k] >= 0) static_cast<ulonglong2*>(dst)[pos[k]] = v[k];
