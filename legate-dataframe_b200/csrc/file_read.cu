@@ -1,8 +1,11 @@
 // A file's bytes into pinned host memory and on to the device: several threads
 // read pieces of the file and queue each piece's copy as soon as it is there,
 // so that reading (a page-cache copy, some 10 GB/s a thread) and the copies
-// to the device (55 GB/s) overlap.  kPiece is small enough that a file of a
-// few tens of MB occupies all threads: a 44 MB file took 4.4 ms as one piece.
+// to the device (55 GB/s) overlap.  The copies go to the staging stream, behind
+// the caller's work so far: the caller's own stream may be the per-thread one,
+// whose handle names another stream in every thread.  kPiece is small enough
+// that a file of a few tens of MB occupies all threads: a 44 MB file took
+// 4.4 ms as one piece.  33 MB now take 1.5 ms, 400 MB 11.5 ms (36 GB/s).
 #include <fcntl.h>
 #include <sys/types.h>
 #include <unistd.h>
@@ -34,6 +37,18 @@ int read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, cud
     LDF_CUDA(cudaGetLastError());
     fail(LDF_ERR_CUDA, "read_file: no current device");
   }
+  cudaStream_t copies = nullptr;
+  cudaEvent_t done    = nullptr;
+  try {
+    copies = staging_stream();
+    LDF_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    LDF_CUDA(cudaEventRecord(done, s));  // `dev` may be memory that earlier work on s still touches
+    LDF_CUDA(cudaStreamWaitEvent(copies, done, 0));
+  } catch (...) {
+    close(fd);
+    if (done != nullptr) cudaEventDestroy(done);
+    throw;
+  }
   const int64_t pieces = ceil_div(nbytes, kPiece);
   std::atomic<int64_t> next{0};
   std::atomic<int> err{0};
@@ -51,7 +66,7 @@ int read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, cud
         }
         at += got;
       }
-      e = cudaMemcpyAsync(dev + a, host + a, static_cast<size_t>(b - a), cudaMemcpyHostToDevice, s);
+      e = cudaMemcpyAsync(dev + a, host + a, static_cast<size_t>(b - a), cudaMemcpyHostToDevice, copies);
     }
     if (e != cudaSuccess) cuda_err.store(e);
   };
@@ -66,10 +81,12 @@ int read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, cud
   for (auto& t : threads) t.join();
   close(fd);
   // the copies read `host`, which the caller may give back on return
-  const cudaError_t done = cudaStreamSynchronize(s);
+  cudaError_t waited = cudaEventRecord(done, copies);
+  if (waited == cudaSuccess) waited = cudaEventSynchronize(done);
+  cudaEventDestroy(done);
   if (err.load() != 0) return err.load();
   LDF_CUDA(static_cast<cudaError_t>(cuda_err.load()));
-  LDF_CUDA(done);
+  LDF_CUDA(waited);
   return 0;
 }
 
