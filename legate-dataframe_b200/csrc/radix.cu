@@ -194,10 +194,11 @@ struct PassArgs {
   int* err;
   // > 0: each tile stages in L2, by bulk prefetches, the rows of the tile
   // this many tiles ahead (about one wave of resident CTAs; tiles are taken
-  // in order): the row ids and carried words of a pass on the carried word,
-  // and the key columns of a first pass over rows in input order
+  // in order): the values (pf_vals) and carried words of a pass on the carried
+  // word, and the key columns of a first pass over rows in input order
   // (pf_columns).
   int64_t pf_ahead;
+  int pf_vals;
   int pf_columns;
 };
 
@@ -649,6 +650,14 @@ bool on_device(const void* p)
 }
 bool column_on_device(const DCol& c) { return on_device(c.data) && on_device(c.valid); }
 
+// Whether pass k prefetches the rows' values: later passes read scratch, the
+// first one `vals`, which may be a column of the caller (null: row ids).
+template <typename F>
+int prefetch_values(size_t pass, const void* vals, F device)
+{
+  return pass > 0 || (vals != nullptr && prefetch_first_pass() != 0 && device(vals)) ? 1 : 0;
+}
+
 // The key columns the first pass of `p` reads in row order are all in
 // device memory.
 bool pass_columns_on_device(const RadixPass& p, const FusedKey* fused)
@@ -695,7 +704,7 @@ __global__ void __launch_bounds__(RT, radix_min_blocks<GATHER>()) onesweep_kerne
     const int64_t hi = min(lo + static_cast<int64_t>(RTILE), a.n);
     if (!GATHER) {
       constexpr int64_t vb = sizeof(VT);
-      if (a.vals_in) l2_prefetch_bulk(a.vals_in, lo * vb, hi * vb);
+      if (a.pf_vals && a.vals_in) l2_prefetch_bulk(a.vals_in, lo * vb, hi * vb);
       if (a.p.src != DigitSrc::CLASS)
         l2_prefetch_bulk(a.keys_in, lo * static_cast<int64_t>(sizeof(KT)), hi * static_cast<int64_t>(sizeof(KT)));
     } else if (a.pf_columns && a.vals_in == nullptr) {  // rows in input order: the key columns are read in order
@@ -983,6 +992,7 @@ void run_passes(const OpContext& ctx, const std::vector<RadixPass>& passes, cons
     if (last && payload) a.pay = *payload;
     if (fused) a.fused = *fused;
     a.err        = ctx.err();
+    a.pf_vals    = prefetch_values(k, first_vals, on_device);
     a.pf_columns = gather && k == 0 && prefetch_first_pass() && pass_columns_on_device(p, fused) ? 1 : 0;
     const bool move = !payload_empty(a.pay);
     if (vb == 8) {
