@@ -71,24 +71,32 @@ inline void launch(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 b
   prof::end(name, s);
 }
 
-// The same for a kernel that runs as one thread-block cluster of `cluster`
-// CTAs (its grid).
-template <typename... KArgs, typename... Args>
-inline void launch_cluster(const char* name, void (*kernel)(KArgs...), unsigned cluster, unsigned threads, size_t smem,
-                           cudaStream_t s, Args&&... args)
+// A launch as one thread-block cluster of `cluster` CTAs (the grid); attr lives
+// as long as the configuration.
+inline cudaLaunchConfig_t cluster_config(unsigned cluster, unsigned threads, size_t smem, cudaStream_t s,
+                                         cudaLaunchAttribute& attr)
 {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim          = dim3(cluster);
-  cfg.blockDim         = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream           = s;
-  cudaLaunchAttribute attr{};
+  cfg.gridDim           = dim3(cluster);
+  cfg.blockDim          = dim3(threads);
+  cfg.dynamicSmemBytes  = smem;
+  cfg.stream            = s;
   attr.id               = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = cluster;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   cfg.attrs             = &attr;
   cfg.numAttrs          = 1;
+  return cfg;
+}
+
+// launch() of a kernel that runs as one cluster.
+template <typename... KArgs, typename... Args>
+inline void launch_cluster(const char* name, void (*kernel)(KArgs...), unsigned cluster, unsigned threads, size_t smem,
+                           cudaStream_t s, Args&&... args)
+{
+  cudaLaunchAttribute attr{};
+  cudaLaunchConfig_t cfg = cluster_config(cluster, threads, smem, s, attr);
   prof::begin(name, s);
   LDF_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...));
   prof::end(name, s);

@@ -44,6 +44,7 @@
 // each pass waits only for the columns it reads.
 #include "radix.cuh"
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1922,7 +1923,47 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_groupby_kernel(const _
 // against 409; of 131 groups 118 against 253).
 constexpr int64_t kSmallGroupbyRows = int64_t(1) << 17;
 
-// False (nothing done): a pair set overflowed its probe limit.
+// The largest cluster of at most `want` CTAs (a power of two) that fits (0:
+// none); active(c): clusters of c CTAs that the device holds at once.
+template <typename F>
+unsigned fit_cluster(unsigned want, F active)
+{
+  while (want > 0 && active(want) < 1) want /= 2;
+  return want;
+}
+
+// The largest cluster of small_groupby_kernel on this device with the most
+// shared memory it takes: 16 CTAs on a whole B200, fewer where a process has
+// only some of its SMs.  Asked for once per device, with the kernel's attributes
+// set first.
+constexpr int kSmallSmem = 208 * 1024;
+template <KeyMode M>
+unsigned small_cluster()
+{
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> known[kMaxDevices];  // the size + 1
+  int dev = 0;
+  LDF_CUDA(cudaGetDevice(&dev));
+  LDF_REQUIRE(dev >= 0 && dev < kMaxDevices, "device ordinal out of range");
+  if (const int k = known[dev].load()) return static_cast<unsigned>(k - 1);
+  LDF_CUDA(cudaFuncSetAttribute(small_groupby_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem));
+  LDF_CUDA(cudaFuncSetAttribute(small_groupby_kernel<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  const unsigned fit = fit_cluster(16, [](unsigned ctas) {
+    cudaLaunchAttribute attr{};
+    cudaLaunchConfig_t cfg = cluster_config(ctas, kSmallThreads, kSmallSmem, nullptr, attr);
+    int n                  = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, small_groupby_kernel<M>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return n;
+  });
+  known[dev].store(static_cast<int>(fit) + 1);
+  return fit;
+}
+
+// False (nothing done): no cluster fits, or a pair set overflowed its probe
+// limit.
 template <KeyMode M>
 bool small_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, const int32_t* keys, int nkeys,
                    const ldf_aggregation* aggs, int naggs, const std::vector<int>& agg_col, ldf_column* out)
@@ -1930,6 +1971,8 @@ bool small_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, cons
   const Allocator& al = ctx.alloc();
   cudaStream_t s      = ctx.stream();
   const int64_t n     = p.n;
+  const unsigned most = small_cluster<M>();
+  if (most == 0) return false;
   layout_records(p);
   p.cap    = static_cast<uint64_t>(2 * n + 64);
   p.id_cap = static_cast<uint64_t>(n);
@@ -1998,9 +2041,7 @@ bool small_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, cons
   bind_outputs(al, table, keys, nkeys, aggs, naggs, agg_col, M == KeyMode::GEN, n, out, a.f, repr);
   // up to 16 CTAs (the largest cluster), about four rows a thread
   unsigned ctas = 1;
-  while (ctas < 16 && static_cast<int64_t>(ctas) * kSmallThreads * 2 < n) ctas *= 2;
-  LDF_CUDA(cudaFuncSetAttribute(small_groupby_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024));
-  LDF_CUDA(cudaFuncSetAttribute(small_groupby_kernel<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  while (ctas < most && static_cast<int64_t>(ctas) * kSmallThreads * 2 < n) ctas *= 2;
   launch_cluster("small_groupby", small_groupby_kernel<M>, ctas, kSmallThreads, smem, s, a);
   unsigned int h[2] = {0, 0};  // groups, overflow
   ctx.fetch(h, misc, sizeof(h));
