@@ -1646,19 +1646,19 @@ void layout_records(GbPlan& p)
 }
 
 // ===========================================================================
-// Small inputs: the whole aggregation in ONE kernel, a thread-block cluster
-// whose CTAs meet at hardware cluster barriers between the phases.  The
-// general plan needs some twenty stream operations and three read-backs,
-// which is all the time a call on a few thousand rows takes; here the host
-// reads back one row count.  SUM and COUNT of 1,000 rows: 222 -> 90 us a
+// Small inputs: the whole aggregation in one kernel, a thread-block cluster
+// whose CTAs meet at hardware cluster barriers between the phases, and one that
+// writes the output.  The general plan needs some twenty stream operations and
+// three read-backs, which is all the time a call on a few thousand rows takes;
+// here the host reads back one row count.  SUM and COUNT of 1,000 rows: 222 -> 90 us a
 // call, of 50,000 rows with 5,000 groups 260 -> 100 us.
 //   1. empty key slots (and NUNIQUE pair sets)
 //   2. every row finds or inserts its key's slot; the row that inserts one
 //      takes the next dense group id and zeroes that group's records
 //   3. rows accumulate into the records of their slot's id; the lowest ids
 //      (the first keys met, so the frequent ones) in shared memory first
-//   4. group id = output row: finalized in place, outputs allocated for as
-//      many groups as rows
+//   4. group id = output row: finalized by a kernel of its own into outputs
+//      allocated for the groups that there are
 // The records, exact float sums and output rules are the general plan's.
 // ===========================================================================
 constexpr int kSmallThreads = 512;
@@ -1819,6 +1819,13 @@ __device__ __forceinline__ void small_flush(const SmallArgs& a, const uint32_t* 
   }
 }
 
+// Out of line: inlined beside the accumulation, it cost wide NUNIQUE calls a
+// fifth more (131,072 rows, six float64 columns of 1,000 groups: 1,290 -> 1,070 us).
+__device__ __noinline__ bool small_pair_insert(const SmallArgs& a, int ci, uint32_t id, int64_t r)
+{
+  return pair_insert(a.f.p, a.f.p.c[ci], id, r);
+}
+
 template <KeyMode M>
 __global__ void __launch_bounds__(kSmallThreads, 1) small_groupby_kernel(const __grid_constant__ SmallArgs a)
 {
@@ -1905,17 +1912,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_groupby_kernel(const _
       for (int ci = 0; ci < p.ncols; ++ci) {
         const ColPlan& c = p.c[ci];
         if (c.cw) small_accumulate(a, sh, ci, id[j], r);
-        if ((c.states & ST_NDIST) && dvalid(c.col, r) && pair_insert(p, c, id[j], r))
+        if ((c.states & ST_NDIST) && dvalid(c.col, r) && small_pair_insert(a, ci, id[j], r))
           red_add(rec0 + id[j] + c.off_nd * a.f.ld, 1);
       }
     }
   }
   __syncthreads();
   for (uint32_t id = threadIdx.x; id < static_cast<uint32_t>(a.hot); id += kSmallThreads) small_flush(a, sh, id);
-  cluster_sync();
-  // 4. output rows
-  const int64_t groups = __ldcg(a.ngroups);
-  for (int64_t i = tid; i < groups; i += total) finalize_row(a.f, i);
 }
 
 // Rows up to which one cluster takes the whole call: its 16 SMs are still
@@ -2037,8 +2040,6 @@ bool small_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, cons
   a.f.ld            = static_cast<uint64_t>(n);
   a.f.key_mode      = static_cast<int>(M);
   a.f.special_ids   = a.special_ids;
-  Buffer<int32_t> repr;
-  bind_outputs(al, table, keys, nkeys, aggs, naggs, agg_col, M == KeyMode::GEN, n, out, a.f, repr);
   // up to 16 CTAs (the largest cluster), about four rows a thread
   unsigned ctas = 1;
   while (ctas < most && static_cast<int64_t>(ctas) * kSmallThreads * 2 < n) ctas *= 2;
@@ -2046,19 +2047,14 @@ bool small_groupby(const OpContext& ctx, GbPlan p, const ldf_column* table, cons
   unsigned int h[2] = {0, 0};  // groups, overflow
   ctx.fetch(h, misc, sizeof(h));
   ctx.finish();
-  if (h[1] != 0) {
-    for (int j = 0; j < nkeys + naggs; ++j) free_out_column(al, out[j]);
-    return false;
-  }
+  if (h[1] != 0) return false;
   const int64_t G = h[0];
-  for (int j = 0; j < nkeys + naggs; ++j) out[j].size = G;
-  bool strings = false;
+  a.f.ngroups     = G;
+  Buffer<int32_t> repr;
+  bind_outputs(al, table, keys, nkeys, aggs, naggs, agg_col, M == KeyMode::GEN, G, out, a.f, repr);
+  launch("finalize", finalize_kernel, gs_blocks(G, 256), 256, 0, s, a.f);
   for (int j = 0; j < nkeys; ++j)
-    if (table[keys[j]].type == LDF_STRING) {
-      gather_strings(ctx, make_dcol(table[keys[j]]), repr.get(), G, out[j]);
-      strings = true;
-    }
-  if (strings) ctx.finish();
+    if (table[keys[j]].type == LDF_STRING) gather_strings(ctx, make_dcol(table[keys[j]]), repr.get(), G, out[j]);
   return true;
 }
 
