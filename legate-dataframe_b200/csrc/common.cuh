@@ -110,9 +110,13 @@ inline void launch_cluster(const char* name, void (*kernel)(KArgs...), unsigned 
 // Device memory of one call.  allocate/deallocate go straight to the
 // caller's allocator (outputs use them: the caller owns what they return).
 // Scratch buffers (Buffer<T>) of at most kSmallScratch bytes are carved from
-// chunks of kScratchChunk bytes (four times that from the second on) instead,
-// which are handed back when the Allocator is destroyed at the end of the call:
-// one allocator round trip per chunk rather than per buffer.
+// chunks of kScratchChunk bytes instead, which are handed back when the
+// Allocator is destroyed at the end of the call: one allocator round trip per
+// chunk rather than per buffer.  A carved buffer's room is carved again (in
+// stream order) once it and all that were carved after it are given back, so
+// that a loop over buffers of its own takes no more than one round of it.
+// Where the pool has no room for a chunk, a buffer gets an allocation of its
+// own size.
 class Allocator {
  public:
   static constexpr size_t kSmallScratch = size_t(8) << 20;
@@ -129,11 +133,19 @@ class Allocator {
   cudaStream_t stream() const { return s_; }
 
  private:
+  struct Block {
+    char* p;
+    size_t chunk, at;  // chunks_[chunk] from byte `at` on
+    bool live;
+  };
+  void* try_allocate(size_t nbytes) const;
+  void add_chunk(size_t nbytes) const;
+
   const ldf_allocator* a_;
   cudaStream_t s_;
-  mutable std::vector<std::pair<void*, size_t>> chunks_;
-  mutable char* bump_  = nullptr;
-  mutable size_t left_ = 0;
+  mutable std::vector<std::pair<char*, size_t>> chunks_;
+  mutable std::vector<Block> blocks_;       // carved and not yet room again, in order
+  mutable size_t chunk_ = 0, used_ = 0;     // the chunk carved from, its bytes in use
 };
 
 template <typename T>

@@ -93,11 +93,8 @@ cudaStream_t staging_stream()
   return streams[dev];
 }
 
-void* Allocator::allocate(size_t nbytes) const
+void* Allocator::try_allocate(size_t nbytes) const
 {
-  if (nbytes == 0) nbytes = 16;
-  // Round to 256 B so vectorised accesses never cross an allocation end.
-  nbytes = (nbytes + 255) & ~size_t(255);
   void* p = nullptr;
   if (a_ && a_->allocate) {
     p = a_->allocate(a_->ctx, nbytes, static_cast<void*>(s_));
@@ -107,6 +104,15 @@ void* Allocator::allocate(size_t nbytes) const
       p = nullptr;
     }
   }
+  return p;
+}
+
+void* Allocator::allocate(size_t nbytes) const
+{
+  if (nbytes == 0) nbytes = 16;
+  // Round to 256 B so vectorised accesses never cross an allocation end.
+  nbytes  = (nbytes + 255) & ~size_t(255);
+  void* p = try_allocate(nbytes);
   if (p == nullptr)
     fail(LDF_ERR_OUT_OF_MEMORY, "device allocation of " + std::to_string(nbytes) + " bytes failed");
   return p;
@@ -124,20 +130,30 @@ void Allocator::deallocate(void* p, size_t nbytes) const
   }
 }
 
+// One more chunk, of nbytes where a whole one is not to be had.
+void Allocator::add_chunk(size_t nbytes) const
+{
+  chunks_.reserve(chunks_.size() + 1);
+  size_t size = kScratchChunk;
+  void* p     = try_allocate(size);
+  if (p == nullptr) p = allocate(size = nbytes);
+  chunks_.emplace_back(static_cast<char*>(p), size);
+}
+
 void* Allocator::allocate_scratch(size_t nbytes) const
 {
   if (nbytes == 0) nbytes = 16;
   nbytes = (nbytes + 255) & ~size_t(255);
   if (nbytes > kSmallScratch) return allocate(nbytes);
-  if (left_ < nbytes) {
-    const size_t chunk = chunks_.empty() ? kScratchChunk : 4 * kScratchChunk;
-    bump_              = static_cast<char*>(allocate(chunk));
-    chunks_.emplace_back(bump_, chunk);
-    left_ = chunk;
+  if (chunks_.empty()) add_chunk(nbytes);
+  while (chunks_[chunk_].second - used_ < nbytes) {
+    if (chunk_ + 1 == chunks_.size()) add_chunk(nbytes);
+    ++chunk_;
+    used_ = 0;
   }
-  void* p = bump_;
-  bump_ += nbytes;
-  left_ -= nbytes;
+  char* p = chunks_[chunk_].first + used_;
+  blocks_.push_back(Block{p, chunk_, used_, true});
+  used_ += nbytes;
   return p;
 }
 
@@ -146,8 +162,20 @@ void Allocator::deallocate_scratch(void* p, size_t nbytes) const
   if (p == nullptr) return;
   if (nbytes == 0) nbytes = 16;
   nbytes = (nbytes + 255) & ~size_t(255);
-  if (nbytes > kSmallScratch) deallocate(p, nbytes);
-  // small scratch lives until its chunk is returned
+  if (nbytes > kSmallScratch) {
+    deallocate(p, nbytes);
+    return;
+  }
+  for (size_t k = blocks_.size(); k-- > 0;)
+    if (blocks_[k].p == p) {
+      blocks_[k].live = false;
+      break;
+    }
+  while (!blocks_.empty() && !blocks_.back().live) {
+    chunk_ = blocks_.back().chunk;
+    used_  = blocks_.back().at;
+    blocks_.pop_back();
+  }
 }
 
 Allocator::~Allocator()

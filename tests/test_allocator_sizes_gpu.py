@@ -56,3 +56,44 @@ def test_groupby_outputs_are_sized_to_the_groups(n, groups, string):
         N.check(L.ldf_b200_free_column(ctypes.byref(c), ctypes.byref(struct), stream))
     torch.cuda.synchronize()
     assert wrong == [] and live == {}
+
+
+def test_sort_scratch_does_not_grow_with_string_length():
+    """20,000 distinct strings that differ behind a common prefix: the scratch of
+    the chunk after chunk ranking at 1,600 bytes is that at 64."""
+    import pyarrow as pa
+    import torch
+
+    from legate_dataframe import LogicalTable
+    from legate_dataframe import _native as N
+
+    def scratch_peak(prefix):
+        n = 20_000
+        order = np.random.default_rng(prefix).permutation(n)
+        col = LogicalTable.from_arrow(pa.table({"k": ["p" * prefix + f"{x:06d}" for x in order.tolist()]})).get_column("k")
+        c = (N.ldf_column * 1)()
+        c[0].type, c[0].nullable, c[0].size, c[0].data = N.LDF_STRING, 0, n, col.data.data_ptr()
+        c[0].chars, c[0].chars_base, c[0].num_chars = col.chars.data_ptr(), col.chars_base, col.num_chars
+        struct, (take, give), live, wrong = ledger_allocator(N, torch)
+        peak = 0
+
+        def counted(ctx, nbytes, stream):
+            nonlocal peak
+            p = take(ctx, nbytes, stream)
+            peak = max(peak, sum(size for size, _ in live.values()))
+            return p
+
+        counted_cb = N.ALLOC_FN(counted)
+        struct = N.ldf_allocator(None, counted_cb, give)
+        out = (N.ldf_column * 1)()
+        stream = ctypes.c_void_p(N.current_stream_handle())
+        N.check(N.lib().ldf_b200_sort(c, 1, N.int32_array([0]), (ctypes.c_uint8 * 1)(1), 1, 1, 1, -(2**63), out,
+                                      ctypes.byref(struct), stream))
+        got = np.frombuffer(live[out[0].chars][1].cpu().numpy().tobytes()[: out[0].num_chars], "S%d" % (prefix + 6))
+        assert np.array_equal(got, np.sort(got)) and len(np.unique(got)) == n
+        held = sum(live[p][0] for p in (out[0].data, out[0].chars))
+        N.check(N.lib().ldf_b200_free_column(ctypes.byref(out[0]), ctypes.byref(struct), stream))
+        assert live == {} and wrong == []
+        return peak - held
+
+    assert scratch_peak(1600) <= scratch_peak(64) + (1 << 20)
