@@ -59,8 +59,8 @@ def test_groupby_outputs_are_sized_to_the_groups(n, groups, string):
 
 
 def test_sort_scratch_does_not_grow_with_string_length():
-    """20,000 distinct strings that differ behind a common prefix: the scratch of
-    the chunk after chunk ranking at 1,600 bytes is that at 64."""
+    """20,000 distinct strings that differ behind one of two prefixes: the scratch
+    of the chunk after chunk ranking at 1,600 bytes is that at 64."""
     import pyarrow as pa
     import torch
 
@@ -70,7 +70,7 @@ def test_sort_scratch_does_not_grow_with_string_length():
     def scratch_peak(prefix):
         n = 20_000
         order = np.random.default_rng(prefix).permutation(n)
-        col = LogicalTable.from_arrow(pa.table({"k": ["p" * prefix + f"{x:06d}" for x in order.tolist()]})).get_column("k")
+        col = LogicalTable.from_arrow(pa.table({"k": ["pq"[x % 2] * prefix + f"{x:06d}" for x in order.tolist()]})).get_column("k")
         c = (N.ldf_column * 1)()
         c[0].type, c[0].nullable, c[0].size, c[0].data = N.LDF_STRING, 0, n, col.data.data_ptr()
         c[0].chars, c[0].chars_base, c[0].num_chars = col.chars.data_ptr(), col.chars_base, col.num_chars
