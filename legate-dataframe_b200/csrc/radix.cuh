@@ -223,8 +223,10 @@ bool rank_sort(const OpContext& ctx, const ldf_column* table, int ncols, const s
                int64_t first, int64_t rows, ldf_column* out);
 
 // rank[d] = bytewise rank of the string of row repr[d] among the D distinct
-// strings of rows repr[0..D), for D of at most kRankStrings.
+// strings of rows repr[0..D), for D of at most kRankStrings; longest: bytes of
+// the longest of them.
 constexpr int64_t kRankStrings = 8192;
-void rank_distinct_strings(const OpContext& ctx, const DCol& col, const int32_t* repr, int64_t D, uint32_t* rank);
+void rank_distinct_strings(const OpContext& ctx, const DCol& col, const int32_t* repr, int64_t D, int64_t longest,
+                           uint32_t* rank);
 
 }  // namespace ldf

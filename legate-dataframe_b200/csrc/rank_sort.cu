@@ -182,16 +182,24 @@ void launch_rank_sort(const OpContext& ctx, RankSortArgs& a)
 }
 
 // ---- ranks of a few thousand distinct strings -------------------------------
-constexpr int kHeadWords = 4;  // first 32 bytes, big-endian
+// Ranked on their first 32 bytes, as rank_sort_kernel ranks rows; while strings
+// of equal bytes so far both go on, in rounds on the rank so far and the next 24.
+constexpr int kHeadWords = 4;
 constexpr int kHeadTile  = 256;
+constexpr int kHeadBytes = 8 * kHeadWords;
+constexpr int kNextBytes = kHeadBytes - 8;
 
-__global__ void __launch_bounds__(256) string_heads_kernel(DCol col, const int32_t* repr, int64_t D, uint64_t* heads)
+// heads: bytes [from, from + 32) of every string, big-endian and zero-padded;
+// from != 0: its rank so far, then bytes [from, from + 24).
+__global__ void __launch_bounds__(256) string_heads_kernel(DCol col, const int32_t* repr, int64_t D, int64_t from,
+                                                           const uint32_t* rank, uint64_t* heads, uint32_t* lens)
 {
   const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (d >= D) return;
-  const int64_t r  = repr[d];
-  const uint8_t* p = dstr_ptr(col, r);
-  const int64_t n  = dstr_len(col, r);
+  const int64_t r   = repr[d];
+  const int64_t len = dstr_len(col, r);
+  const uint8_t* p  = dstr_ptr(col, r) + (len > from ? from : 0);
+  const int64_t n   = len > from ? (len - from < kHeadBytes ? len - from : kHeadBytes) : 0;
   uint64_t w[kHeadWords];
   if (!str_words(col, p, n, w)) {
 #pragma unroll
@@ -201,46 +209,47 @@ __global__ void __launch_bounds__(256) string_heads_kernel(DCol col, const int32
         if (8 * k + b < n) w[k] |= static_cast<uint64_t>(p[8 * k + b]) << (8 * b);
     }
   }
+  const int shift = from != 0 ? 1 : 0;
 #pragma unroll
   for (int k = 0; k < kHeadWords; ++k) {
+    if (k + shift >= kHeadWords) continue;
     const uint32_t lo = static_cast<uint32_t>(w[k]), hi = static_cast<uint32_t>(w[k] >> 32);
-    heads[k * D + d] = (static_cast<uint64_t>(__byte_perm(lo, 0, 0x0123)) << 32) | __byte_perm(hi, 0, 0x0123);
+    heads[(k + shift) * D + d] =
+      (static_cast<uint64_t>(__byte_perm(lo, 0, 0x0123)) << 32) | __byte_perm(hi, 0, 0x0123);
   }
+  if (shift) heads[d] = rank[d];
+  lens[d] = static_cast<uint32_t>(len < 0xffffffffll ? len : 0xffffffffll);
 }
 
-// Strings a and b of equal (zero-padded) heads: a sorts before b.
-__device__ __forceinline__ bool tail_less(const DCol& col, int64_t ra, int64_t rb)
-{
-  const int64_t la = dstr_len(col, ra), lb = dstr_len(col, rb);
-  const int64_t m  = la < lb ? la : lb;
-  const uint8_t *pa = dstr_ptr(col, ra), *pb = dstr_ptr(col, rb);
-  for (int64_t i = 8 * kHeadWords; i < m; ++i)
-    if (pa[i] != pb[i]) return pa[i] < pb[i];
-  return la < lb;
-}
-
-// Same scheme as rank_sort_kernel; the strings are distinct, so no row ties
-// with another, and bytes beyond the heads are read only where the heads of
-// two strings are equal.  Sorting 8,000 distinct ids of 8 to 24 characters:
-// 509 -> 251 us a call against radix passes over 8-byte chunks with their
-// read-backs (100 rows of 50 ids: 465 -> 158 us).
-__global__ void __launch_bounds__(kRankThreads) rank_strings_kernel(DCol col, const int32_t* repr, int64_t D,
-                                                                    const uint64_t* heads, uint32_t* rank)
+// rank[d] = strings that sort before string d; covered: the bytes that the
+// heads stand for.  Of two strings of equal heads the one that ends within them
+// is a prefix of the other; two that both go on tie (*ties = 1), and share
+// their rank.  Sorting 8,000 distinct ids of 8 to 24 characters: 509 -> 251 us a
+// call against radix passes over 8-byte chunks with their read-backs (100 rows
+// of 50 ids: 465 -> 158 us).
+__global__ void __launch_bounds__(kRankThreads) rank_strings_kernel(int64_t D, const uint64_t* heads,
+                                                                    const uint32_t* lens, int64_t covered,
+                                                                    uint32_t* rank, int* ties)
 {
   __shared__ uint64_t tile[kHeadWords][kHeadTile];
+  __shared__ uint32_t tile_len[kHeadTile];
   __shared__ uint32_t part[kRankWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane;
   uint64_t w[kHeadWords];
 #pragma unroll
   for (int k = 0; k < kHeadWords; ++k) w[k] = i < D ? __ldg(heads + k * D + i) : 0;
-  uint32_t cnt = 0;
+  const uint32_t len = i < D ? __ldg(lens + i) : 0;
+  uint32_t cnt       = 0;
+  int tie            = 0;
   for (int64_t t0 = 0; t0 < D; t0 += kHeadTile) {
     const int m = static_cast<int>(D - t0 < kHeadTile ? D - t0 : kHeadTile);
     __syncthreads();
-    if (static_cast<int>(threadIdx.x) < m)
+    if (static_cast<int>(threadIdx.x) < m) {
 #pragma unroll
       for (int k = 0; k < kHeadWords; ++k) tile[k][threadIdx.x] = __ldg(heads + k * D + t0 + threadIdx.x);
+      tile_len[threadIdx.x] = __ldg(lens + t0 + threadIdx.x);
+    }
     __syncthreads();
     const int per = (m + kRankWarps - 1) / kRankWarps;
     const int lo = warp * per, hi = min(m, lo + per);
@@ -252,14 +261,17 @@ __global__ void __launch_bounds__(kRankThreads) rank_strings_kernel(DCol col, co
 #pragma unroll
         for (int k = 0; k < kHeadWords; ++k) x[k] = tile[k][j];
         lt = words_less<kHeadWords>(x, w);
-        if (!lt && i < D && x[1] == w[1] && x[2] == w[2] && x[3] == w[3] && t0 + j != i)
-          lt = tail_less(col, repr[t0 + j], repr[i]);
+        if (!lt && x[1] == w[1] && x[2] == w[2] && x[3] == w[3] && t0 + j != i) {
+          const uint32_t l = tile_len[j];
+          if (l <= covered || len <= covered) lt = l < len;
+          else tie = 1;
+        }
       }
       cnt += lt ? 1u : 0u;
     }
   }
   part[warp][lane] = cnt;
-  __syncthreads();
+  if (__syncthreads_or(tie != 0 && i < D) && threadIdx.x == 0) *ties = 1;
   if (warp != 0 || i >= D) return;
   uint32_t r = 0;
 #pragma unroll
@@ -269,14 +281,32 @@ __global__ void __launch_bounds__(kRankThreads) rank_strings_kernel(DCol col, co
 
 }  // namespace
 
-void rank_distinct_strings(const OpContext& ctx, const DCol& col, const int32_t* repr, int64_t D, uint32_t* rank)
+void rank_distinct_strings(const OpContext& ctx, const DCol& col, const int32_t* repr, int64_t D, int64_t longest,
+                           uint32_t* rank)
 {
   LDF_REQUIRE(D >= 1 && D <= kRankStrings, "rank_distinct_strings: too many strings");
+  cudaStream_t s = ctx.stream();
   Buffer<uint64_t> heads(ctx.alloc(), kHeadWords * D);
-  launch("string_heads", string_heads_kernel, static_cast<unsigned>(ceil_div(D, 256)), 256, 0, ctx.stream(), col, repr,
-         D, heads.get());
-  launch("rank_strings", rank_strings_kernel, static_cast<unsigned>(ceil_div(D, 32)), kRankThreads, 0, ctx.stream(),
-         col, repr, D, static_cast<const uint64_t*>(heads.get()), rank);
+  Buffer<uint32_t> lens(ctx.alloc(), D);
+  Buffer<int> ties(ctx.alloc(), 1);
+  auto round = [&](int64_t from, int64_t covered) {
+    LDF_CUDA(cudaMemsetAsync(ties.get(), 0, sizeof(int), s));
+    launch("string_heads", string_heads_kernel, static_cast<unsigned>(ceil_div(D, 256)), 256, 0, s, col, repr, D, from,
+           static_cast<const uint32_t*>(rank), heads.get(), lens.get());
+    launch("rank_strings", rank_strings_kernel, static_cast<unsigned>(ceil_div(D, 32)), kRankThreads, 0, s, D,
+           static_cast<const uint64_t*>(heads.get()), static_cast<const uint32_t*>(lens.get()), covered, rank,
+           ties.get());
+  };
+  int64_t covered = kHeadBytes;
+  round(0, covered);
+  while (longest > covered) {
+    int tied = 0;
+    ctx.fetch(&tied, ties.get(), sizeof(int));
+    ctx.finish();
+    if (tied == 0) break;
+    round(covered, covered + kNextBytes);
+    covered += kNextBytes;
+  }
 }
 
 bool rank_sort(const OpContext& ctx, const ldf_column* table, int ncols, const std::vector<SortKeyDesc>& kd, int64_t n,

@@ -161,10 +161,11 @@ __global__ void distinct_stats_kernel(const unsigned int* count, int64_t cap, un
 // slot -> dense distinct id; distinct id -> representative row.  The
 // occupied slots of a warp take their ids with one atomic (order is
 // irrelevant: the ids get sorted).
-__global__ void str_compact_kernel(const unsigned long long* slots, uint64_t cap, int32_t* slot_id,
-                                   int32_t* repr, unsigned long long* count)
+__global__ void str_compact_kernel(DCol col, const unsigned long long* slots, uint64_t cap, int32_t* slot_id,
+                                   int32_t* repr, unsigned long long* count, unsigned long long* max_len)
 {
-  const int lane = threadIdx.x & 31;
+  const int lane            = threadIdx.x & 31;
+  unsigned long long longest = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   // every lane of a warp runs the same number of iterations (ballots below)
   for (int64_t base = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); base < static_cast<int64_t>(cap);
@@ -181,7 +182,10 @@ __global__ void str_compact_kernel(const unsigned long long* slots, uint64_t cap
     const unsigned long long d = first + __popc(ballot & ((1u << lane) - 1u));
     slot_id[i]                 = static_cast<int32_t>(d);
     repr[d]                    = static_cast<int32_t>(v >> 32);
+    longest                    = max(longest, static_cast<unsigned long long>(dstr_len(col, v >> 32)));
   }
+  for (int d = 16; d > 0; d >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, d));
+  if (lane == 0 && longest != 0) atomicMax(max_len, longest);
 }
 
 // chunk c (8 bytes, big-endian, zero padded) of each distinct string
@@ -233,15 +237,6 @@ __global__ void row_rank_kernel(const int32_t* row_slot, const int32_t* slot_id,
     if (rep_out) rep_out[r] = d >= 0 ? repr[d] : -1;
   }
 }
-__global__ void max_len_kernel(DCol col, const int32_t* repr, int64_t D, unsigned long long* out)
-{
-  unsigned long long m = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x)
-    m = max(m, static_cast<unsigned long long>(dstr_len(col, repr[i])));
-  for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 unsigned blocks_for(int64_t n)
 {
   int64_t b   = ceil_div(n, 256);
@@ -337,7 +332,7 @@ int64_t string_ranks(const OpContext& ctx, const DCol& col, int64_t n, uint32_t*
   Buffer<unsigned long long> slots;
   Buffer<int32_t> slot_id;
   Buffer<int32_t> repr(al, n);
-  int64_t D = 0;
+  int64_t D = 0, L = 0;  // distinct strings, length of the longest
   int* overflow              = reinterpret_cast<int*>(misc.get());
   unsigned long long* dcount = reinterpret_cast<unsigned long long*>(misc.get() + 1);
   unsigned long long* maxlen = reinterpret_cast<unsigned long long*>(misc.get() + 2);
@@ -350,11 +345,12 @@ int64_t string_ranks(const OpContext& ctx, const DCol& col, int64_t n, uint32_t*
     // compacted at once: a table that overflowed is compacted in vain, one
     // that did not (the usual case) needs a single read-back
     slot_id = Buffer<int32_t>(al, cap);
-    launch("str_compact", str_compact_kernel, blocks_for(cap), 256, 0, s, slots.get(), cap, slot_id.get(), repr.get(),
-           dcount);
+    launch("str_compact", str_compact_kernel, blocks_for(cap), 256, 0, s, col, slots.get(), cap, slot_id.get(),
+           repr.get(), dcount, maxlen);
     int ov = 0;
     ctx.fetch(&ov, overflow, sizeof(int));
     ctx.fetch(&D, dcount, sizeof(D));
+    ctx.fetch(&L, maxlen, sizeof(L));
     ctx.finish();
     if (ov == 0) break;
     const uint64_t full = static_cast<uint64_t>(2 * n + 64);
@@ -363,11 +359,8 @@ int64_t string_ranks(const OpContext& ctx, const DCol& col, int64_t n, uint32_t*
   }
   Buffer<uint32_t> rank(al, std::max<int64_t>(D, 1));
   if (D > 0 && D <= kRankStrings) {
-    rank_distinct_strings(ctx, col, repr.get(), D, rank.get());
+    rank_distinct_strings(ctx, col, repr.get(), D, L, rank.get());
   } else if (D > 0) {
-    launch("max_len", max_len_kernel, blocks_for(D), 256, 0, s, col, repr.get(), D, maxlen);
-    LDF_CHECK_LAUNCH();
-    const int64_t L = ctx.read_i64(misc.get() + 2);
     LDF_CUDA(cudaMemsetAsync(rank.get(), 0, D * 4, s));
     Buffer<uint64_t> word(al, D);
     Buffer<uint32_t> lens(al, D);
