@@ -52,10 +52,18 @@ constexpr int kProbeThreads = 256;
 constexpr int kProbeItems   = 4;
 constexpr int kProbeTile    = kProbeThreads * kProbeItems;
 constexpr uint64_t kEmpty64 = ~0ull;
-// Fewest build rows for which a direct-address table, and packed payload
-// records, are considered.
-constexpr int64_t kDirectMinRows = int64_t(1) << 17;
-constexpr int64_t kPackMinRows   = int64_t(1) << 17;
+// Whether a direct-address table, and packed payload records, are considered.
+// They cost a read-back of the key range and a pass over the build rows, which
+// large build sides and many probe rows outweigh: against the hash table, dense
+// int32 keys and two payload columns, 100,000 probe rows on 10,000 / 120,000
+// build rows take 131 us instead of 125 / 144 instead of 135, 5M probe rows 219
+// instead of 228 / 249 instead of 261 us, 50M 0.90 instead of 1.15 / 1.06 instead
+// of 1.36 ms.  A table of 1,000 rows is slower the more rows probe it (50M: 2.6
+// instead of 1.5 ms): its few lines are wanted by every SM at once.
+inline bool direct_considered(int64_t n_build, int64_t n_probe)
+{
+  return n_build >= int64_t(1) << 17 || (n_build >= int64_t(1) << 13 && n_probe >= int64_t(1) << 21);
+}
 
 struct Slot16 {
   uint64_t key;
@@ -1106,13 +1114,10 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
   // Dense integer keys: when the build keys' value range is at most twice the
   // build rows (and 2^31), a direct-address table of build rows replaces the
   // hash table.  The table is 4 bytes per key value, so the probe's lookups
-  // mostly stay in L2, and probe keys outside the range need no lookup at
-  // all.  Below kDirectMinRows the hash table stays in L2 by itself, and the
-  // range's read-back outweighs what the lookups save: both take 147 us at
-  // 131,072 x 131,072 int32 rows, the hash table 131 us at 20,000.
+  // mostly stay in L2, and probe keys outside the range need no lookup at all.
   Buffer<int32_t> direct;
   unsigned long long dup = 0;
-  if (M != KeyMode::GEN && !plan && n_build >= kDirectMinRows && !is_float(bk.c[0].type)) {
+  if (M != KeyMode::GEN && !plan && direct_considered(n_build, n_probe) && !is_float(bk.c[0].type)) {
     unsigned long long* mm = misc.get() + 4;
     launch("key_range", key_range_kernel, grid_stride_blocks(n_build, 256), 256, 0, s, bk.c[0], n_build, mm);
     unsigned long long h[3];
@@ -1233,9 +1238,8 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
   }
 
   // Build-side outputs: the build key column comes from the probe key, and two
-  // other non-nullable fixed-width columns of a table too large for L2 are
-  // packed into one 16-byte record per build row, so a matched probe row
-  // reads them with one random access.
+  // other non-nullable fixed-width columns are packed into one 16-byte record
+  // per build row, so a matched probe row reads them with one random access.
   a.rkey = -1;
   Buffer<ulonglong2> rpack;
   if (M != KeyMode::GEN && !need_maps && tiles > 0 && n_build > 0) {
@@ -1244,7 +1248,7 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
       if (a.rkey < 0 && ro.src[j].data == bk.c[0].data && ro.src[j].type == bk.c[0].type) a.rkey = j;
       else rest.push_back(j);
     }
-    bool packable = rest.size() == 2 && n_build >= kPackMinRows;
+    bool packable = rest.size() == 2 && direct_considered(n_build, n_probe);
     for (int j : rest) packable = packable && ro.src[j].valid == nullptr && ro.src[j].type != LDF_STRING;
     if (packable) {
       const DCol& c0 = ro.src[rest[0]];
