@@ -1921,10 +1921,17 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_groupby_kernel(const _
   for (uint32_t id = threadIdx.x; id < static_cast<uint32_t>(a.hot); id += kSmallThreads) small_flush(a, sh, id);
 }
 
-// Rows up to which one cluster takes the whole call: its 16 SMs are still
-// ahead of the general plan there (131,072 rows of one group each: 219 us
-// against 409; of 131 groups 118 against 253).
+// Whether one cluster takes the whole call: up to 131,072 rows its 16 SMs are
+// still ahead of the general plan (six columns of SUM, MIN, MAX and MEAN over one
+// group a row: 659 us against 730; of 10 groups 374 against 581), but not with
+// many NUNIQUE columns, whose pair sets are random global atomics: 131,072 rows
+// of 6,500 groups with 2 of them take 404 us against 484, with 4 718 against 680
+// (of 10 groups 683 against 813), with 6 1,047 against 860.
 constexpr int64_t kSmallGroupbyRows = int64_t(1) << 17;
+inline bool small_plan(int64_t rows, int nunique_columns)
+{
+  return rows > 0 && rows <= kSmallGroupbyRows && rows * nunique_columns <= 4 * kSmallGroupbyRows;
+}
 
 // The largest cluster of at most `want` CTAs (a power of two) that fits (0:
 // none); active(c): clusters of c CTAs that the device holds at once.
@@ -3814,7 +3821,9 @@ void groupby_aggregation(const ldf_column* table, int ncols, const int32_t* keys
       fail(LDF_ERR_UNSUPPORTED, "min/max of a string column is not supported");
   }
   if (try_partitioned(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out, hs, col_of_plan)) return;
-  if (n > 0 && n <= kSmallGroupbyRows && hs.staged_bytes() == 0) {
+  int nunique = 0;
+  for (int ci = 0; ci < p.ncols; ++ci) nunique += (p.c[ci].states & ST_NDIST) ? 1 : 0;
+  if (small_plan(n, nunique) && hs.staged_bytes() == 0) {
     const KeyMode m = key_mode(k);
     if (m == KeyMode::K32 ? small_groupby<KeyMode::K32>(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out)
         : m == KeyMode::K64 ? small_groupby<KeyMode::K64>(ctx, p, table, keys, nkeys, aggs, naggs, agg_col, out)
