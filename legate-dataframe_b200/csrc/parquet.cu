@@ -1328,7 +1328,7 @@ unsigned pq_blocks(int64_t work, int threads)
 constexpr int64_t kFragBytes    = 65536;
 constexpr int kFragSeg          = 4096;
 constexpr int kExitThreads      = 256;
-constexpr int64_t kFragMaxInput = int64_t(128) << 20;  // stream bytes per round (8 bytes of exits each)
+constexpr int64_t kFragMaxInput = int64_t(128) << 20;  // bytes per round of pages (8 bytes of exits each)
 // Ring of recent output of a fragment's warp.  8 KB lets 14 warps share an SM
 // where the per-page kernel's 32 KB lets 5 (4.5 ms); copies from further back
 // read the output (median offset 1 to 3 KB).
@@ -1504,12 +1504,24 @@ __global__ void __launch_bounds__(kLanes) snap_fragment_kernel(const uint8_t* fi
 // per segment.  For pages of 20,000 strings 0.8 ms and 0.7 ms in the data
 // kernel, whose thread 0 walked the prefixes in 4.3 ms.
 constexpr int kPlainChainMin     = 256;  // values from which a page takes this path
-constexpr int64_t kPlainMaxInput = int64_t(512) << 20;  // page bytes per call (8 bytes of exits each)
+constexpr int64_t kPlainMaxInput = int64_t(512) << 20;  // larger pages are walked by the data kernel
 struct PlainPage {
   int page;
   int nullable;
-  int64_t exit0, seg0, entry0;
+  int64_t exit0, seg0;  // first exit and segment in the page's round
+  int64_t entry0;
 };
+struct PageRound {  // pages [first, first + count) of a list, kFragMaxInput bytes or one page
+  size_t first, count;
+  int64_t in, segs, frags;  // bytes with exits, segments, fragments
+};
+// The round that takes `bytes` more bytes with exits; `next`: the list's pages so far.
+PageRound& round_for(std::vector<PageRound>& rounds, size_t next, int64_t bytes)
+{
+  if (rounds.empty() || (rounds.back().in > 0 && rounds.back().in + bytes > kFragMaxInput))
+    rounds.push_back(PageRound{next, 0, 0, 0, 0});
+  return rounds.back();
+}
 
 // A data page's value bytes (behind its definition levels).
 __device__ __forceinline__ const uint8_t* page_values(const PqPage& pg, bool nullable, int64_t& n)
@@ -1727,7 +1739,8 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   std::vector<int64_t> covered(ncols, 0);
   std::vector<int> frag, dict_strings, dict_chain, data_pages;
   std::vector<PlainPage> plain;
-  int64_t scratch_bytes = 0, nentries = 0, dict_in = 0, plain_in = 0, plain_segs = 0;
+  std::vector<PageRound> plain_rounds;
+  int64_t scratch_bytes = 0, nentries = 0, dict_in = 0;
   std::vector<PqPage> dev_pages(npages);
   for (int p = 0; p < npages; ++p) {
     const ldf_parquet_page& h = pages[p];
@@ -1769,18 +1782,18 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
                     "parquet_decode: a dictionary-encoded page without its dictionary");
       LDF_REQUIRE(h.row0 >= 0 && h.row0 + h.num_values <= nrows, "parquet_decode: page rows out of range");
       if (h.encoding == 0 && C.physical[h.column] == LDF_PQ_BYTE_ARRAY && h.num_values >= kPlainChainMin) {
-        PlainPage f{};
-        f.page     = p;
-        f.nullable = C.nullable[h.column];
-        f.exit0    = plain_in;
-        f.seg0     = plain_segs;
-        f.entry0   = nentries;
-        plain_in += dev_pages[p].data_bytes;
-        plain_segs += ceil_div(dev_pages[p].data_bytes, int64_t(kFragSeg));
-        if (plain_in > kPlainMaxInput) {  // its bytes' exits would take too much room: walked by the data kernel
-          plain_in   = f.exit0;
-          plain_segs = f.seg0;
-        } else {
+        const int64_t bytes = dev_pages[p].data_bytes;
+        if (bytes <= kPlainMaxInput) {
+          PageRound& r = round_for(plain_rounds, plain.size(), bytes);
+          PlainPage f{};
+          f.page     = p;
+          f.nullable = C.nullable[h.column];
+          f.exit0    = r.in;
+          f.seg0     = r.segs;
+          f.entry0   = nentries;
+          r.in += bytes;
+          r.segs += ceil_div(bytes, int64_t(kFragSeg));
+          ++r.count;
           dev_pages[p].plain0 = nentries;
           nentries += h.num_values;
           plain.push_back(f);
@@ -1838,11 +1851,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   Buffer<unsigned long long> exits;
   Buffer<FragStart> starts;
   if (!frag.empty()) {
-    struct Round {
-      size_t first, count;
-      int64_t in, segs, frags;
-    };
-    std::vector<Round> rounds;
+    std::vector<PageRound> rounds;
     int64_t most_in = 0, most_frags = 0;
     for (size_t q = 0; q < frag.size(); ++q) {
       const ldf_parquet_page& h = pages[frag[q]];
@@ -1855,9 +1864,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
       f.nfrag    = static_cast<int>(std::max<int64_t>(1, ceil_div(f.u, kFragBytes)));
       const int64_t exits_n = f.nfrag > 1 ? f.n : 0;
       f.dst      = scratch.get() + frag_off[q];
-      if (rounds.empty() || (rounds.back().in > 0 && rounds.back().in + exits_n > kFragMaxInput))
-        rounds.push_back(Round{q, 0, 0, 0, 0});
-      Round& r = rounds.back();
+      PageRound& r = round_for(rounds, q, exits_n);
       f.exit0  = r.in;
       f.seg0   = r.segs;
       f.frag0  = r.frags;
@@ -1873,7 +1880,7 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
     starts = Buffer<FragStart>(al, most_frags);
     LDF_CUDA(cudaMemcpyAsync(d_fp.get(), fpages.data(), frag.size() * sizeof(FragPage), cudaMemcpyHostToDevice, s));
     LDF_CUDA(cudaMemsetAsync(d_redo.get(), 0, frag.size() * sizeof(int), s));
-    for (const Round& r : rounds) {
+    for (const PageRound& r : rounds) {
       const FragPage* fp = d_fp.get() + r.first;
       const int np       = static_cast<int>(r.count);
       if (r.segs > 0)
@@ -1967,20 +1974,33 @@ void parquet_decode(const uint8_t* file, int64_t file_bytes, const ldf_parquet_p
   if (!plain.empty()) {
     const int np = static_cast<int>(plain.size());
     Buffer<PlainPage> d_pp(al, np);
-    if (static_cast<int64_t>(exits.size()) < plain_in) exits = Buffer<unsigned long long>(al, plain_in);
-    if (static_cast<int64_t>(starts.size()) < plain_segs) starts = Buffer<FragStart>(al, std::max<int64_t>(plain_segs, 1));
+    int64_t most_in = 1, most_segs = 1;
+    for (const PageRound& r : plain_rounds) {
+      most_in   = std::max(most_in, r.in);
+      most_segs = std::max(most_segs, r.segs);
+    }
+    if (static_cast<int64_t>(exits.size()) < most_in) {
+      exits.reset();
+      exits = Buffer<unsigned long long>(al, most_in);
+    }
+    if (static_cast<int64_t>(starts.size()) < most_segs) {
+      starts.reset();
+      starts = Buffer<FragStart>(al, most_segs);
+    }
     LDF_CUDA(cudaMemcpyAsync(d_pp.get(), plain.data(), np * sizeof(PlainPage), cudaMemcpyHostToDevice, s));
-    if (plain_segs > 0) LDF_CUDA(cudaMemsetAsync(starts.get(), 0xff, plain_segs * sizeof(FragStart), s));
     const PqPage* dp = d_pages.get();
-    if (plain_segs > 0)
-      launch("str_exits", str_exits_kernel, static_cast<unsigned>(plain_segs), kExitThreads, 0, s, dp,
-             static_cast<const PlainPage*>(d_pp.get()), np, exits.get());
-    launch("str_starts", str_starts_kernel, static_cast<unsigned>(np), 32, 0, s, dp,
-           static_cast<const PlainPage*>(d_pp.get()), static_cast<const unsigned long long*>(exits.get()), starts.get());
-    if (plain_segs > 0)
-      launch("str_entries", str_entries_kernel, static_cast<unsigned>(plain_segs), kLanes, 0, s, dp,
-             static_cast<const PlainPage*>(d_pp.get()), np, static_cast<const FragStart*>(starts.get()),
-             entry_off.get(), entry_len.get());
+    for (const PageRound& r : plain_rounds) {
+      if (r.segs == 0) continue;
+      const PlainPage* pp = d_pp.get() + r.first;
+      const int nr        = static_cast<int>(r.count);
+      const unsigned segs = static_cast<unsigned>(r.segs);
+      LDF_CUDA(cudaMemsetAsync(starts.get(), 0xff, r.segs * sizeof(FragStart), s));
+      launch("str_exits", str_exits_kernel, segs, kExitThreads, 0, s, dp, pp, nr, exits.get());
+      launch("str_starts", str_starts_kernel, static_cast<unsigned>(nr), 32, 0, s, dp, pp,
+             static_cast<const unsigned long long*>(exits.get()), starts.get());
+      launch("str_entries", str_entries_kernel, segs, kLanes, 0, s, dp, pp, nr,
+             static_cast<const FragStart*>(starts.get()), entry_off.get(), entry_len.get());
+    }
   }
   if (ndp > 0)
     launch("pq_data", pq_data_kernel, static_cast<unsigned>(ndp), kPqThreads, 0, s,
