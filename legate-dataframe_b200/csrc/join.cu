@@ -421,7 +421,6 @@ struct ProbeArgs {
   int rkey;
   const ulonglong2* rpack;
   int pcol[2];
-  int* err;
 };
 
 // Output rows produced by one probe row with m matches.
@@ -785,7 +784,6 @@ struct TailArgs {
   int32_t* lmap;
   int32_t* rmap;
   int64_t* total;
-  int* err;
 };
 
 __global__ void __launch_bounds__(kProbeThreads) full_tail_kernel(TailArgs a)
@@ -1160,7 +1158,6 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
   a.join_type = join_type;
   a.lo        = lo;
   a.ro        = ro;
-  a.err       = ctx.err();
 
   const bool full = join_type == LDF_JOIN_FULL;
   Buffer<int64_t> d_total(al, 2);
@@ -1291,7 +1288,6 @@ void run_join(const OpContext& ctx, const KeyCols& pk, int64_t n_probe, const Ke
     ta.lmap     = a.lmap;
     ta.rmap     = a.rmap;
     ta.total    = d_total.get() + 1;
-    ta.err      = ctx.err();
     launch("full_tail", full_tail_kernel, static_cast<unsigned>(btiles), kProbeThreads, 0, s, ta);
     LDF_CHECK_LAUNCH();
     int64_t h[2];

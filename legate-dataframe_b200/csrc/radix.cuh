@@ -145,19 +145,10 @@ int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, bo
 constexpr int kTieRunMax = 4096;
 bool order_ties(const OpContext& ctx, const FusedKey& f, const void* words, int word_bytes, int64_t n, int32_t* perm);
 
-// Stable sort of rows by a list of passes (least significant first).
-// Returns the permutation (row ids) in `perm` (n entries, caller allocated).
-// `hist_only` variants are used by the planner.
-struct RadixPlan {
-  std::vector<RadixPass> passes;  // in execution order (LS first)
-};
-
 // Upfront digit histograms of every candidate pass: hist[p * 256 + d].
 void radix_histograms(const OpContext& ctx, const std::vector<RadixPass>& passes, int64_t n,
                       uint32_t* d_hist, const FusedKey* fused = nullptr);
 
-// Run the passes; `perm` receives the row order.  Passes whose histogram has a
-// single bucket holding every row are skipped.
 // Columns the last radix pass moves into sorted order itself: dst[j][pos] =
 // src[j][row] (and the null masks), written as the pass's coalesced runs
 // while the tile's source rows are still in cache.  Widths 1, 2, 4, 8, and 16
@@ -181,6 +172,9 @@ struct RadixPayload {
 
 inline bool payload_empty(const RadixPayload& p) { return p.n == 0 && p.nparts == 0; }
 
+// Stable sort of rows by a list of passes, least significant first; `perm` (n
+// entries) receives the row order.  A pass whose digit is the same in every row
+// is skipped.
 // `inv` (optional, n entries): inv[row] = the row's position in the sorted
 // order, written by the last pass.  `payload` (optional): columns the last
 // pass writes in sorted order.  `fused`: the FusedKey of FUSED passes.
