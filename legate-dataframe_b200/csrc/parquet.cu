@@ -1360,6 +1360,25 @@ __device__ __forceinline__ int frag_page_of(const FragPage* fp, int n, int64_t g
   return lo;
 }
 
+// Follows every chain of a segment's entries e[0..m) out of the segment: pointer
+// jumping, the low halves added up.
+__device__ __forceinline__ void jump_to_exits(unsigned long long* e, int m)
+{
+  int more;
+  do {
+    __syncthreads();
+    more = 0;
+    for (int x = threadIdx.x; x < m; x += kExitThreads) {
+      const unsigned long long v = e[x];
+      const uint32_t nxt         = static_cast<uint32_t>(v >> 32);
+      if (nxt >= static_cast<uint32_t>(m)) continue;
+      const unsigned long long w = *static_cast<volatile unsigned long long*>(e + nxt);
+      e[x] = (w & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(v) + static_cast<uint32_t>(w));
+      more = 1;
+    }
+  } while (__syncthreads_or(more));
+}
+
 __global__ void __launch_bounds__(kExitThreads) snap_exits_kernel(const uint8_t* file, const FragPage* fp, int npages,
                                                                   unsigned long long* exits)
 {
@@ -1391,19 +1410,7 @@ __global__ void __launch_bounds__(kExitThreads) snap_exits_kernel(const uint8_t*
     const uint64_t nxt = x + size < 0xffffffffull ? x + size : 0xffffffffull;
     e[x]               = nxt << 32 | (out < 0xffffffffull ? out : 0xffffffffull);
   }
-  int more;
-  do {
-    __syncthreads();
-    more = 0;
-    for (int x = threadIdx.x; x < m; x += kExitThreads) {
-      const unsigned long long v = e[x];
-      const uint32_t nxt         = static_cast<uint32_t>(v >> 32);
-      if (nxt >= static_cast<uint32_t>(m)) continue;
-      const unsigned long long w = *static_cast<volatile unsigned long long*>(e + nxt);
-      e[x] = (w & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(v) + static_cast<uint32_t>(w));
-      more = 1;
-    }
-  } while (__syncthreads_or(more));
+  jump_to_exits(e, m);
   for (int x = threadIdx.x; x < m; x += kExitThreads) exits[f.exit0 + s0 + x] = e[x];
 }
 
@@ -1561,19 +1568,7 @@ __global__ void __launch_bounds__(kExitThreads) str_exits_kernel(const PqPage* p
     // (a value that runs past the page ends the chain uncounted)
     e[x] = end <= n && s0 + x + 4 <= n ? static_cast<unsigned long long>(end - s0) << 32 | 1u : 0xffffffffull << 32;
   }
-  int more;
-  do {
-    __syncthreads();
-    more = 0;
-    for (int x = threadIdx.x; x < m; x += kExitThreads) {
-      const unsigned long long v = e[x];
-      const uint32_t nxt         = static_cast<uint32_t>(v >> 32);
-      if (nxt >= static_cast<uint32_t>(m)) continue;
-      const unsigned long long w = *static_cast<volatile unsigned long long*>(e + nxt);
-      e[x] = (w & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(v) + static_cast<uint32_t>(w));
-      more = 1;
-    }
-  } while (__syncthreads_or(more));
+  jump_to_exits(e, m);
   for (int x = threadIdx.x; x < m; x += kExitThreads) exits[f.exit0 + s0 + x] = e[x];
 }
 
