@@ -198,10 +198,10 @@ int ldf_b200_arrow_offsets_to_ranges(const void* offsets, int32_t offset_bytes, 
 
 /* ---- file bytes -> pinned host memory -> device ---------------------------- */
 /* The first `nbytes` bytes of the file at `path` read into `host` (pinned) by
- * several threads, each piece copied to `dev` on `stream` as soon as it has
- * been read; the copies are complete when the call returns.  *os_error: 0, or
- * the errno of the read that failed (the call itself then still returns
- * LDF_OK). */
+ * several threads, each piece copied to `dev` as soon as it has been read, on a
+ * stream of the library behind the work that `stream` holds at the call; the
+ * copies are complete when the call returns.  *os_error: 0, or the errno of the
+ * read that failed (the call itself then still returns LDF_OK). */
 int ldf_b200_read_file(const char* path, int64_t nbytes, uint8_t* host, uint8_t* dev, int32_t* os_error,
                        void* stream);
 
