@@ -1570,6 +1570,7 @@ void radix_sort_pairs(const OpContext& ctx, FusedKey f, int bits, int64_t n, con
 
 int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, bool whole_rows)
 {
+  if (n < kDropMinRows) return 0;
   TieSampleArgs a{};
   a.f    = f;
   a.n    = n;
@@ -1582,7 +1583,7 @@ int choose_drop(const OpContext& ctx, const FusedKey& f, int bits, int64_t n, bo
   const int full = (bits + 7) / 8;
   for (int k = 2; k <= full - (whole_rows ? 1 : 2) && k <= 8; ++k)
     if (bits - 8 * k >= 8 && (int64_t(1) << std::min(8 * k, 62)) >= n / 16) a.drop[a.ncand++] = bits - 8 * k;
-  if (n < kDropMinRows || a.ncand == 0) return 0;
+  if (a.ncand == 0) return 0;
   cudaStream_t s = ctx.stream();
   Buffer<unsigned long long> slots(ctx.alloc(), static_cast<size_t>(a.ncand) * 2 * kSampleTies);
   Buffer<unsigned int> ties(ctx.alloc(), 2 * kDropCands), same;
